@@ -61,6 +61,8 @@ Plan::~Plan() {
   dfree(d_trees);
   dfree(d_fdown);
   dfree(d_fup);
+  dfree(d_deferred);
+  if (d_res) cudaFree(d_res);
 }
 
 // DcfrParams -> Discount (cfr.rs:86-106), host f64 pow as the reference.
@@ -212,9 +214,10 @@ Engine::~Engine() {
 
 void Engine::free_graphs() {
   if (iter_graph_) cudaGraphExecDestroy(iter_graph_);
+  if (chunk_graph_) cudaGraphExecDestroy(chunk_graph_);
   if (br_graph_) cudaGraphExecDestroy(br_graph_);
   if (avg_graph_) cudaGraphExecDestroy(avg_graph_);
-  iter_graph_ = br_graph_ = avg_graph_ = nullptr;
+  iter_graph_ = chunk_graph_ = br_graph_ = avg_graph_ = nullptr;
   if (prof_exec_) cudaGraphExecDestroy(prof_exec_);
   if (prof_graph_) cudaGraphDestroy(prof_graph_);
   prof_exec_ = nullptr;
@@ -250,6 +253,7 @@ Status Engine::init() {
   CK(cudaEventCreate(&ev0_));
   CK(cudaEventCreate(&ev1_));
   CK(terminal_kernel_setup());
+  CK(segment_setup());
   hp_[0] = pad8(g.n[0]);
   hp_[1] = pad8(g.n[1]);
   stride_ = std::max(hp_[0], hp_[1]);
@@ -372,7 +376,7 @@ Status Engine::init() {
   // Rows.
   if (!(s = dalloc(reach_, (size_t)max_slots_ * stride_, "reach rows")).ok()) return s;
   if (!(s = dalloc(vals_, (size_t)N * stride_, "value rows")).ok()) return s;
-  if (!(s = dalloc(alive_, (size_t)max_slots_, "liveness flags")).ok()) return s;
+  if (!(s = dalloc(alive_, (size_t)2 * max_slots_, "liveness flags")).ok()) return s;
   CK(cudaMemsetAsync(reach_, 0, (size_t)max_slots_ * stride_ * 4, stream_));
   CK(cudaMemsetAsync(vals_, 0, (size_t)N * stride_ * 4, stream_));
   {
@@ -401,7 +405,17 @@ Status Engine::init() {
   }
   for (int p = 0; p < 2; p++)
     if (!(s = upload_plan(*full_[p])).ok()) return s;
+  // The merged pass has the largest shared memory of the three.
+  if (full_[0]->seg && (segment_smem(segment_pass(full_[0].get(), full_[1].get())) > SEG_SMEM_MAX ||
+                        segment_smem(segment_pass(full_[1].get(), full_[0].get())) > SEG_SMEM_MAX))
+    for (int p = 0; p < 2; p++) drop_segment(*full_[p]);
   phase(setup.plans_ms);
+  // A block per terminal where every terminal gets a block of its own: a warp
+  // of the warp kernel takes it longer (river, 40 classes of hands: 7.1 us a
+  // launch against 4.8).
+  if (term_group_auto_ && term_kernel_ == TK_WARP && full_[0]->h_fast.size() <= (size_t)term_sms_ &&
+      full_[1]->h_fast.size() <= (size_t)term_sms_)
+    term_kernel_ = TK_BLOCK;
   // Default f32 terminal kernel: two warps per terminal where both
   // traversals have at least four terminal tasks per SM (measured faster there
   // than both the warp and the block kernel); the warp or block kernel for
@@ -884,6 +898,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
       plan.seg_up[l].push_back(Plan::Level{(uint32_t)plan.h_up.size(), (uint32_t)sup[l][d].size(), maxa, {0, 0, 0}});
       plan.h_up.insert(plan.h_up.end(), sup[l][d].begin(), sup[l][d].end());
     }
+  plan.seg = !compressed_ && g.nodes[root].kind == N_PLAYER;
   // Exact precision's terminal groups: showdowns by (kind, board), folds by
   // kind, 32 lanes each (fast precision uses h_fast only).
   if (!fast_)
@@ -1042,6 +1057,12 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
     for (auto& l : ls) seg_down_launches += l.count > 0;
   for (auto& ls : plan.seg_up)
     for (auto& l : ls) seg_up_launches += l.count > 0;
+  if (plan.seg) {  // the root segment: one launch each way
+    for (auto& l : plan.seg_down[0]) seg_down_launches -= l.count > 0;
+    for (auto& l : plan.seg_up[0]) seg_up_launches -= l.count > 0;
+    seg_down_launches++;
+    seg_up_launches++;
+  }
   kernels += seg_down_launches + seg_up_launches;
   const int term_kernels = fast_ ? (plan.h_fast.empty() ? 0 : 1) : (int)plan.waves.size();
   kernels += term_kernels;
@@ -1098,6 +1119,7 @@ Status Engine::upload_plan(Plan& plan) {
   if (!plan.h_panels.empty())
     CK(cudaMemcpy(plan.d_panels, plan.h_panels.data(), plan.h_panels.size() * sizeof(PanelD),
                   cudaMemcpyHostToDevice));
+  if (plan.seg && !(s = upload_segment(plan)).ok()) return s;
   if (!(s = dalloc(plan.d_trees, plan.h_trees.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fdown, plan.h_fdown.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fup, plan.h_fup.size(), "plan")).ok()) return s;
@@ -1125,6 +1147,96 @@ Status Engine::upload_plan(Plan& plan) {
   return Status();
 }
 
+// The root segment in its own numbering (SegRes): value row 0 is the root's,
+// then each decision node's children in a run; slot 0 the root's, then the
+// opponent nodes' children in a run; storage rows as the nodes' blocks.
+Status Engine::upload_segment(Plan& plan) {
+  const std::vector<Plan::Level>&ul = plan.seg_up[0], &dl = plan.seg_down[0];
+  std::vector<uint32_t> nodes;  // its decision nodes, parents first
+  for (const Plan::Level& lv : ul)
+    for (uint32_t i = 0; i < lv.count; i++) nodes.push_back(plan.h_up[lv.first + i].node);
+  std::sort(nodes.begin(), nodes.end());
+  std::unordered_map<uint32_t, uint32_t> row_of, slot_of, store_of;  // by node, global slot, node
+  std::vector<uint64_t> own[2];
+  std::vector<uint32_t> slots{0};
+  std::vector<SegRow> vals;
+  uint32_t nrows = 1;
+  row_of[plan.root] = 0;
+  slot_of[0] = 0;
+  plan.seg_maxa = 1;
+  for (uint32_t v : nodes) {
+    const GNode& nd = g.nodes[v];
+    plan.seg_maxa = std::max<int>(plan.seg_maxa, nd.nchild);
+    store_of[v] = (uint32_t)own[nd.player].size();
+    for (uint32_t a = 0; a < nd.nchild; a++) {
+      own[nd.player].push_back(gpu_off_[v] + (uint64_t)a * hp_[nd.player]);
+      row_of[nd.first + a] = nrows;
+      if (!std::binary_search(nodes.begin(), nodes.end(), nd.first + a)) vals.push_back(SegRow{nd.first + a, nrows});
+      nrows++;
+    }
+  }
+  std::unordered_map<uint64_t, uint32_t> node_at;  // block -> node
+  for (uint32_t v : nodes) node_at[gpu_off_[v]] = v;
+  std::vector<SegDown> down;
+  std::vector<SegUp> up;
+  std::vector<uint32_t> ulevs{0}, dlevs{0};
+  for (const Plan::Level& lv : dl) {
+    for (uint32_t i = 0; i < lv.count; i++) {
+      const DownTask& T = plan.h_down[lv.first + i];
+      const uint32_t first = (uint32_t)slots.size();
+      for (uint32_t a = 0; a < T.nchild; a++) {
+        slot_of[T.out_slot + a] = first + a;
+        slots.push_back(T.out_slot + a);
+      }
+      down.push_back(SegDown{slot_of[T.in_slot], first, T.nchild, store_of[node_at[T.store]], T.store, T.out_slot,
+                             1.0f / (float)T.nchild});
+    }
+    dlevs.push_back((uint32_t)down.size());
+  }
+  for (size_t l = ul.size(); l-- > 0;) {
+    for (uint32_t i = 0; i < ul[l].count; i++) {
+      const UpTask& T = plan.h_up[ul[l].first + i];
+      up.push_back(SegUp{T.kind, T.nchild, slot_of[T.slot], row_of[T.node], row_of[T.child], slot_of[T.child_slot],
+                         T.kind == U_OWN ? store_of[T.node] : 0u, T.node, T.store, 1.0f / (float)T.nchild, 0});
+    }
+    ulevs.push_back((uint32_t)up.size());
+  }
+  SegRes& R = plan.res;
+  R.nup = (uint32_t)ul.size();
+  R.ndown = (uint32_t)dl.size();
+  R.n_up = (uint32_t)up.size();
+  R.n_down = (uint32_t)down.size();
+  R.n_vals = (uint32_t)vals.size();
+  R.n_rows = nrows;
+  R.n_slots = (uint32_t)slots.size();
+  for (int q = 0; q < 2; q++) R.n_own[q] = (uint32_t)own[q].size();
+  R.root = plan.root;
+  ulevs.insert(ulevs.end(), dlevs.begin(), dlevs.end());
+  // One allocation, every array 16-byte aligned.
+  std::vector<unsigned char> h;
+  auto put = [&](const void* src, size_t bytes) {
+    const size_t at = h.size();
+    const unsigned char* b = static_cast<const unsigned char*>(src);
+    h.insert(h.end(), b, b + bytes);
+    h.resize((h.size() + 15) & ~(size_t)15);
+    return (uint32_t)at;
+  };
+  put(up.data(), up.size() * sizeof(SegUp));
+  R.o_down = put(down.data(), down.size() * sizeof(SegDown));
+  R.o_vals = put(vals.data(), vals.size() * sizeof(SegRow));
+  R.o_slots = put(slots.data(), slots.size() * 4);
+  R.o_levs = put(ulevs.data(), ulevs.size() * 4);
+  R.bytes = (uint32_t)h.size();
+  uint32_t o_own[2];
+  for (int q = 0; q < 2; q++) o_own[q] = put(own[q].data(), own[q].size() * 8);
+  CK(cudaMalloc(&plan.d_res, h.size()));
+  CK(cudaMemcpy(plan.d_res, h.data(), h.size(), cudaMemcpyHostToDevice));
+  R.blob = static_cast<const unsigned char*>(plan.d_res);
+  for (int q = 0; q < 2; q++) R.own[q] = reinterpret_cast<const uint64_t*>(R.blob + o_own[q]);
+  const size_t slices = (size_t)((stride_ + SEG_SLICE - 1) / SEG_SLICE);
+  return dalloc(plan.d_deferred, down.size() * slices, "plan");
+}
+
 void Engine::row_args(int p, RowArgs& A) const {
   A.regrets = regrets_;
   A.sums = sums_;
@@ -1135,7 +1247,7 @@ void Engine::row_args(int p, RowArgs& A) const {
   A.compressed = compressed_ ? 1 : 0;
   A.reach = reach_;
   A.vals = vals_;
-  A.alive = alive_;
+  A.alive = alive(p);
   for (int q = 0; q < 2; q++) {
     A.hc1[q] = hc1_[q];
     A.hc2[q] = hc2_[q];
@@ -1153,7 +1265,7 @@ void Engine::row_args(int p, RowArgs& A) const {
 void Engine::term_args(int p, TermArgs& A) const {
   A.reach = reach_;
   A.vals = vals_;
-  A.alive = alive_;
+  A.alive = alive(p);
   A.warp_scratch = warp_scratch_;
   A.warp_scratch_floats = warp_scratch_floats_;
   A.group_scratch = group_scratch_;
@@ -1184,7 +1296,7 @@ void Engine::term_args(int p, TermArgs& A) const {
 void Engine::fast_args(int p, FastArgs& A) const {
   A.reach = reach_;
   A.vals = vals_;
-  A.alive = alive_;
+  A.alive = alive(p);
   A.cat = fcat_;
   A.seg = fseg_;
   A.rec = frec_;
@@ -1200,23 +1312,61 @@ void Engine::fast_args(int p, FastArgs& A) const {
   A.p = p;
 }
 
-// Enqueues one traversal: liveness reset, root row, down levels, terminals,
-// up levels (deepest first); the root's value row is copied to root_out.
-void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row, float* root_out, bool advance) {
-  const int p = plan.p, o = p ^ 1;
-  launch_traversal_start(alive_, (int)plan.nslots, reach_, root_row, stride_, advance ? counter_ : nullptr,
-                         disc_table_, disc_len_, cur_disc_, stream_);
-  mark(DCFR_KERNEL_OTHER);
+// A root segment too large for segment passes: one launch per level.
+void Engine::drop_segment(Plan& plan) {
+  plan.seg = false;
+  int levels = 0;
+  for (auto& l : plan.seg_down[0]) levels += l.count > 0;
+  plan.class_kernels[DCFR_KERNEL_DOWN] += levels - 1;
+  plan.kernels += levels - 1;
+  levels = 0;
+  for (auto& l : plan.seg_up[0]) levels += l.count > 0;
+  plan.class_kernels[DCFR_KERNEL_UP] += levels - 1;
+  plan.kernels += levels - 1;
+}
+
+SegPass Engine::segment_pass(const Plan* up, const Plan* down) const {
+  SegPass P{};
+  P.slices = (stride_ + SEG_SLICE - 1) / SEG_SLICE;
+  const int q = up ? up->p : down->p ^ 1;
+  P.rows = (up ? up : down)->res.own[q];
+  P.n_rows = (up ? up : down)->res.n_own[q];
+  if (up) {
+    row_args(up->p, P.up);
+    P.U = up->res;
+    P.up_deferred = up->d_deferred;
+  }
+  if (down) {
+    row_args(down->p, P.down);
+    P.D = down->res;
+    P.down_deferred = down->d_deferred;
+  }
+  return P;
+}
+
+// A segment pass: the up pass of `up`'s root segment (its value row to
+// root_out, if given), then the down pass of `down`'s from root_row; either
+// may be null.
+void Engine::enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out) {
+  SegPass P = segment_pass(up, down);
+  P.root_out = root_out;
+  P.roots = root_row;
+  launch_segment(mode, std::max(up ? up->seg_maxa : 1, down ? down->seg_maxa : 1), P, stream_);
+}
+
+// Down levels below the root segment pass (or all, without one): segment
+// layer l (fused segments, then wide ones level by level), then the chance
+// nodes of layer l.
+void Engine::enqueue_down(const Plan& plan, int mode) {
+  const int o = plan.p ^ 1;
   RowArgs A;
-  row_args(p, A);
+  row_args(plan.p, A);
   const size_t layers = std::max({plan.tree_layers.size(), plan.down.size(), plan.seg_down.size()});
-  // Down: segment layer l (fused segments, then wide ones level by level),
-  // then the chance nodes of layer l.
   for (size_t l = 0; l < layers; l++) {
     if (l < plan.tree_layers.size() && plan.tree_layers[l].second)
       launch_fused_down(mode, plan.fused_maxa, A, plan.d_trees + plan.tree_layers[l].first,
                         (int)plan.tree_layers[l].second, plan.d_fdown, hp_[o], stream_);
-    if (l < plan.seg_down.size())
+    if (l < plan.seg_down.size() && !(l == 0 && plan.seg))
       for (const Plan::Level& lv : plan.seg_down[l])
         if (lv.count) launch_down(mode, lv.maxa, A, plan.d_down + lv.first, (int)lv.count, hp_[o], stream_);
     if (l < plan.down.size() && plan.down[l].count)
@@ -1224,6 +1374,11 @@ void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row
                   stream_);
   }
   mark(DCFR_KERNEL_DOWN);
+}
+
+// Terminals and leaves of a traversal.
+void Engine::enqueue_terminals(const Plan& plan) {
+  const int p = plan.p;
   if (fast_) {
     if (!plan.h_fast.empty()) {
       FastArgs F;
@@ -1259,12 +1414,19 @@ void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row
   }
   enqueue_leaves(plan);
   mark(DCFR_KERNEL_TERMINAL);
-  // Up: the chance nodes of layer l (their children are done), then segment
-  // layer l.
+}
+
+// Up levels below the root segment pass (or all): the chance nodes of layer
+// l (their children are done), then segment layer l.
+void Engine::enqueue_up(const Plan& plan, int mode) {
+  const int p = plan.p;
+  RowArgs A;
+  row_args(p, A);
+  const size_t layers = std::max({plan.tree_layers.size(), plan.down.size(), plan.seg_down.size()});
   for (size_t l = layers; l-- > 0;) {
     if (l < plan.up.size() && plan.up[l].count)
       launch_up(mode, plan.up[l].maxa, A, plan.d_up + plan.up[l].first, (int)plan.up[l].count, hp_[p], stream_);
-    if (l < plan.seg_up.size())
+    if (l < plan.seg_up.size() && !(l == 0 && plan.seg))
       for (size_t d = plan.seg_up[l].size(); d-- > 0;) {
         const Plan::Level& lv = plan.seg_up[l][d];
         if (lv.count) launch_up(mode, lv.maxa, A, plan.d_up + lv.first, (int)lv.count, hp_[p], stream_);
@@ -1273,10 +1435,53 @@ void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row
       launch_fused_up(mode, plan.fused_maxa, A, plan.d_trees + plan.tree_layers[l].first,
                       (int)plan.tree_layers[l].second, plan.d_fup, hp_[p], stream_);
   }
+}
+
+// Enqueues one traversal: liveness reset, root row, down levels, terminals,
+// up levels (deepest first); the root's value row is copied to root_out.
+void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row, float* root_out, bool advance) {
+  launch_traversal_start(alive(plan.p), (int)plan.nslots, nullptr, 0, reach_, root_row, stride_,
+                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, stream_);
+  mark(DCFR_KERNEL_OTHER);
+  if (plan.seg) enqueue_segment(nullptr, &plan, mode, root_row, nullptr);
+  enqueue_down(plan, mode);
+  enqueue_terminals(plan);
+  enqueue_up(plan, mode);
+  if (plan.seg) enqueue_segment(&plan, nullptr, mode, nullptr, root_out);
   mark(DCFR_KERNEL_UP);
-  if (root_out)
+  if (root_out && !plan.seg)
     cudaMemcpyAsync(root_out, vals_ + (size_t)plan.root * stride_, (size_t)stride_ * 4, cudaMemcpyDeviceToDevice,
                     stream_);
+}
+
+// Both players' traversals. Where both root segments take segment passes, one
+// start clears both traversals' flags and one pass takes player 0's hands up
+// the first traversal and down the second.
+void Engine::enqueue_pair(int mode, float* root_out, bool advance) {
+  const Plan &a = *full_[0], &b = *full_[1];
+  float* out1 = root_out ? root_out + stride_ : nullptr;
+  if (!a.seg || !b.seg) {
+    enqueue_traversal(a, mode, root_rows_, root_out, advance);
+    enqueue_traversal(b, mode, root_rows_ + stride_, out1);
+    return;
+  }
+  launch_traversal_start(alive(0), (int)a.nslots, alive(1), (int)b.nslots, reach_, root_rows_, stride_,
+                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, stream_);
+  enqueue_segment(nullptr, &a, mode, root_rows_, nullptr);
+  enqueue_down(a, mode);
+  enqueue_terminals(a);
+  enqueue_up(a, mode);
+  enqueue_segment(&a, &b, mode, root_rows_ + stride_, root_out);
+  enqueue_down(b, mode);
+  enqueue_terminals(b);
+  enqueue_up(b, mode);
+  enqueue_segment(&b, nullptr, mode, nullptr, out1);
+}
+
+// Kernels of enqueue_pair: the second start and one segment pass less than
+// two traversals where it merges them.
+int Engine::pair_launches() const {
+  return full_[0]->kernels + full_[1]->kernels - (full_[0]->seg && full_[1]->seg ? 2 : 0);
 }
 
 // Depth-limited solves: buffers of the leaf evaluation, and both players'
@@ -1328,7 +1533,7 @@ void Engine::enqueue_leaves(const Plan& plan) {
   LeafArgs A;
   A.reach = reach_;
   A.vals = vals_;
-  A.alive = alive_;
+  A.alive = alive(p);
   for (int q = 0; q < 2; q++) {
     A.leaf_reach[q] = leaf_reach_[q];
     A.combos[q] = combos_[q];
@@ -1413,21 +1618,39 @@ Status Engine::ensure_discounts(uint32_t max_t) {
   return Status();
 }
 
-Status Engine::capture_graphs() {
-  if (iter_graph_) return Status();
+// n DCFR iterations: t += 1, then player 0's and player 1's traversals with
+// the same discounts (lib.rs:577-585), each. The first traversal's start
+// kernel advances the iteration.
+Status Engine::capture_iterations(uint32_t n, cudaGraphExec_t& exec) {
   const auto t0 = std::chrono::steady_clock::now();
   cudaGraph_t graph;
-  // One DCFR iteration: t += 1, then player 0's and player 1's traversals
-  // with the same discounts (lib.rs:577-585).
-  // The first traversal's start kernel advances the iteration.
   CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  enqueue_traversal(*full_[0], M_CFR, root_rows_, nullptr, true);
-  enqueue_traversal(*full_[1], M_CFR, root_rows_ + stride_, nullptr);
+  for (uint32_t i = 0; i < n; i++) enqueue_pair(M_CFR, nullptr, true);
   CK(cudaStreamEndCapture(stream_, &graph));
-  CK(cudaGraphInstantiate(&iter_graph_, graph, 0));
+  const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
-  iter_kernels_ = full_[0]->kernels + full_[1]->kernels;
+  CK(e);
   setup.iteration_graph_ms += ms_since(t0);
+  return Status();
+}
+
+Status Engine::capture_graphs() {
+  if (iter_graph_) return Status();
+  iter_kernels_ = pair_launches();
+  return capture_iterations(1, iter_graph_);
+}
+
+// Launches iterations, at most `most`: `done` of them.
+Status Engine::launch_iterations(uint32_t most, uint32_t& done) {
+  const bool chunk = most >= ITER_CHUNK && singles_ >= ITER_SINGLES && g.nodes.size() <= ITER_CHUNK_NODES;
+  if (chunk && !chunk_graph_) {
+    Status s = capture_iterations(ITER_CHUNK, chunk_graph_);
+    if (!s.ok()) return s;
+  }
+  done = chunk ? ITER_CHUNK : 1;
+  if (!chunk) singles_++;
+  CK(cudaGraphLaunch(chunk ? chunk_graph_ : iter_graph_, stream_));
+  launches += (uint64_t)done * (uint64_t)iter_kernels_;
   return Status();
 }
 
@@ -1439,13 +1662,12 @@ Status Engine::capture_eval_graphs() {
   cudaGraph_t graph;
   for (int mode : {M_BR, M_AVG}) {
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    enqueue_traversal(*full_[0], mode, root_rows_, root_out_);
-    enqueue_traversal(*full_[1], mode, root_rows_ + stride_, root_out_ + stride_);
+    enqueue_pair(mode, root_out_);
     CK(cudaStreamEndCapture(stream_, &graph));
     CK(cudaGraphInstantiate(mode == M_BR ? &br_graph_ : &avg_graph_, graph, 0));
     cudaGraphDestroy(graph);
   }
-  pair_kernels_ = full_[0]->kernels + full_[1]->kernels;
+  pair_kernels_ = pair_launches();
   setup.eval_graphs_ms += ms_since(t0);
   return Status();
 }
@@ -1503,7 +1725,7 @@ Status Engine::iterate_profiled(uint32_t n, dcfr_kernel_profile& out) {
     for (size_t m = 0; m < M; m++)
       CK(cudaGraphExecEventRecordNodeSetEvent(prof_exec_, marks_[m].node, prof_events_[(size_t)i * M + m]));
     CK(cudaGraphLaunch(prof_exec_, stream_));
-    launches += iter_kernels_;
+    launches += full_[0]->kernels + full_[1]->kernels;
   }
   iterations += n;
   CK(cudaStreamSynchronize(stream_));
@@ -1536,10 +1758,8 @@ Status Engine::iterate(uint32_t n) {
   if (!(s = ensure_discounts(iterations + n + 1)).ok()) return s;
   if (!(s = capture_graphs()).ok()) return s;
   CK(cudaEventRecord(ev0_, stream_));
-  for (uint32_t i = 0; i < n; i++) {
-    CK(cudaGraphLaunch(iter_graph_, stream_));
-    launches += iter_kernels_;
-  }
+  for (uint32_t i = 0, k = 0; i < n; i += k)
+    if (!(s = launch_iterations(n - i, k)).ok()) return s;
   CK(cudaEventRecord(ev1_, stream_));
   iterations += n;
   CK(cudaEventSynchronize(ev1_));
@@ -1758,9 +1978,11 @@ Status Engine::solve_loop(const dcfr_solve_options& opts, const volatile int32_t
       CK(cudaStreamSynchronize(stream_));
       return Status();
     }
-    iterations += 1;
-    CK(cudaGraphLaunch(iter_graph_, stream_));
-    launches += iter_kernels_;
+    uint32_t k = 0;
+    if (!(s = launch_iterations(std::min(opts.max_iterations, std::max(next_check, iterations + 1)) - iterations, k))
+             .ok())
+      return s;
+    iterations += k;
     bool last = iterations >= opts.max_iterations;
     if (iterations >= next_check || last) {
       double e;
@@ -2094,6 +2316,9 @@ Status Engine::subtree_values(uint32_t root, int p, const std::vector<float>& op
     return s;
   }
   if (!(s = upload_plan(plan)).ok()) return s;
+  if (plan.seg && (segment_smem(segment_pass(nullptr, &plan)) > SEG_SMEM_MAX ||
+                   segment_smem(segment_pass(&plan, nullptr)) > SEG_SMEM_MAX))
+    drop_segment(plan);
   std::vector<float> row(stride_, 0.0f);
   std::copy(opp_reach.begin(), opp_reach.end(), row.begin());
   float* d_row = root_out_ + (size_t)(p ^ 1) * stride_;  // scratch row

@@ -26,6 +26,10 @@ void launch_fused_down(int mode, int maxa, const RowArgs& A, const FusedTree* tr
                        const DownTask* tasks, int hp, cudaStream_t s);
 void launch_fused_up(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees, const UpTask* tasks,
                      int hp, cudaStream_t s);
+// Segment passes (segment.cu).
+cudaError_t segment_setup();
+size_t segment_smem(const SegPass& P);
+void launch_segment(int mode, int maxa, const SegPass& P, cudaStream_t s);
 void launch_terminal(const TermArgs& A, const TermGroup* groups, const TermLane* lanes, const TermTask* tasks,
                      int ntasks, cudaStream_t s);
 cudaError_t terminal_kernel_setup();
@@ -72,7 +76,8 @@ void launch_evaluate(const unsigned long long* masks, uint32_t* out, int n, cuda
 void launch_five_card_counts(unsigned long long* counts, cudaStream_t s);
 // counter non-null: also advance the DCFR iteration (t += 1, the discounts
 // of iteration t from the table into cur).
-void launch_traversal_start(uint32_t* alive, int nslots, float* reach, const float* root_row, int stride,
+// alive2 non-null: also clear the flags of another traversal.
+void launch_traversal_start(uint32_t* alive, int nslots, uint32_t* alive2, int nslots2, float* reach, const float* root_row, int stride,
                             uint32_t* counter, const DiscountD* table, uint32_t table_len, DiscountD* cur,
                             cudaStream_t s);
 // Storage blocks between the device layout and the reference's packed
@@ -119,6 +124,13 @@ struct Plan {
   std::vector<DownTask> h_fdown;
   std::vector<UpTask> h_fup;
   int fused_maxa = 0;
+  // The root segment, where it takes segment passes (segment.cu): f32
+  // storage, a decision node at the root.
+  bool seg = false;
+  int seg_maxa = 0;
+  SegRes res{};
+  void* d_res = nullptr;           // its arrays
+  uint8_t* d_deferred = nullptr;   // [slices][down task]
   // Segments by layer (the number of chance nodes above): [first tree, count].
   std::vector<std::pair<uint32_t, uint32_t>> tree_layers;
   FusedTree* d_trees = nullptr;
@@ -256,7 +268,7 @@ class Engine {
   Status storage_in(void* dev, const void* host, int elem_bytes);
   float* reach_ = nullptr;
   float* vals_ = nullptr;
-  uint32_t* alive_ = nullptr;
+  uint32_t* alive_ = nullptr;    // [2][max_slots_] liveness flags per traverser
   float* root_rows_ = nullptr;   // [2][stride] opponent root weights per traverser
   float* root_out_ = nullptr;    // [2][stride] root values after a traversal pair
   uint8_t* hc1_[2] = {nullptr, nullptr};
@@ -325,6 +337,17 @@ class Engine {
   std::vector<uint32_t> cc_off_, iso_first_;
   std::unique_ptr<Plan> full_[2];
   cudaGraphExec_t iter_graph_ = nullptr, br_graph_ = nullptr, avg_graph_ = nullptr;
+  // ITER_CHUNK iterations in one graph, for small trees once a handle has run
+  // ITER_SINGLES of them: launching a graph leaves the GPU idle for about
+  // 4 us, a fifth of a river iteration (measured 4.2 of 26.6 us at 1081
+  // hands) and 1% of a turn's; capturing the chunk costs about 0.4 ms, which
+  // a solve of a few iterations would not earn back.
+  static constexpr uint32_t ITER_CHUNK = 10, ITER_SINGLES = 32;
+  static constexpr size_t ITER_CHUNK_NODES = 32768;
+  cudaGraphExec_t chunk_graph_ = nullptr;
+  uint32_t singles_ = 0;
+  Status launch_iterations(uint32_t most, uint32_t& done);
+  Status capture_iterations(uint32_t n, cudaGraphExec_t& exec);
   // Profiled iteration graph: event-record nodes at kernel-class boundaries.
   struct Mark {
     cudaGraphNode_t node;
@@ -344,10 +367,21 @@ class Engine {
   Status alloc_storage();
   Status build_plan(uint32_t root, int p, Plan& plan);
   Status upload_plan(Plan& plan);
+  Status upload_segment(Plan& plan);
+  SegPass segment_pass(const Plan* up, const Plan* down) const;
+  static void drop_segment(Plan& plan);
   void row_args(int p, RowArgs& A) const;
   void term_args(int p, TermArgs& A) const;
   void fast_args(int p, FastArgs& A) const;
+  uint32_t* alive(int p) const { return alive_ + (size_t)p * max_slots_; }
   void enqueue_traversal(const Plan& plan, int mode, const float* root_row, float* root_out, bool advance = false);
+  // Both traversals of an iteration (or of an evaluation).
+  void enqueue_pair(int mode, float* root_out, bool advance = false);
+  int pair_launches() const;
+  void enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out);
+  void enqueue_down(const Plan& plan, int mode);
+  void enqueue_terminals(const Plan& plan);
+  void enqueue_up(const Plan& plan, int mode);
   Status ensure_discounts(uint32_t max_t);
   Status capture_graphs();
   Status capture_eval_graphs();

@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "plan.hpp"
 #include "row_items.cuh"
 
@@ -23,8 +24,6 @@ namespace dcfr {
 // launch: a level's grid is launched while the previous one drains and waits
 // (griddepcontrol.wait) until that grid has completed and its writes are
 // visible.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
 // COMP: 16-bit compressed storage (one block covers a node's row).
 template <int MODE, int MAXA, bool COMP>
@@ -37,7 +36,7 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) down_kernel(RowArgs A, const 
   int phase = 0;  // block_max scratch row (compressed storage)
   if (T.kind == D_OPP_SPLIT) down_item<MODE, MAXA, D_OPP_SPLIT, COMP>(A, T, h0, threadIdx.x & 31, &phase);
   else down_item<MODE, 1, D_CHANCE_SPLIT>(A, T, h0, threadIdx.x & 31);
-  pdl_launch_dependents();
+  pdl_trigger();
 }
 
 template <int MODE, int MAXA, bool COMP>
@@ -50,7 +49,7 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) up_kernel(RowArgs A, const Up
   if (T.kind == U_OWN) up_item<MODE, MAXA, U_OWN, COMP>(A, T, h0, &phase);
   else if (T.kind == U_OPP_SUM) up_item<MODE, MAXA, U_OPP_SUM>(A, T, h0);
   else up_item<MODE, 1, U_CHANCE_SUM>(A, T, h0);
-  pdl_launch_dependents();
+  pdl_trigger();
 }
 
 // Fused river subtrees: one block per subtree walks its nodes (see
@@ -70,7 +69,7 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) fused_down_kernel(RowArgs A, 
     if (T.kind & LEVEL_BREAK) __syncthreads();
     down_item<MODE, MAXA, D_OPP_SPLIT, COMP>(A, T, h0, lane, &phase);
   }
-  pdl_launch_dependents();
+  pdl_trigger();
 }
 
 template <int MODE, int MAXA, bool COMP>
@@ -86,7 +85,7 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) fused_up_kernel(RowArgs A, co
     if ((T.kind & KIND_MASK) == U_OWN) up_item<MODE, MAXA, U_OWN, COMP>(A, T, h0, &phase);
     else up_item<MODE, MAXA, U_OPP_SUM>(A, T, h0);
   }
-  pdl_launch_dependents();
+  pdl_trigger();
 }
 
 // ------------------------------------------------------------ setup kernels
@@ -267,17 +266,7 @@ static int row_threads(int hp) {
 template <typename K, typename Task>
 static void launch_level(K kernel, const RowArgs& A, const Task* tasks, int ntasks, int hp, cudaStream_t s) {
   const int threads = row_threads(hp), chunks = (hp + threads * VEC - 1) / (threads * VEC);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ntasks * chunks));
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, A, tasks, chunks);
+  launch_dependent(kernel, (unsigned)(ntasks * chunks), (unsigned)threads, 0, s, A, tasks, chunks);
 }
 
 template <int MODE>
@@ -307,17 +296,7 @@ static void launch_up_m(int maxa, const RowArgs& A, const UpTask* tasks, int nta
 template <typename K, typename Task>
 static void launch_fused(K kernel, const RowArgs& A, const FusedTree* trees, int ntrees, const Task* tasks, int hp,
                          cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ntrees);
-  cfg.blockDim = dim3((unsigned)row_threads(hp));
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, A, trees, tasks);
+  launch_dependent(kernel, (unsigned)ntrees, (unsigned)row_threads(hp), 0, s, A, trees, tasks);
 }
 
 template <int MODE>
@@ -388,15 +367,16 @@ void launch_five_card_counts(unsigned long long* counts, cudaStream_t s) {
 }
 
 
-// Start of a traversal: every liveness flag cleared but the root slot's, and
-// the root's reach row copied into slot 0. One launch in place of two
+// Start of a traversal (or, with alive2, of a pair of them): every liveness
+// flag cleared but the root slot's, and the root's reach row copied into slot 0. One launch in place of two
 // memsets and a copy, chained to the traversal's level launches by
 // programmatic dependent launch (the flags are cleared only once the
 // previous traversal's kernels, which read them, are complete). The first
 // traversal of a DCFR iteration also advances the iteration (counter given):
 // t += 1 and the iteration's discounts from the table, read by the
 // traversal's row kernels after their wait.
-__global__ void traversal_start_kernel(uint32_t* __restrict__ alive, int nslots, float* __restrict__ reach,
+__global__ void traversal_start_kernel(uint32_t* __restrict__ alive, int nslots, uint32_t* __restrict__ alive2,
+                                       int nslots2, float* __restrict__ reach,
                                        const float* __restrict__ root_row, int stride, uint32_t* counter,
                                        const DiscountD* table, uint32_t table_len, DiscountD* cur) {
   pdl_wait();
@@ -407,9 +387,10 @@ __global__ void traversal_start_kernel(uint32_t* __restrict__ alive, int nslots,
   }
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   for (int i = i0; i < nslots; i += step) alive[i] = i == 0 ? 1u : 0u;
+  for (int i = i0; i < nslots2; i += step) alive2[i] = 0u;
   for (int i = i0; i < stride / 4; i += step)
     reinterpret_cast<float4*>(reach)[i] = reinterpret_cast<const float4*>(root_row)[i];
-  pdl_launch_dependents();
+  pdl_trigger();
 }
 
 // Storage blocks between the device layout (each action's row padded to hp
@@ -466,25 +447,15 @@ void launch_storage_unpack(int elem_bytes, void* dev, const void* packed, const 
         static_cast<uint16_t*>(dev), static_cast<const uint16_t*>(packed), blocks, nblocks);
 }
 
-void launch_traversal_start(uint32_t* alive, int nslots, float* reach, const float* root_row, int stride,
-                            uint32_t* counter, const DiscountD* table, uint32_t table_len, DiscountD* cur,
+void launch_traversal_start(uint32_t* alive, int nslots, uint32_t* alive2, int nslots2, float* reach,
+                            const float* root_row, int stride, uint32_t* counter, const DiscountD* table, uint32_t table_len, DiscountD* cur,
                             cudaStream_t s) {
-  const int threads = 256, work = nslots > stride / 4 ? nslots : stride / 4;
+  const int threads = 256, rows = nslots > nslots2 ? nslots : nslots2, work = rows > stride / 4 ? rows : stride / 4;
   int blocks = (work + threads - 1) / threads;
   if (blocks > 1184) blocks = 1184;
   if (blocks < 1) blocks = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)blocks);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, traversal_start_kernel, alive, nslots, reach, root_row, stride, counter, table, table_len,
-                     cur);
+  launch_dependent(traversal_start_kernel, (unsigned)blocks, (unsigned)threads, 0, s, alive, nslots, alive2, nslots2, reach,
+                   root_row, stride, counter, table, table_len, cur);
 }
 
 }  // namespace dcfr

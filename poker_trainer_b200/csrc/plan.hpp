@@ -231,6 +231,58 @@ struct RowArgs {
   int p;
 };
 
+// Segment passes (segment.cu). Tasks count slots, value rows and storage rows
+// in the segment's own numbering; g* are the global ones.
+constexpr int SEG_SLICE = 32;                  // hands per block
+constexpr size_t SEG_SMEM_MAX = 200 << 10;     // shared memory of a pass
+struct SegUp {
+  uint32_t kind, nchild;
+  uint32_t slot, node, child, child_slot;
+  uint32_t store;   // traverser node: its first storage row
+  uint32_t gnode;
+  uint64_t gstore;  // traverser node: float offset of its block
+  float uniform;    // 1 / nchild
+  uint32_t pad;
+};
+struct SegDown {
+  uint32_t in_slot, out_slot, nchild, store;
+  uint64_t gstore;
+  uint32_t gslot;   // first child's slot
+  float uniform;
+};
+// A value row another kernel fills (a terminal's, a chance node's, a leaf's):
+// its node and its row in the segment's numbering.
+struct SegRow {
+  uint32_t node, row;
+};
+// One traversal's root segment: its records in one array, the up tasks first,
+// then at byte offsets the down tasks, the value rows to fetch, the global
+// slot of each of its slots, and the level boundaries of the up (deepest
+// first) and then the down tasks.
+struct SegRes {
+  const unsigned char* blob;
+  uint32_t o_down, o_vals, o_slots, o_levs, bytes;
+  const uint64_t* own[2];  // per player: float offsets of its storage rows
+  uint32_t nup, ndown;     // levels
+  uint32_t n_up, n_down;   // tasks
+  uint32_t n_vals, n_rows, n_slots, n_own[2];  // fetched rows, value rows, slots, storage rows
+  uint32_t root;           // the root's node
+};
+
+// One launch: the up pass of the traversal U (of traverser up.p) and then the
+// down pass of D (of down.p); one that is not wanted has no blob.
+struct SegPass {
+  RowArgs up, down;
+  SegRes U, D;
+  const uint64_t* rows;        // storage rows of the player that both update
+  uint32_t n_rows;
+  int slices;
+  const uint8_t* up_deferred;  // [slices][down task]
+  uint8_t* down_deferred;
+  float* root_out;             // the root's value row, or null
+  const float* roots;          // the root's reach row
+};
+
 // Arguments of the FP64 best-response kernels (br64.cu): double reach and
 // value rows, the f32 strategy sums.
 struct Row64Args {

@@ -24,6 +24,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "plan.hpp"
 #include "warp_terminal.cuh"
 
@@ -191,10 +192,26 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     for (int i = tid; i < hpo / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
     cp_async_commit();
   };
-  prefetch(t0, 0);
   uint32_t board = NONE32;
   int L = 0;
   FastTask T = tasks[t0];
+  auto stage = [&](uint32_t b) {
+    board = b;
+    const size_t lay = (size_t)board * 2 + p;
+    const uint16_t* gseg = A.seg + lay * FAST_SEGS;
+    if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
+    L = gseg[FAST_SEGS - 1];
+    const uint16_t* gcat = A.cat + lay * A.cstride;
+    for (int k = tid; k < L; k += FAST_THREADS) scat[k] = gcat[k];
+    const uint4* grec = A.rec + lay * A.tstride;
+    for (int h = tid; h < np; h += FAST_THREADS) srec[h] = grec[h];
+  };
+  // The first task's layout is staged while the grid before this one drains;
+  // the rows and flags come after it.
+  stage(T.board);
+  pdl_wait();
+  pdl_trigger();
+  prefetch(t0, 0);
 
   // Three block barriers per terminal: after the row maxima (1), after the
   // scan's warp totals (2) and after the prefixes are written (3). The next
@@ -244,15 +261,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     ti = next;
     if (A.alive[cur.slot] == 0) continue;  // dead subtree (cfr.rs:267-274): row untouched
     if (cur.board != board) {
-      board = cur.board;
-      const size_t lay = (size_t)board * 2 + p;
-      const uint16_t* gseg = A.seg + lay * FAST_SEGS;
-      if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
-      L = gseg[FAST_SEGS - 1];
-      const uint16_t* gcat = A.cat + lay * A.cstride;
-      for (int k = tid; k < L; k += FAST_THREADS) scat[k] = gcat[k];
-      const uint4* grec = A.rec + lay * A.tstride;
-      for (int h = tid; h < np; h += FAST_THREADS) srec[h] = grec[h];
+      stage(cur.board);
       __syncthreads();  // the new layout is staged (once per board)
     }
     mx = 0;
@@ -497,6 +506,8 @@ __global__ void __launch_bounds__(512, 1) warp_terminal_kernel(FastArgsT<R> A, c
   int buf = 0;
   int next = t0 + warp;  // this warp's current task
   bool live = false;
+  pdl_wait();
+  pdl_trigger();
   if (next < t1) {
     live = A.alive[tasks[next].slot] != 0;
     if (live) warp_row_prefetch<R>(A, tasks[next].slot, row, lane);
@@ -715,7 +726,8 @@ static void launch_warp_terminal_t(const FastArgsT<R>& A, const FastTask* tasks,
   // At most one block per task: every block's range is non-empty.
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
   const size_t smem = warp_terminal_smem(A.stride, A.cstride, A.tstride, (int)sizeof(R), warps);
-  warp_terminal_kernel<R><<<blocks, warps * 32, smem, s>>>(A, tasks, units, nunits, ntasks);
+  launch_dependent(warp_terminal_kernel<R>, (unsigned)blocks, (unsigned)(warps * 32), smem, s, A, tasks, units, nunits,
+                   ntasks);
 }
 
 void launch_warp_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
@@ -745,7 +757,7 @@ static void launch_fast_terminal_t(const FastArgsT<R>& A, const FastTask* tasks,
   switch (A.emax) {
 #define FAST_E(e_)                                                                     \
   case e_:                                                                             \
-    fast_terminal_kernel<e_, R><<<blocks, FAST_THREADS, smem, s>>>(A, tasks, ntasks); \
+    launch_dependent(fast_terminal_kernel<e_, R>, (unsigned)blocks, FAST_THREADS, smem, s, A, tasks, ntasks, nullptr); \
     break;
     FAST_E(1) FAST_E(3) FAST_E(5) FAST_E(7) FAST_E(9) FAST_E(11) FAST_E(13) FAST_E(15) FAST_E(17)
 #undef FAST_E

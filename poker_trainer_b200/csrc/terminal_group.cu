@@ -25,6 +25,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "plan.hpp"
 #include "warp_terminal.cuh"
 
@@ -303,6 +304,22 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
       else hi = mid;
     }
   }
+  int L = 0;
+  auto stage = [&](uint32_t layout) {
+    const size_t lay = (size_t)layout * 2 + p;
+    const uint16_t* gseg = A.seg + lay * FAST_SEGS;
+    if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
+    L = gseg[FAST_SEGS - 1];
+    const uint16_t* gcat = A.cat + lay * A.cstride;
+    for (int k = tid; k < L; k += blockDim.x) scat[k] = gcat[k];
+    const uint4* grec = A.rec + lay * A.tstride;
+    for (int h = tid; h < np; h += blockDim.x) srec[h] = grec[h];
+  };
+  // The first unit's layout is staged while the grid before this one drains.
+  const int u0 = u;
+  stage(units[u].layout);
+  pdl_wait();
+  pdl_trigger();
   int buf = 0;
   int next = t0 + grp;  // this group's current task
   bool live = false;
@@ -313,15 +330,10 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   cp_async_commit();
   for (; u < nunits && (int)units[u].first < t1; u++) {
     const TermUnit U = units[u];
-    __syncthreads();  // the previous unit's groups are done with the layout
-    const size_t lay = (size_t)U.layout * 2 + p;
-    const uint16_t* gseg = A.seg + lay * FAST_SEGS;
-    if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
-    const int L = gseg[FAST_SEGS - 1];
-    const uint16_t* gcat = A.cat + lay * A.cstride;
-    for (int k = tid; k < L; k += blockDim.x) scat[k] = gcat[k];
-    const uint4* grec = A.rec + lay * A.tstride;
-    for (int h = tid; h < np; h += blockDim.x) srec[h] = grec[h];
+    if (u != u0) {
+      __syncthreads();  // the previous unit's groups are done with the layout
+      stage(U.layout);
+    }
     __syncthreads();
     const WarpLayout Y{ssame, scat, srec, sseg, L};
     // This thread's first segment boundary at or after its first element.
@@ -390,7 +402,8 @@ void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermU
   // At most one block per task: every block's range is non-empty.
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
   const size_t smem = group_terminal_smem(A.stride, A.cstride, A.tstride, groups);
-  group_terminal_kernel<<<blocks, groups * GROUP_THREADS, smem, s>>>(A, tasks, units, nunits, ntasks);
+  launch_dependent(group_terminal_kernel, (unsigned)blocks, (unsigned)(groups * GROUP_THREADS), smem, s, A, tasks, units,
+                   nunits, ntasks);
 }
 
 }  // namespace dcfr
