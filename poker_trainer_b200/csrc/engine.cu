@@ -51,9 +51,6 @@ static inline int pad8(int n) { return (n + 7) & ~7; }
 Plan::~Plan() {
   dfree(d_down);
   dfree(d_up);
-  dfree(d_groups);
-  dfree(d_lanes);
-  dfree(d_tasks);
   dfree(d_fast);
   dfree(d_units);
   dfree(d_panels);
@@ -179,16 +176,6 @@ Engine::~Engine() {
   dfree(iso_);
   dfree(tables_);
   dfree(table_count_);
-  dfree(progs_);
-  dfree(prog_count_);
-  dfree(posmap_);
-  for (int q = 0; q < 2; q++) {
-    dfree(fold_prog_[q]);
-    dfree(emit_rec_[q]);
-  }
-  dfree(warp_scratch_);
-  dfree(group_scratch_);
-  dfree(counters_);
   dfree(term_counter_);
   dfree(fcat_);
   dfree(fseg_);
@@ -252,7 +239,6 @@ Status Engine::init() {
   CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev0_));
   CK(cudaEventCreate(&ev1_));
-  CK(terminal_kernel_setup());
   CK(segment_setup());
   hp_[0] = pad8(g.n[0]);
   hp_[1] = pad8(g.n[1]);
@@ -272,7 +258,6 @@ Status Engine::init() {
   compressed_ = g.compressed;
 
   tstride_ = std::max(g.n[0], g.n[1]);
-  pstride_ = (2 * tstride_ + TERM_CHUNK - 1) / TERM_CHUNK * TERM_CHUNK;
   // Hands.
   for (int q = 0; q < 2; q++) {
     std::vector<uint8_t> a(hp_[q], 255), b(hp_[q], 255);
@@ -288,14 +273,6 @@ Status Engine::init() {
     CK(cudaMemcpy(hc1_[q], a.data(), hp_[q], cudaMemcpyHostToDevice));
     CK(cudaMemcpy(hc2_[q], b.data(), hp_[q], cudaMemcpyHostToDevice));
     CK(cudaMemcpy(same_[q], sm.data(), hp_[q] * 4, cudaMemcpyHostToDevice));
-    if (fast_) continue;
-    // The player's hands in hand order as sweep steps (fold sums) and per-hand
-    // emit records (terminal.cu).
-    const int npad = (g.n[q] + TERM_CHUNK - 1) / TERM_CHUNK * TERM_CHUNK;
-    if (!(s = dalloc(fold_prog_[q], npad, "hands")).ok()) return s;
-    if (!(s = dalloc(emit_rec_[q], g.n[q], "hands")).ok()) return s;
-    launch_hand_program(hc1_[q], hc2_[q], same_[q], g.n[q], npad, fold_prog_[q], emit_rec_[q], stream_);
-    CK(cudaGetLastError());
   }
   {
     std::vector<uint16_t> perm((size_t)12 * stride_, 0);
@@ -341,18 +318,10 @@ Status Engine::init() {
       launch_strength(d_boards, nb, hc1_[0], hc2_[0], hc1_[1], hc2_[1], g.n[0], g.n[1], tables_, table_count_,
                       tstride_, stream_);
       CK(cudaGetLastError());
-      if (!fast_) {
-        // Sweep programs (terminal.cu): per board, traverser and pass.
-        if (!(s = dalloc(progs_, (size_t)nb * 6 * pstride_, "sweep programs")).ok()) return s;
-        if (!(s = dalloc(prog_count_, (size_t)nb * 6, "sweep programs")).ok()) return s;
-        if (!(s = dalloc(posmap_, (size_t)nb * 6 * tstride_, "sweep programs")).ok()) return s;
-        launch_programs(tables_, table_count_, tstride_, progs_, prog_count_, posmap_, pstride_, nb, stream_);
-        CK(cudaGetLastError());
-      }
       CK(cudaStreamSynchronize(stream_));
       cudaFree(d_boards);
     }
-    if (fast_ && !(s = ensure_fast_layouts()).ok()) return s;
+    if (!(s = ensure_fast_layouts()).ok()) return s;
   }
   phase(setup.tables_ms);
   // Plans for the two traversals of an iteration, built on two host threads
@@ -388,21 +357,6 @@ Status Engine::init() {
     if (!(s = dalloc(root_out_, rr.size(), "root rows")).ok()) return s;
   }
   phase(setup.rows_ms);
-  // Terminal scratch, sized for the largest terminal launch of the two plans.
-  if (!fast_) {
-    for (int p = 0; p < 2; p++)
-      for (const Plan::Wave& w : full_[p]->waves) {
-        wave_tasks_ = std::max<int>(wave_tasks_, (int)w.count);
-        wave_groups_ = std::max<int>(wave_groups_, (int)w.groups);
-      }
-    warp_scratch_floats_ = (size_t)(pstride_ + 1) * 32 + (size_t)stride_ * 32;
-    if (!(s = dalloc(warp_scratch_, (size_t)std::max(wave_tasks_, 1) * warp_scratch_floats_, "terminal scratch")).ok())
-      return s;
-    if (!(s = dalloc(group_scratch_, (size_t)std::max(wave_groups_, 1) * 2 * tstride_ * 32, "terminal scratch")).ok())
-      return s;
-    if (!(s = dalloc(counters_, (size_t)std::max(wave_groups_, 1), "terminal scratch")).ok()) return s;
-    CK(cudaMemsetAsync(counters_, 0, (size_t)std::max(wave_groups_, 1) * 4, stream_));
-  }
   for (int p = 0; p < 2; p++)
     if (!(s = upload_plan(*full_[p])).ok()) return s;
   // The merged pass has the largest shared memory of the three.
@@ -458,9 +412,8 @@ Status Engine::alloc_storage() {
   return Status();
 }
 
-// Scan layouts of the fast terminal kernel (terminal_fast.cu): the boards'
-// strength tables, then the fold layout. Built in init for fast precision,
-// and on first use by the FP64 best-response oracle in exact precision.
+// Scan layouts of the terminal kernels: the boards' strength tables, then the
+// fold layout.
 Status Engine::ensure_fast_layouts() {
   if (fcat_) return Status();
   Status s;
@@ -485,6 +438,11 @@ Status Engine::ensure_fast_layouts() {
     return s;
   }
   fast_blocks_ = sms * per_sm;
+  if (!fast_) {
+    const int bps = exact_terminal_setup(stride_, fcstride_, tstride_);
+    if (bps <= 0) return Status{DCFR_ERR_CUDA, "exact terminal kernel: shared-memory layout does not fit an SM"};
+    exact_blocks_ = sms * bps;
+  }
   // The f32 solve's terminal kernel: a warp per terminal for short hand
   // lists, a block-wide scan per terminal for long ones (measured fastest);
   // DCFR_TERMINAL_KERNEL selects another one (panel, panel4, panel8, warp,
@@ -899,31 +857,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
       plan.h_up.insert(plan.h_up.end(), sup[l][d].begin(), sup[l][d].end());
     }
   plan.seg = !compressed_ && g.nodes[root].kind == N_PLAYER;
-  // Exact precision's terminal groups: showdowns by (kind, board), folds by
-  // kind, 32 lanes each (fast precision uses h_fast only).
-  if (!fast_)
-    std::stable_sort(sd.begin(), sd.end(), [](const SdLane& a, const SdLane& b) {
-      return a.kind != b.kind ? a.kind < b.kind : a.board < b.board;
-    });
-  plan.h_groups.clear();
-  plan.h_lanes.clear();
-  for (size_t i = 0; !fast_ && i < sd.size();) {
-    size_t j = i;
-    while (j < sd.size() && j - i < 32 && sd[j].kind == sd[i].kind && sd[j].board == sd[i].board) j++;
-    TermGroup G{sd[i].kind, sd[i].board, (uint32_t)plan.h_lanes.size(), (uint32_t)(j - i)};
-    for (size_t k = i; k < j; k++) plan.h_lanes.push_back(sd[k].lane);
-    plan.h_groups.push_back(G);
-    i = j;
-  }
-  for (int b = 0; b < 2 && !fast_; b++)
-    for (size_t i = 0; i < folds[b].size(); i += 32) {
-      size_t j = std::min(folds[b].size(), i + 32);
-      TermGroup G{b ? (uint32_t)T_FOLD_BATCH : (uint32_t)T_FOLD_SCALAR, 0, (uint32_t)plan.h_lanes.size(),
-                  (uint32_t)(j - i)};
-      for (size_t k = i; k < j; k++) plan.h_lanes.push_back(folds[b][k]);
-      plan.h_groups.push_back(G);
-    }
-  // Fast precision: one task per terminal, grouped by layout. A fold below
+  // One task per terminal, grouped by layout. A fold below
   // a river decision node is evaluated on its river board's layout: the
   // opponent hands that layout leaves out hold a board card and have zero
   // reach there, so every integer sum is the same as on the all-hands fold
@@ -1014,38 +948,6 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
     plan.h_units.push_back(TermUnit{plan.h_fast[i].board, (uint32_t)i, (uint32_t)(j - i), 0});
     i = j;
   }
-  // Terminal tasks: one warp per fold group; per showdown group, the
-  // ascending and descending passes and, when a terminal has a paired fold,
-  // the paired fold's pass. Launches ("waves") are bounded in tasks and in
-  // showdown groups (scratch).
-  plan.h_tasks.clear();
-  plan.waves.clear();
-  Plan::Wave wave;
-  auto close_wave = [&]() {
-    if (wave.count) plan.waves.push_back(wave);
-    wave = Plan::Wave();
-    wave.first = (uint32_t)plan.h_tasks.size();
-  };
-  wave.first = 0;
-  for (size_t gi = 0; gi < plan.h_groups.size(); gi++) {
-    const TermGroup& G = plan.h_groups[gi];
-    if (G.kind == T_FOLD_SCALAR || G.kind == T_FOLD_BATCH) {
-      if (wave.count + 1 > (uint32_t)MAX_WAVE_TASKS) close_wave();
-      plan.h_tasks.push_back(TermTask{R_FOLD, (uint32_t)gi, 0, 0});
-      wave.count += 1;
-      continue;
-    }
-    bool paired = false;
-    for (uint32_t k = 0; k < G.count; k++) paired |= plan.h_lanes[G.first + k].frow != NONE32;
-    const uint32_t need = paired ? 3 : 2;
-    if (wave.count + need > (uint32_t)MAX_WAVE_TASKS || wave.groups + 1 > (uint32_t)MAX_WAVE_GROUPS) close_wave();
-    const uint32_t wg = wave.groups++;
-    plan.h_tasks.push_back(TermTask{R_ASC, (uint32_t)gi, wg, 0});
-    plan.h_tasks.push_back(TermTask{R_DESC, (uint32_t)gi, wg, 0});
-    if (paired) plan.h_tasks.push_back(TermTask{R_PAIRED, (uint32_t)gi, wg, 0});
-    wave.count += need;
-  }
-  close_wave();
   int kernels = 0;
   int tree_launches = 0;
   for (auto& tl : plan.tree_layers) tree_launches += tl.second > 0;
@@ -1064,7 +966,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
     seg_up_launches++;
   }
   kernels += seg_down_launches + seg_up_launches;
-  const int term_kernels = fast_ ? (plan.h_fast.empty() ? 0 : 1) : (int)plan.waves.size();
+  const int term_kernels = plan.h_fast.empty() ? 0 : 1;
   kernels += term_kernels;
   kernels += 1;  // the traversal's start (liveness flags, root row)
   plan.kernels = kernels;
@@ -1104,9 +1006,6 @@ Status Engine::upload_plan(Plan& plan) {
   Status s;
   if (!(s = dalloc(plan.d_down, plan.h_down.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_up, plan.h_up.size(), "plan")).ok()) return s;
-  if (!(s = dalloc(plan.d_groups, plan.h_groups.size(), "plan")).ok()) return s;
-  if (!(s = dalloc(plan.d_lanes, plan.h_lanes.size(), "plan")).ok()) return s;
-  if (!(s = dalloc(plan.d_tasks, plan.h_tasks.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fast, plan.h_fast.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_units, plan.h_units.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_leaves, plan.h_leaves.size(), "plan")).ok()) return s;
@@ -1133,17 +1032,10 @@ Status Engine::upload_plan(Plan& plan) {
   }
   if (!plan.h_fast.empty())
     CK(cudaMemcpy(plan.d_fast, plan.h_fast.data(), plan.h_fast.size() * sizeof(FastTask), cudaMemcpyHostToDevice));
-  if (!plan.h_tasks.empty())
-    CK(cudaMemcpy(plan.d_tasks, plan.h_tasks.data(), plan.h_tasks.size() * sizeof(TermTask), cudaMemcpyHostToDevice));
   if (!plan.h_down.empty())
     CK(cudaMemcpy(plan.d_down, plan.h_down.data(), plan.h_down.size() * sizeof(DownTask), cudaMemcpyHostToDevice));
   if (!plan.h_up.empty())
     CK(cudaMemcpy(plan.d_up, plan.h_up.data(), plan.h_up.size() * sizeof(UpTask), cudaMemcpyHostToDevice));
-  if (!plan.h_groups.empty())
-    CK(cudaMemcpy(plan.d_groups, plan.h_groups.data(), plan.h_groups.size() * sizeof(TermGroup),
-                  cudaMemcpyHostToDevice));
-  if (!plan.h_lanes.empty())
-    CK(cudaMemcpy(plan.d_lanes, plan.h_lanes.data(), plan.h_lanes.size() * sizeof(TermLane), cudaMemcpyHostToDevice));
   return Status();
 }
 
@@ -1262,37 +1154,6 @@ void Engine::row_args(int p, RowArgs& A) const {
   A.p = p;
 }
 
-void Engine::term_args(int p, TermArgs& A) const {
-  A.reach = reach_;
-  A.vals = vals_;
-  A.alive = alive(p);
-  A.warp_scratch = warp_scratch_;
-  A.warp_scratch_floats = warp_scratch_floats_;
-  A.group_scratch = group_scratch_;
-  A.counters = counters_;
-  A.tables = tables_;
-  A.table_count = table_count_;
-  A.progs = progs_;
-  A.prog_count = prog_count_;
-  A.posmap = posmap_;
-  for (int q = 0; q < 2; q++) {
-    A.fold_prog[q] = fold_prog_[q];
-    A.emit_rec[q] = emit_rec_[q];
-  }
-  A.pstride = pstride_;
-  for (int q = 0; q < 2; q++) {
-    A.hc1[q] = hc1_[q];
-    A.hc2[q] = hc2_[q];
-    A.same[q] = same_[q];
-    A.n[q] = g.n[q];
-    A.hp[q] = hp_[q];
-  }
-  A.stride = stride_;
-  A.tstride = tstride_;
-  A.nmax = tstride_;
-  A.p = p;
-}
-
 void Engine::fast_args(int p, FastArgs& A) const {
   A.reach = reach_;
   A.vals = vals_;
@@ -1406,11 +1267,10 @@ void Engine::enqueue_terminals(const Plan& plan) {
       else
         launch_fast_terminal(F, plan.d_fast, (int)plan.h_fast.size(), fast_blocks_, stream_);
     }
-  } else if (!plan.waves.empty()) {
-    TermArgs T;
-    term_args(p, T);
-    for (const Plan::Wave& w : plan.waves)
-      launch_terminal(T, plan.d_groups, plan.d_lanes, plan.d_tasks + w.first, (int)w.count, stream_);
+  } else if (!plan.h_fast.empty()) {
+    FastArgs F;
+    fast_args(p, F);
+    launch_exact_terminal(F, plan.d_fast, (int)plan.h_fast.size(), (uint32_t)g.boards.size(), exact_blocks_, stream_);
   }
   enqueue_leaves(plan);
   mark(DCFR_KERNEL_TERMINAL);
@@ -2304,12 +2164,6 @@ Status Engine::subtree_values(uint32_t root, int p, const std::vector<float>& op
   Plan plan;
   Status s;
   if (!(s = build_plan(root, p, plan)).ok()) return s;
-  for (const Plan::Wave& w : plan.waves)
-    if (!fast_ && ((int)w.count > wave_tasks_ || (int)w.groups > wave_groups_)) {
-      s.code = DCFR_ERR_INVALID_ARG;
-      s.msg = "subtree plan exceeds the terminal scratch";
-      return s;
-    }
   if (plan.nslots > max_slots_) {
     s.code = DCFR_ERR_INVALID_ARG;
     s.msg = "subtree plan exceeds the reach buffer";

@@ -17,7 +17,6 @@ struct dcfr_mlp;
 namespace dcfr {
 
 struct RowArgs;
-struct TermArgs;
 
 // Kernel launchers (kernels.cu).
 void launch_down(int mode, int maxa, const RowArgs& A, const DownTask* tasks, int ntasks, int hp, cudaStream_t s);
@@ -30,14 +29,9 @@ void launch_fused_up(int mode, int maxa, const RowArgs& A, const FusedTree* tree
 cudaError_t segment_setup();
 size_t segment_smem(const SegPass& P);
 void launch_segment(int mode, int maxa, const SegPass& P, cudaStream_t s);
-void launch_terminal(const TermArgs& A, const TermGroup* groups, const TermLane* lanes, const TermTask* tasks,
-                     int ntasks, cudaStream_t s);
-cudaError_t terminal_kernel_setup();
-size_t terminal_smem_bytes();
-void launch_programs(const EntryD* tables, const uint32_t* count, int tstride, uint32_t* progs, uint32_t* prog_count,
-                     uint32_t* posmap, int pstride, int nboards, cudaStream_t s);
-void launch_hand_program(const uint8_t* c1, const uint8_t* c2, const uint32_t* same, int n, int npad,
-                         uint32_t* fold_prog, uint2* emit_rec, cudaStream_t s);
+int exact_terminal_setup(int stride, int cstride, int tstride);
+void launch_exact_terminal(const FastArgs& A, const FastTask* tasks, int ntasks, uint32_t fold_layout, int max_blocks,
+                           cudaStream_t s);
 void launch_strength(const uint8_t* boards, int nboards, const uint8_t* hc1_0, const uint8_t* hc2_0,
                      const uint8_t* hc1_1, const uint8_t* hc2_1, int n0, int n1, EntryD* out, uint32_t* count,
                      int tstride, cudaStream_t s);
@@ -109,10 +103,7 @@ struct Plan {
   std::vector<std::vector<Level>> seg_down, seg_up;  // wide segments: [layer][depth]
   std::vector<DownTask> h_down;
   std::vector<UpTask> h_up;
-  std::vector<TermGroup> h_groups;
-  std::vector<TermLane> h_lanes;
-  std::vector<TermTask> h_tasks;
-  std::vector<FastTask> h_fast;  // fast precision: one task per terminal
+  std::vector<FastTask> h_fast;  // one task per terminal
   std::vector<TermUnit> h_units; // runs of h_fast on one layout (warp terminal kernel)
   TermUnit* d_units = nullptr;
   std::vector<PanelD> h_panels;  // panels of h_fast (panel terminal kernel)
@@ -136,15 +127,8 @@ struct Plan {
   FusedTree* d_trees = nullptr;
   DownTask* d_fdown = nullptr;
   UpTask* d_fup = nullptr;
-  struct Wave {
-    uint32_t first = 0, count = 0, groups = 0;
-  };
-  std::vector<Wave> waves;
-  TermTask* d_tasks = nullptr;
   DownTask* d_down = nullptr;
   UpTask* d_up = nullptr;
-  TermGroup* d_groups = nullptr;
-  TermLane* d_lanes = nullptr;
   FastTask* d_fast = nullptr;
   int kernels = 0;  // kernel launches per traversal
   int class_kernels[DCFR_KERNEL_CLASSES] = {0, 0, 0, 0};
@@ -280,17 +264,7 @@ class Engine {
   EntryD* tables_ = nullptr;
   uint32_t* table_count_ = nullptr;
   int tstride_ = 0;
-  uint32_t* progs_ = nullptr;
-  uint32_t* prog_count_ = nullptr;
-  uint32_t* posmap_ = nullptr;
-  uint32_t* fold_prog_[2] = {nullptr, nullptr};
-  uint2* emit_rec_[2] = {nullptr, nullptr};
-  int pstride_ = 0;
-  float* warp_scratch_ = nullptr;
-  size_t warp_scratch_floats_ = 0;
-  double* group_scratch_ = nullptr;
-  uint32_t* counters_ = nullptr;
-  int wave_tasks_ = 0, wave_groups_ = 0;
+  int exact_blocks_ = 0;  // exact precision: blocks of the terminal kernel
   // Fast precision (terminal_fast.cu): scan layouts per (layout, traverser).
   bool fast_ = true;
   uint16_t* fcat_ = nullptr;
@@ -371,7 +345,6 @@ class Engine {
   SegPass segment_pass(const Plan* up, const Plan* down) const;
   static void drop_segment(Plan& plan);
   void row_args(int p, RowArgs& A) const;
-  void term_args(int p, TermArgs& A) const;
   void fast_args(int p, FastArgs& A) const;
   uint32_t* alive(int p) const { return alive_ + (size_t)p * max_slots_; }
   void enqueue_traversal(const Plan& plan, int mode, const float* root_row, float* root_out, bool advance = false);

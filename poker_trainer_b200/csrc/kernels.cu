@@ -8,7 +8,7 @@
 //     128-bit loads and stores; all their arithmetic is per hand;
 //   * chance sums accumulate children in f64 in card order, then the
 //     isomorphic cards through the suit permutation (cfr.rs:462-478);
-//   * terminal values are in terminal.cu.
+//   * terminal values are in terminal.cu (exact) and terminal_fast.cu.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -5,8 +5,7 @@
 //   down levels  — opponent nodes split the opponent reach by their
 //                  strategy (regret matching + strategy-sum update in CFR
 //                  mode), chance nodes fan the reach out per dealt card;
-//   terminals    — fold and showdown values of every live terminal, one
-//                  warp per group of up to 32 terminals;
+//   terminals    — fold and showdown values of every live terminal;
 //   up levels    — deepest first: traverser nodes combine child values
 //                  (and update regrets), opponent nodes and chance nodes sum.
 // Reach rows live in "slots" (a traverser node's children share its slot);
@@ -21,8 +20,6 @@ namespace dcfr {
 constexpr int VEC = 4;             // hands per thread in the row kernels (float4)
 constexpr int ROW_MAX_THREADS = 352;  // row-kernel block: a thread per 4 hands, whole warps (1328 hands max)
 constexpr int MAX_ACTIONS = 16;
-constexpr int TERM_WARPS = 4;      // warps per terminal-kernel block
-constexpr int TERM_CHUNK = 32;     // sweep steps staged per cp.async batch
 constexpr uint32_t NONE32 = 0xFFFFFFFFu;
 
 enum DownKind : uint32_t { D_OPP_SPLIT = 0, D_CHANCE_SPLIT = 1 };
@@ -81,26 +78,6 @@ struct TermLane {
   double b;       // showdown lose
   double c;       // showdown tie
   double d;       // paired fold payoff
-};
-
-// One warp's work in the terminal kernel: a fold group, or one of the
-// passes of a showdown group (ascending win part, descending lose part,
-// paired fold). wgroup indexes the per-launch win/lose scratch and counter.
-enum TermRole : uint32_t { R_FOLD = 0, R_ASC = 1, R_DESC = 2, R_PAIRED = 3 };
-struct TermTask {
-  uint32_t role;
-  uint32_t group;
-  uint32_t wgroup;
-  uint32_t pad;
-};
-constexpr int MAX_WAVE_TASKS = 1024;   // warps per terminal launch
-constexpr int MAX_WAVE_GROUPS = 384;   // showdown groups per terminal launch
-
-struct TermGroup {
-  uint32_t kind;
-  uint32_t board;  // showdown strength table
-  uint32_t first;  // first lane in the lane array
-  uint32_t count;  // lanes used (1..32)
 };
 
 // Strength-table entry (eval::Entry, crates/solver/src/eval.rs:11-18).
@@ -300,34 +277,6 @@ struct Row64Args {
   int n[2];
   int hp[2];
   int stride;
-  int p;
-};
-
-// Arguments of the terminal kernel.
-struct TermArgs {
-  const float* reach;
-  float* vals;
-  const uint32_t* alive;
-  float* warp_scratch;          // per warp: Rp [pstride+1][32], O [stride][32]
-  size_t warp_scratch_floats;
-  double* group_scratch;        // per showdown group: win and lose parts [2][nmax][32]
-  uint32_t* counters;           // per showdown group: passes finished
-  const EntryD* tables;
-  const uint32_t* table_count;
-  const uint32_t* progs;        // [((board*2+p)*3+dir)][pstride] sweep programs
-  const uint32_t* prog_count;   // steps per program (a multiple of TERM_CHUNK)
-  const uint32_t* posmap;       // [((board*2+p)*3+dir)][tstride] opponent hand -> step
-  const uint32_t* fold_prog[2]; // each player's hands in hand order as steps
-  const uint2* emit_rec[2];     // per hand: blocker rows word, identical opponent hand
-  int pstride;
-  const uint8_t* hc1[2];
-  const uint8_t* hc2[2];
-  const uint32_t* same[2];
-  int n[2];
-  int hp[2];
-  int stride;
-  int tstride;
-  int nmax;
   int p;
 };
 
