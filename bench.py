@@ -723,20 +723,12 @@ def run_batch(args, world, rank, local):
     it_bytes_all = grp.reduce(it_bytes, "sum")
     value = S_total * K / (ms / 1000.0)
     peak, peak_kind = measured_peak()
-    # The persistent kernel is the only kernel of the timed region: its
-    # algorithmic bytes per launch are every spot's B_iter times the
-    # iterations per launch; the committed ncu traffic is for 10 iterations
-    # per launch and scales with that count.
-    ipl = max(int(tuned.iterations_per_launch), 1)
-    n_launch = max(int(launches), 1)
-    per_launch_ms = ms / n_launch
-    per_launch_bytes = it_bytes * K / n_launch
-    traffic = ncu_traffic("batch_kernel", "batch")
-    roof = {"bound": "hbm", "kernel": "batch_kernel",
-            "achieved": per_launch_bytes / (per_launch_ms / 1000.0) / 1e9 if per_launch_ms > 0 else 0.0,
-            "peak": peak, "unit": "GB/s", "peak_kind": f"of {peak_kind}",
-            "traffic": traffic * ipl / 10.0 if traffic else None,
-            "bytes_per_launch": per_launch_bytes, "ms_per_launch": per_launch_ms}
+    # An iteration is a fixed sequence of launches over all spots; the roofline
+    # is the sequence's: every spot's B_iter over its device time.
+    roof = {"bound": "hbm", "kernel": "batch iteration (row passes and terminals)",
+            "achieved": it_bytes * K / (ms / 1000.0) / 1e9 if ms > 0 else 0.0,
+            "peak": peak, "unit": "GB/s", "peak_kind": f"of {peak_kind}", "traffic": None,
+            "bytes_per_launch": it_bytes * K / max(int(launches), 1), "ms_per_launch": ms / max(int(launches), 1)}
     roof["frac"] = roof["achieved"] / peak
     cpu = None
     if world == 1 and not args.no_cpu_baseline and rank == 0:

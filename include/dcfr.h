@@ -421,16 +421,15 @@ int dcfr_iterate_profiled(dcfr_solver* s, uint32_t iterations, dcfr_kernel_profi
  * Many independent river spots (5-card board, river root, fast precision,
  * one shared DcfrParams) solved together: each DCFR iteration of every spot
  * is the same as a single dcfr_create/dcfr_iterate solve of that spot, done
- * by one persistent kernel per block of iterations launched from a captured
- * CUDA graph; spots of uneven tree size are taken from a work counter,
- * longest first. */
+ * by a few launches over all of them from a captured CUDA graph; spots of
+ * uneven tree size are taken longest first. */
 typedef struct dcfr_batch dcfr_batch;
 
 /* Launch shape of the batched kernel, chosen by dcfr_batch_autotune. */
 typedef struct dcfr_batch_tuning {
-  int32_t warps;                  /* warps per block (each evaluates terminals) */
+  int32_t warps;                  /* terminals in flight per block */
   int32_t blocks_per_sm;          /* resident blocks per SM (grid = SMs x this) */
-  uint32_t iterations_per_launch; /* iterations of a spot per persistent launch */
+  uint32_t iterations_per_launch; /* iterations per launched graph */
   int32_t longest_first;          /* 1: spots taken by decreasing work; 0: input order */
   int32_t candidates;             /* autotune: candidates timed */
   int32_t _pad;

@@ -1,5 +1,5 @@
 // Batched river solves (batch.cu): many independent river spots solved
-// together by one persistent kernel per block of iterations.
+// together, a few launches an iteration over all of them.
 #pragma once
 
 #include <cstdint>

@@ -47,7 +47,8 @@ void launch_warp_terminal64(const FastArgs64& A, const FastTask* tasks, const Te
                             int warps,
                             int max_blocks, cudaStream_t s);
 int warp_terminal_setup(int stride, int cstride, int tstride, int rsize, int max_warps, int& blocks_per_sm);
-int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm);
+int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm, bool multi = false);
+int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, bool multi);
 void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
                            int groups, int max_blocks, cudaStream_t s);
 int panel_terminal_setup(int hpo, int hpp, int cstride, int tstride, int T, int& blocks_per_sm);

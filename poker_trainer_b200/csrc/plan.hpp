@@ -171,6 +171,9 @@ struct FastArgsT {
   const uint16_t* seg;   // [(layout*2+p)][FAST_SEGS]
   const uint4* rec;      // [(layout*2+p)][tstride]
   const uint32_t* same;  // traverser hand -> identical opponent hand (or NONE32)
+  // A batch's spots (layout 2 * spot): {n0, n1, hp0, hp1} of each, and `same`
+  // has rows of `stride` per (spot, traverser). Null: one game, n and hp.
+  const int4* dims = nullptr;
   int cstride;
   int tstride;
   int emax;              // elements per thread (odd) for the largest layout

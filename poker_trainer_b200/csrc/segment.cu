@@ -36,6 +36,7 @@
 #include "pdl.cuh"
 #include "plan.hpp"
 #include "row_items.cuh"
+#include "segment.cuh"
 
 namespace dcfr {
 
@@ -79,27 +80,6 @@ __device__ __forceinline__ void copies_landed() {
 
 __device__ __forceinline__ void stage(unsigned char* dst, const unsigned char* src, uint32_t bytes) {
   for (uint32_t i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16) copy16(dst + i, src + i);
-}
-
-// Strategy from regrets (regret_match_into, cfr.rs:161-192) or from strategy
-// sums (normalize_in_place, cfr.rs:124-154), in place.
-template <int MAXA, bool REGRETS>
-__device__ __forceinline__ void to_strategy(float (&x)[MAXA], int na, float uniform) {
-#pragma unroll
-  for (int a = 0; a < MAXA; a++)
-    if (REGRETS) x[a] = max0(x[a]);
-  float s = x[0];
-#pragma unroll
-  for (int a = 1; a < MAXA; a++) s = a < na ? s + x[a] : s;
-  const float inv = recipf(s);
-#pragma unroll
-  for (int a = 0; a < MAXA; a++) x[a] = inv == 0.0f ? uniform : x[a] * inv;
-}
-
-// Strategy sum after an iteration (cfr.rs:395-407).
-__device__ __forceinline__ float next_sum(float s, float sigma, float r, const DiscountD& d) {
-  const float add = d.reach_weighted ? sigma * r : sigma;
-  return s * d.strat + add;
 }
 
 template <int MODE, int MAXA>
@@ -240,22 +220,11 @@ __global__ void __launch_bounds__(SEG_WARPS * 32, 2) segment_kernel(const __grid
           float r[MAXA];
 #pragma unroll
           for (int a = 0; a < MAXA; a++) r[a] = reg[(T.store + min(a, na - 1)) * SEG_SLICE + lane];
-          float s = max0(r[0]);
-#pragma unroll
-          for (int a = 1; a < MAXA; a++) s = a < na ? s + max0(r[a]) : s;
-          const float iv = recipf(s);
-          float m = -0.0f;
-#pragma unroll
-          for (int a = 0; a < MAXA; a++) {
-            out = a < na ? out + max0(r[a]) * v[a] : out;
-            m = a < na ? m + v[a] : m;
-          }
-          out = iv == 0.0f ? m * T.uniform : out * iv;
+          own_value<MAXA>(r, v, na, T.uniform, out);
           float* to = P.up.regrets + T.gstore + h;
 #pragma unroll
           for (int a = 0; a < MAXA; a++) {
-            const float disc = r[a] > 0.0f ? d.pos : d.neg;
-            const float x = r[a] * disc + v[a] - out;
+            const float x = next_regret(r[a], v[a], out, d);
             if (a < na) {
               reg[(T.store + a) * SEG_SLICE + lane] = x;
               if (valid) to[(size_t)a * hp] = x;

@@ -166,7 +166,9 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   uint16_t* sseg = reinterpret_cast<uint16_t*>(smem_fast + L_.seg);
 
   const int p = A.p, o = p ^ 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
+  int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
+  const bool multi = sizeof(R) == 4 && A.dims != nullptr;  // a batch's spots (FastArgsT::dims)
+  const int fetch = multi ? A.stride : hpo;
   __shared__ int s_claim[2];  // DYN: the first chunk, then the chunk after the current one
   int t0, t1;
   if constexpr (DYN) {
@@ -182,14 +184,17 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   if (t0 >= t1) return;
   int cbeg = t0, cend = min(t1, t0 + FAST_DYN_CHUNK), claimed = t1;  // DYN: current chunk, next chunk
 
-  for (int h = tid; h < hpp; h += FAST_THREADS) {
-    const uint32_t sm = h < np ? A.same[h] : NONE32;
-    ssame[h] = sm == NONE32 ? (uint16_t)0xFFFF : (uint16_t)sm;
-  }
+  auto stage_same = [&](const uint32_t* same) {
+    for (int h = tid; h < hpp; h += FAST_THREADS) {
+      const uint32_t sm = h < np ? same[h] : NONE32;
+      ssame[h] = sm == NONE32 ? (uint16_t)0xFFFF : (uint16_t)sm;
+    }
+  };
+  if (!multi) stage_same(A.same);
   auto prefetch = [&](int ti, int buf) {
     const R* src = A.reach + (size_t)tasks[ti].slot * A.stride;
     R* dst = rbuf + (size_t)buf * A.stride;
-    for (int i = tid; i < hpo / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
+    for (int i = tid; i < fetch / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
     cp_async_commit();
   };
   uint32_t board = NONE32;
@@ -198,6 +203,13 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   auto stage = [&](uint32_t b) {
     board = b;
     const size_t lay = (size_t)board * 2 + p;
+    if (multi) {
+      const int4 d = A.dims[board >> 1];
+      np = p ? d.y : d.x;
+      hpp = p ? d.w : d.z;
+      hpo = o ? d.w : d.z;
+      stage_same(A.same + ((size_t)(board >> 1) * 2 + p) * A.stride);
+    }
     const uint16_t* gseg = A.seg + lay * FAST_SEGS;
     if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
     L = gseg[FAST_SEGS - 1];
@@ -233,7 +245,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
         mx = row_max(mx, row_max(v.x, v.y));
       }
     } else {
-      for (int i = tid; i < hpo / 4; i += FAST_THREADS) {
+      for (int i = tid; i < fetch / 4; i += FAST_THREADS) {
         const float4 v = reinterpret_cast<const float4*>(r)[i];
         mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
       }

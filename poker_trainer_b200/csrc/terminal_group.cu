@@ -68,8 +68,7 @@ __device__ __forceinline__ void group_sync(int id) {
 // The group's threads copy the row of `slot` in 16-byte chunks: thread gt
 // takes chunks gt, gt + GROUP_THREADS, ... (the same chunks it reads back
 // for its part of the row maximum).
-__device__ __forceinline__ void group_row_prefetch(const FastArgs& A, uint32_t slot, float* row, int gt) {
-  const int hpo = (A.p ^ 1) ? A.hp[1] : A.hp[0];
+__device__ __forceinline__ void group_row_prefetch(const FastArgs& A, int hpo, uint32_t slot, float* row, int gt) {
   const char* src = reinterpret_cast<const char*>(A.reach + (size_t)slot * A.stride);
   const uint32_t dst = (uint32_t)__cvta_generic_to_shared(row);
   for (int i = gt; i < hpo / 4; i += GROUP_THREADS)
@@ -80,14 +79,13 @@ __device__ __forceinline__ void group_row_prefetch(const FastArgs& A, uint32_t s
 // One terminal task evaluated by the GROUP_THREADS threads of a group (gt
 // = thread in the group). row: the group's copy of the task's reach row, its
 // own chunks waited for by every thread. next_slot / next_row: the row to
-// request after barrier (1) (NONE32: none). bfirst: the first segment
+// request after barrier (1) (NONE32: none), `fetch` entries of it. bfirst: the first segment
 // boundary b >= 1 with seg[b] >= this thread's first scan element.
-__device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T, const WarpLayout& Y, const float* row,
-                                           long long* G, long long* cst, long long* gsum, float* gmax, int gt, int bar,
-                                           int bfirst, uint32_t next_slot, float* next_row) {
+__device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T, const WarpLayout& Y, int hpo, int hpp,
+                                           int np, int fetch, const float* row, long long* G, long long* cst,
+                                           long long* gsum, float* gmax, int gt, int bar, int bfirst,
+                                           uint32_t next_slot, float* next_row) {
   const int lane = gt & 31, w = gt >> 5;
-  const int p = A.p, o = p ^ 1;
-  const int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
   const int L = Y.L;
   // 1. Row maximum: each thread's own copied chunks, then the group's.
   float mx = 0.0f;
@@ -99,7 +97,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   if (lane == 0) gmax[w] = mx;
   group_sync(bar);  // (1)
-  if (next_slot != NONE32) group_row_prefetch(A, next_slot, next_row, gt);
+  if (next_slot != NONE32) group_row_prefetch(A, fetch, next_slot, next_row, gt);
   cp_async_commit();
 #pragma unroll
   for (int k = 0; k < GROUP_WARPS; k++) mx = fmaxf(mx, gmax[k]);
@@ -267,6 +265,10 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
 // tasks g, g + NG, ...). The block stages a unit's layout (a maximal run of
 // tasks on one layout) once, with a block barrier only where its range
 // crosses from one unit to the next.
+// MULTI: a batch's spots, a unit each: the players' hand counts and the
+// identical-hand map change with the unit, and rows are fetched to their
+// common stride (a spot's entries past its own hands are zero).
+template <bool MULTI>
 __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
     group_terminal_kernel(FastArgs A, const FastTask* __restrict__ tasks, const TermUnit* __restrict__ units,
                           int nunits, int ntasks) {
@@ -287,12 +289,16 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   float* gmax = reinterpret_cast<float*>(gb + L_.red_off + GROUP_WARPS * 8);
   const int bar = 1 + grp;
 
-  const int p = A.p;
-  const int hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
-  for (int h = tid; h < hpp; h += blockDim.x) {
-    const uint32_t sm = h < np ? A.same[h] : NONE32;
-    ssame[h] = sm == NONE32 ? (uint16_t)0xFFFF : (uint16_t)sm;
-  }
+  const int p = A.p, o = p ^ 1;
+  int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
+  const int fetch = MULTI ? A.stride : hpo;
+  auto stage_same = [&](const uint32_t* same) {
+    for (int h = tid; h < hpp; h += blockDim.x) {
+      const uint32_t sm = h < np ? same[h] : NONE32;
+      ssame[h] = sm == NONE32 ? (uint16_t)0xFFFF : (uint16_t)sm;
+    }
+  };
+  if (!MULTI) stage_same(A.same);
   const int t0 = (int)(((long long)blockIdx.x * ntasks) / gridDim.x);
   const int t1 = (int)(((long long)(blockIdx.x + 1) * ntasks) / gridDim.x);
   int u = 0;
@@ -307,6 +313,13 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   int L = 0;
   auto stage = [&](uint32_t layout) {
     const size_t lay = (size_t)layout * 2 + p;
+    if (MULTI) {
+      const int4 d = A.dims[layout >> 1];
+      np = p ? d.y : d.x;
+      hpp = p ? d.w : d.z;
+      hpo = o ? d.w : d.z;
+      stage_same(A.same + ((size_t)(layout >> 1) * 2 + p) * A.stride);
+    }
     const uint16_t* gseg = A.seg + lay * FAST_SEGS;
     if (tid < FAST_SEGS) sseg[tid] = gseg[tid];
     L = gseg[FAST_SEGS - 1];
@@ -325,7 +338,7 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   bool live = false;
   if (next < t1) {
     live = A.alive[tasks[next].slot] != 0;
-    if (live) group_row_prefetch(A, tasks[next].slot, row_a, gt);
+    if (live) group_row_prefetch(A, fetch, tasks[next].slot, row_a, gt);
   }
   cp_async_commit();
   for (; u < nunits && (int)units[u].first < t1; u++) {
@@ -349,14 +362,14 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
       float* const nxt_row = buf ? row_a : row_b;
       // Dead subtree (cfr.rs:267-274): row untouched.
       if (live) {
-        group_task(A, tasks[next], Y, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
+        group_task(A, tasks[next], Y, hpo, hpp, np, fetch, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
                    nlive ? tasks[nx].slot : NONE32, nxt_row);
       } else {
         // The group's other warps may still read the previous task's row
         // from the buffer the next row goes to.
         if (nlive) {
           group_sync(bar);
-          group_row_prefetch(A, tasks[nx].slot, nxt_row, gt);
+          group_row_prefetch(A, fetch, tasks[nx].slot, nxt_row, gt);
         }
         cp_async_commit();
       }
@@ -371,15 +384,25 @@ size_t group_terminal_smem(int stride, int cstride, int tstride, int groups) {
   return GroupSmem(stride, cstride, tstride, groups).total;
 }
 
+// Resident blocks per SM of `groups` groups; 0 if none fits.
+int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, bool multi) {
+  int b = 0;
+  const void* fn = multi ? (const void*)group_terminal_kernel<true> : (const void*)group_terminal_kernel<false>;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, groups * GROUP_THREADS,
+                                                    group_terminal_smem(stride, cstride, tstride, groups)) != cudaSuccess)
+    return 0;
+  return b;
+}
+
 // Groups per block (1..GROUP_MAX) that maximise resident groups per SM, and
 // the blocks per SM at that count; 0 if none fits.
-int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm) {
+int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm, bool multi) {
   int dev = 0, optin = 0;
   blocks_per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return 0;
-  const void* fn = (const void*)group_terminal_kernel;
+  const void* fn = multi ? (const void*)group_terminal_kernel<true> : (const void*)group_terminal_kernel<false>;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return 0;
   int best_g = 0, best_b = 0;
   for (int g = 1; g <= GROUP_MAX; g++) {
@@ -402,8 +425,8 @@ void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermU
   // At most one block per task: every block's range is non-empty.
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
   const size_t smem = group_terminal_smem(A.stride, A.cstride, A.tstride, groups);
-  launch_dependent(group_terminal_kernel, (unsigned)blocks, (unsigned)(groups * GROUP_THREADS), smem, s, A, tasks, units,
-                   nunits, ntasks);
+  launch_dependent(A.dims ? group_terminal_kernel<true> : group_terminal_kernel<false>, (unsigned)blocks,
+                   (unsigned)(groups * GROUP_THREADS), smem, s, A, tasks, units, nunits, ntasks);
 }
 
 }  // namespace dcfr

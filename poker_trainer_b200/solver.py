@@ -516,7 +516,7 @@ class Solver:
 
 class BatchSolver:
     """Batched river solves (dcfr_batch_*): many independent river spots
-    solved together by a persistent kernel under a captured CUDA graph."""
+    solved together, a few launches an iteration under a captured CUDA graph."""
 
     def __init__(self, handle, count):
         self._h = handle
