@@ -184,7 +184,8 @@ Engine::~Engine() {
     dfree(leaf_reach_[q]);
     dfree(combos_[q]);
   }
-  dfree(leaf_x_);
+  dfree(leaf_mass_);
+  dfree(leaf_shift_);
   dfree(leaf_cards_);
   dfree(sblk_);
   dfree(reach64_);
@@ -1376,8 +1377,8 @@ Status Engine::init_leaves() {
     if (!(s = dalloc(combos_[q], cb.size(), "leaf combos")).ok()) return s;
     CK(cudaMemcpy(combos_[q], cb.data(), cb.size() * 2, cudaMemcpyHostToDevice));
   }
-  if (!(s = dalloc(leaf_x_, (size_t)std::max(L, 1) * leaf_nc_ * (2 * DCFR_NUM_COMBOS + 54), "leaf inputs")).ok())
-    return s;
+  if (!(s = dalloc(leaf_mass_, (size_t)std::max(L, 1) * 2, "leaf masses")).ok()) return s;
+  if (!(s = dalloc(leaf_shift_, (size_t)std::max(L, 1) * leaf_nc_, "leaf masses")).ok()) return s;
   if (!(s = dalloc(leaf_cards_, cards.size(), "leaf cards")).ok()) return s;
   CK(cudaMemcpy(leaf_cards_, cards.data(), cards.size(), cudaMemcpyHostToDevice));
   for (int p = 0; p < 2; p++)
@@ -1399,7 +1400,9 @@ void Engine::enqueue_leaves(const Plan& plan) {
     A.combos[q] = combos_[q];
     A.n[q] = g.n[q];
   }
-  A.x = leaf_x_;
+  A.mass = leaf_mass_;
+  A.shift = leaf_shift_;
+  A.x = mlp_input(net_, &A.ldx);
   A.y = nullptr;
   A.ldy = 0;
   A.cards = leaf_cards_;
@@ -1410,11 +1413,10 @@ void Engine::enqueue_leaves(const Plan& plan) {
   A.factor = leaf_factor_;
   A.norm = g.norm;
   const int nl = (int)plan.h_leaves.size();
-  launch_leaf_capture(A, plan.d_leaves, nl, stream_);
   launch_leaf_inputs(A, plan.d_leaves, nl, hc1_[0], hc2_[0], hc1_[1], hc2_[1], stream_);
   const float* y = nullptr;
   int ldy = 0;
-  if (mlp_enqueue_forward(net_, leaf_x_, (int)g.leaves.size() * leaf_nc_, stream_, &y, &ldy) != DCFR_OK) {
+  if (mlp_enqueue_forward(net_, (int)g.leaves.size() * leaf_nc_, stream_, &y, &ldy) != DCFR_OK) {
     leaf_status_ = Status{DCFR_ERR_CUDA, "leaf network forward pass failed"};
     return;
   }

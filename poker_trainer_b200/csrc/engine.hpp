@@ -2,6 +2,7 @@
 // the per-traversal plans and the captured CUDA graphs of one solver handle.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -138,6 +139,14 @@ struct Plan {
   ~Plan();
 };
 
+// One side's reach at a leaf (leaf.cu): in combo order, its total, and that of
+// the hands holding each card.
+struct LeafMass {
+  double total;
+  double card[52];
+  float reach[DCFR_NUM_COMBOS];
+};
+
 // Leaf evaluation of depth-limited solves (leaf.cu).
 struct LeafArgs {
   const float* reach;       // reach rows (slots x stride)
@@ -145,7 +154,10 @@ struct LeafArgs {
   const uint32_t* alive;
   float* leaf_reach[2];     // per player: its reach at each leaf [leaves][stride], hand order
   const uint16_t* combos[2];// per player: combo id of each hand
-  float* x;                 // network input [leaves * nc][in_dim]
+  LeafMass* mass;           // [leaves][2]: opponent, traverser
+  double* shift;            // [leaves][nc]: zero-sum shift of each card's values
+  __nv_bfloat16* x;         // network input [leaves * nc][ldx], as the network packs it
+  int ldx;
   const float* y;           // network output, row stride ldy: EV / pot per combo, player 0 then 1
   int ldy;
   const uint8_t* cards;     // the nc cards dealt at the leaves (ascending)
@@ -157,15 +169,16 @@ struct LeafArgs {
   float factor;             // chance factor of the leaf's deal (tree.rs:520-542)
   double norm;              // 1 / num_combinations
 };
-void launch_leaf_capture(const LeafArgs& A, const LeafTask* tasks, int ntasks, cudaStream_t s);
 void launch_leaf_inputs(const LeafArgs& A, const LeafTask* tasks, int ntasks, const uint8_t* hc1_0,
                         const uint8_t* hc2_0, const uint8_t* hc1_1, const uint8_t* hc2_1, cudaStream_t s);
 void launch_leaf_values(const LeafArgs& A, const LeafTask* tasks, int ntasks, const uint8_t* hc1_p,
                         const uint8_t* hc2_p, const uint8_t* hc1_o, const uint8_t* hc2_o, int hp, cudaStream_t s);
-// The leaf-value network (mlp.cu): shape check, and a forward pass enqueued on
-// stream s (no synchronisation) whose padded output y has row stride ldy.
+// The leaf-value network (mlp.cu): shape check, its packed input rows (bf16,
+// row stride ldx), and a forward pass on m of them enqueued on stream s (no
+// synchronisation) whose padded output y has row stride ldy.
 int mlp_shape(const dcfr_mlp* n, int* in_dim, int* out_dim, int* max_batch);
-int mlp_enqueue_forward(dcfr_mlp* n, const float* x, int m, cudaStream_t s, const float** y, int* ldy);
+__nv_bfloat16* mlp_input(dcfr_mlp* n, int* ldx);
+int mlp_enqueue_forward(dcfr_mlp* n, int m, cudaStream_t s, const float** y, int* ldy);
 
 class Engine {
  public:
@@ -290,7 +303,8 @@ class Engine {
   // Depth-limited solves: the leaf-value network and its buffers.
   dcfr_mlp* net_ = nullptr;
   float* leaf_reach_[2] = {nullptr, nullptr};
-  float* leaf_x_ = nullptr;
+  LeafMass* leaf_mass_ = nullptr;
+  double* leaf_shift_ = nullptr;
   uint8_t* leaf_cards_ = nullptr;
   uint16_t* combos_[2] = {nullptr, nullptr};
   int leaf_nc_ = 0;

@@ -4,15 +4,26 @@
 //   C[M][N] = epilogue( sum_k A[M][K] * B[N][K] )
 //
 // A and B are row-major with K contiguous (both operands "K-major"). One CTA
-// computes a 128 x 128 tile of C:
-//   * warp 0, one thread: TMA loads of 128 x 64 tiles of A and B into a
-//     GEMM_STAGES-deep shared-memory ring (128-byte swizzle, the canonical
+// computes a 128 x BN tile of C:
+//   * warp 0, one thread: TMA loads of 128 x 64 tiles of A and BN x 64 tiles of
+//     B into a ring of STAGES in shared memory (128-byte swizzle, the canonical
 //     K-major layout the tensor core reads);
-//   * warp 1, one thread: tcgen05.mma (M=128, N=128, K=16 per instruction,
+//   * warp 1, one thread: tcgen05.mma (M=128, N=BN, K=16 per instruction,
 //     FP32 accumulator in tensor memory), a tcgen05.commit per stage frees
 //     the stage, a last commit marks the accumulator complete;
-//   * all four warps: the epilogue reads the accumulator with tcgen05.ld
-//     (warp w owns rows 32w..32w+31) and writes C through the epilogue.
+//   * all eight warps: the epilogue reads the accumulator with tcgen05.ld
+//     (warp w owns rows 32 (w % 4) on, and half the columns) and writes C
+//     through the epilogue.
+// The tile and the ring depend on how many CTAs a product gives (gemm_shape):
+// the network's products at a few hundred rows are a few dozen 128 x 128
+// tiles, bound by the ring's latency (a TMA round trip is about 1 us, a
+// 64-deep step of the tile a tenth of that) and, with GELU, by the epilogue.
+// Narrower tiles put more SMs to work on both, and a CTA that has an SM to
+// itself takes a ring twice as deep. us a launch, against 128 x 128 tiles with
+// 3 stages and 4 warps throughout: 896 x 1024 x 2816 with GELU 44.8 to 18.7,
+// 896 x 1024 x 1024 37.1 to 10.9, 256 x 1024 x 2816 41.3 to 17.4, 256 x 1024 x
+// 1024 33.0 to 9.4, 896 x 2688 x 1024 with bias 18.2 to 12.4; 8192 x 1024 x 2816
+// with GELU 105.7 to 60.0, plain 4096 x 1024 x 2816 28.4 to 27.6.
 // Every wait on an mbarrier is bounded; a wait that gives up records an error
 // code and the CTA skips the rest of its work, frees its tensor memory and
 // returns.
@@ -24,20 +35,15 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace dcfr {
 
-// Two CTAs per SM (a 3-stage ring each, 97 KB of shared memory and 128
-// tensor-memory columns): one CTA's epilogue runs under the other's MMAs,
-// and a 4096 x 1024 output (256 tiles) fits the 148 SMs in one wave.
-#ifndef GEMM_STAGES_CFG
-#define GEMM_STAGES_CFG 3
-#endif
-#ifndef GEMM_CTAS_PER_SM
-#define GEMM_CTAS_PER_SM 2
-#endif
-constexpr int GEMM_BM = 128, GEMM_BN = 128, GEMM_BK = 64, GEMM_STAGES = GEMM_STAGES_CFG, GEMM_THREADS = 128;
-constexpr uint32_t GEMM_TILE_BYTES = GEMM_BM * GEMM_BK * 2;  // one 128 x 64 bf16 tile
-constexpr size_t GEMM_SMEM = 1024 + 2 * GEMM_STAGES * (size_t)GEMM_TILE_BYTES + 256;
+constexpr int GEMM_BM = 128, GEMM_BK = 64, GEMM_THREADS = 256;
+constexpr uint32_t GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;  // one 128 x 64 bf16 tile
+constexpr size_t gemm_smem(int bn, int stages) {
+  return 1024 + (size_t)stages * (GEMM_A_BYTES + (size_t)bn * GEMM_BK * 2) + 256;
+}
 constexpr long long GEMM_WAIT_LIMIT = 1ll << 22;  // polls before a wait gives up (well over a second)
 
 // Epilogues.
@@ -55,6 +61,7 @@ struct GemmArgs {
   int ldc;
   int epi;
   int M, N, K;
+  int wide;              // bf16 outputs: c, z and ldc allow 16-byte accesses
   int* error;            // set to a nonzero code when a bounded wait gives up
 };
 
@@ -137,26 +144,28 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.3989422804014327f * expf(-0.5f * x * x);
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
+template <int BN, int STAGES, int CTAS>
+__global__ void __launch_bounds__(GEMM_THREADS, CTAS)
     gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                         GemmArgs G) {
   extern __shared__ __align__(1024) unsigned char gemm_smem_raw[];
+  constexpr uint32_t B_BYTES = BN * GEMM_BK * 2;
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)gemm_smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sa = smem;
-  unsigned char* sb = smem + GEMM_STAGES * GEMM_TILE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + 2 * GEMM_STAGES * GEMM_TILE_BYTES);
-  uint64_t* empty = full + GEMM_STAGES;
-  uint64_t* accf = empty + GEMM_STAGES;
+  unsigned char* sb = smem + STAGES * GEMM_A_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sb + STAGES * B_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* accf = empty + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 1);
   __shared__ int failed;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * GEMM_BM, n0 = blockIdx.x * GEMM_BN;
+  const int m0 = blockIdx.y * GEMM_BM, n0 = blockIdx.x * BN;
   const int nk = G.K / GEMM_BK;
 
   if (tid == 0) {
     failed = 0;
-    for (int s = 0; s < GEMM_STAGES; s++) {
+    for (int s = 0; s < STAGES; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -165,7 +174,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(GEMM_BN)
+                 "r"(BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -173,30 +182,32 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0 && lane == 0) {
     // Producer.
     for (int kb = 0; kb < nk; kb++) {
-      const int s = kb % GEMM_STAGES;
-      if (kb >= GEMM_STAGES && !mbar_wait(&empty[s], ((kb / GEMM_STAGES) - 1) & 1)) {
+      const int s = kb % STAGES;
+      if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) {
         failed = 1;
         break;
       }
-      mbar_expect_tx(&full[s], 2 * GEMM_TILE_BYTES);
-      tma_load_2d(sa + s * GEMM_TILE_BYTES, &map_a, &full[s], kb * GEMM_BK, m0);
-      tma_load_2d(sb + s * GEMM_TILE_BYTES, &map_b, &full[s], kb * GEMM_BK, n0);
+      mbar_expect_tx(&full[s], GEMM_A_BYTES + B_BYTES);
+      tma_load_2d(sa + s * GEMM_A_BYTES, &map_a, &full[s], kb * GEMM_BK, m0);
+      tma_load_2d(sb + s * B_BYTES, &map_b, &full[s], kb * GEMM_BK, n0);
     }
   } else if (warp == 1 && lane == 0) {
     // Tensor-core issue.
-    const uint32_t idesc = idesc_bf16_f32(GEMM_BM, GEMM_BN);
+    const uint32_t idesc = idesc_bf16_f32(GEMM_BM, BN);
     for (int kb = 0; kb < nk; kb++) {
-      const int s = kb % GEMM_STAGES;
-      if (!mbar_wait(&full[s], (kb / GEMM_STAGES) & 1)) {
+      const int s = kb % STAGES;
+      if (!mbar_wait(&full[s], (kb / STAGES) & 1)) {
         failed = 2;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t da = sw128_desc(sa + s * GEMM_TILE_BYTES), db = sw128_desc(sb + s * GEMM_TILE_BYTES);
+      const uint64_t da = sw128_desc(sa + s * GEMM_A_BYTES), db = sw128_desc(sb + s * B_BYTES);
 #pragma unroll
       for (int k = 0; k < GEMM_BK / 16; k++)  // K = 16 per instruction: 32 bytes along the swizzled row
         umma_bf16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
@@ -205,7 +216,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
     umma_commit(accf);
   }
   __syncwarp();
-  // Epilogue: every thread owns one row of the tile.
+  // Epilogue: every thread owns half a row of the tile.
   const bool ok = mbar_wait(accf, 0);
   if (!ok && lane == 0) atomicExch(&failed, 3);
   __syncwarp();
@@ -213,26 +224,39 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
   // tcgen05.ld is warp-collective: decide once per warp.
   const bool go = __all_sync(0xffffffffu, ok && *(volatile int*)&failed == 0);
   if (go) {
-    const int m = m0 + warp * 32 + lane;
-    const uint32_t row_addr = tmem + ((uint32_t)(warp * 32) << 16);
+    constexpr int HALF = BN / 2, STEP = HALF < 32 ? HALF : 32;
+    const int quarter = warp & 3;
+    const int m = m0 + quarter * 32 + lane;
+    const uint32_t row_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    const int cbeg = (warp >> 2) * HALF;
 #pragma unroll 1
-    for (int c0 = 0; c0 < GEMM_BN; c0 += 32) {
-      uint32_t v[32];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
-          "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-            "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-            "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-          : "r"(row_addr + (uint32_t)c0));
+    for (int c0 = cbeg; c0 < cbeg + HALF; c0 += STEP) {
+      uint32_t v[STEP];
+      if constexpr (STEP == 32) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+            "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+              "=r"(v[16 % STEP]), "=r"(v[17 % STEP]), "=r"(v[18 % STEP]), "=r"(v[19 % STEP]), "=r"(v[20 % STEP]),
+              "=r"(v[21 % STEP]), "=r"(v[22 % STEP]), "=r"(v[23 % STEP]), "=r"(v[24 % STEP]), "=r"(v[25 % STEP]),
+              "=r"(v[26 % STEP]), "=r"(v[27 % STEP]), "=r"(v[28 % STEP]), "=r"(v[29 % STEP]), "=r"(v[30 % STEP]),
+              "=r"(v[31 % STEP])
+            : "r"(row_addr + (uint32_t)c0));
+      } else {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(row_addr + (uint32_t)c0));
+      }
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (m < G.M) {
         const int nb = n0 + c0;
         if (G.epi == EPI_F32 || G.epi == EPI_BIAS_F32) {
           float* out = reinterpret_cast<float*>(G.c) + (size_t)m * G.ldc + nb;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
+          for (int j = 0; j < STEP; j += 4) {
             float4 o;
             o.x = __uint_as_float(v[j]) + (G.epi == EPI_BIAS_F32 ? G.bias[nb + j] : 0.0f);
             o.y = __uint_as_float(v[j + 1]) + (G.epi == EPI_BIAS_F32 ? G.bias[nb + j + 1] : 0.0f);
@@ -244,19 +268,38 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
           __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(G.c) + (size_t)m * G.ldc + nb;
           __nv_bfloat16* zz = G.z + (size_t)m * G.ldc + nb;
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float a = __uint_as_float(v[j]), b = __uint_as_float(v[j + 1]);
-            __nv_bfloat162 r;
-            if (G.epi == EPI_BIAS_GELU) {
-              a += G.bias[nb + j];
-              b += G.bias[nb + j + 1];
-              *reinterpret_cast<__nv_bfloat162*>(zz + j) = __floats2bfloat162_rn(a, b);
-              r = __floats2bfloat162_rn(gelu(a), gelu(b));
-            } else {
-              const __nv_bfloat162 zv = *reinterpret_cast<const __nv_bfloat162*>(zz + j);
-              r = __floats2bfloat162_rn(a * gelu_grad(__bfloat162float(zv.x)), b * gelu_grad(__bfloat162float(zv.y)));
+          for (int j = 0; j < STEP; j += 8) {
+            union {
+              uint4 u;
+              __nv_bfloat162 h[4];
+            } z4, r4;
+            if (G.epi == EPI_GELU_GRAD) {
+              if (G.wide) z4.u = *reinterpret_cast<const uint4*>(zz + j);
+              else
+                for (int i = 0; i < 4; i++) z4.h[i] = *reinterpret_cast<const __nv_bfloat162*>(zz + j + 2 * i);
             }
-            *reinterpret_cast<__nv_bfloat162*>(out + j) = r;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              float a = __uint_as_float(v[j + 2 * i]), b = __uint_as_float(v[j + 2 * i + 1]);
+              if (G.epi == EPI_BIAS_GELU) {
+                a += G.bias[nb + j + 2 * i];
+                b += G.bias[nb + j + 2 * i + 1];
+                z4.h[i] = __floats2bfloat162_rn(a, b);
+                r4.h[i] = __floats2bfloat162_rn(gelu(a), gelu(b));
+              } else {
+                r4.h[i] = __floats2bfloat162_rn(a * gelu_grad(__bfloat162float(z4.h[i].x)),
+                                                b * gelu_grad(__bfloat162float(z4.h[i].y)));
+              }
+            }
+            if (G.wide) {
+              if (G.epi == EPI_BIAS_GELU) *reinterpret_cast<uint4*>(zz + j) = z4.u;
+              *reinterpret_cast<uint4*>(out + j) = r4.u;
+            } else {
+              for (int i = 0; i < 4; i++) {
+                if (G.epi == EPI_BIAS_GELU) *reinterpret_cast<__nv_bfloat162*>(zz + j + 2 * i) = z4.h[i];
+                *reinterpret_cast<__nv_bfloat162*>(out + j + 2 * i) = r4.h[i];
+              }
+            }
           }
         }
       }
@@ -267,7 +310,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS_PER_SM)
   if (failed && tid == 0 && G.error) atomicExch(G.error, failed);
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GEMM_BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
   }
 }
 

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -68,14 +69,14 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // Tensor map of a row-major bf16 matrix [rows][cols] (cols contiguous), read
-// in 128-row x 64-column boxes with the 128-byte swizzle.
-int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols) {
+// in boxes of box_rows x 64 with the 128-byte swizzle.
+int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
   auto enc = tensor_map_encoder();
   if (!enc) return fail(DCFR_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   if (((uintptr_t)base & 15) || (cols * 2) % 16) return fail(DCFR_ERR_INVALID_ARG, "GEMM operand is not 16-byte aligned");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {GEMM_BK, GEMM_BM};
+  cuuint32_t box[2] = {GEMM_BK, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -84,43 +85,95 @@ int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols) {
   return DCFR_OK;
 }
 
+using GemmKernel = void (*)(CUtensorMap, CUtensorMap, GemmArgs);
+struct GemmShape {
+  GemmKernel kernel;
+  int bn;
+  size_t smem;
+};
+template <int BN, int STAGES, int CTAS>
+GemmShape gemm_variant() {
+  return GemmShape{(GemmKernel)gemm_bf16_tc_kernel<BN, STAGES, CTAS>, BN, gemm_smem(BN, STAGES)};
+}
+
+// The tile of an [M][N] output. 128 x 128 where that gives three fifths of the
+// SMs a CTA: two to an SM with 3-stage rings once there are more CTAs than
+// SMs (one's epilogue runs under the other's MMAs), else one with 6 stages.
+// Narrower tiles below (M = 896: 64 wide, M = 256: 32 wide; a 9-stage ring
+// there gains 3%).
+GemmShape gemm_shape(int M, int N) {
+  const int rows = M / GEMM_BM;
+  if (rows * (N / 128) > 148) return gemm_variant<128, 3, 2>();
+  if (rows * (N / 128) >= 90) return gemm_variant<128, 6, 1>();
+  if (rows * (N / 64) >= 90) return gemm_variant<64, 8, 1>();
+  return gemm_variant<32, 5, 2>();
+}
+
 // C = epi(A[M][K] x B[N][K]^T); M, N multiples of 128, K of 64.
 int gemm(const bf16* A, const bf16* B, int M, int N, int K, int epi, void* C, int ldc, bf16* z, const float* bias,
          int* err, cudaStream_t s) {
-  if (M % GEMM_BM || N % GEMM_BN || K % GEMM_BK || M <= 0 || N <= 0 || K <= 0)
+  if (M % GEMM_BM || N % 128 || K % GEMM_BK || M <= 0 || N <= 0 || K <= 0)
     return fail(DCFR_ERR_INVALID_ARG, "GEMM: M and N must be multiples of 128 and K of 64");
-  static bool attr = false;
-  if (!attr) {
-    MK(cudaFuncSetAttribute(gemm_bf16_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
-    attr = true;
-  }
+  const GemmShape v = gemm_shape(M, N);
+  MK(cudaFuncSetAttribute((const void*)v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
   CUtensorMap ma, mb;
-  int rc = make_map(&ma, A, (uint64_t)M, (uint64_t)K);
+  int rc = make_map(&ma, A, (uint64_t)M, (uint64_t)K, GEMM_BM);
   if (rc) return rc;
-  if ((rc = make_map(&mb, B, (uint64_t)N, (uint64_t)K))) return rc;
-  GemmArgs G{C, z, bias, ldc, epi, M, N, K, err};
-  gemm_bf16_tc_kernel<<<dim3((unsigned)(N / GEMM_BN), (unsigned)(M / GEMM_BM)), GEMM_THREADS, GEMM_SMEM, s>>>(ma, mb, G);
-  MK(cudaGetLastError());
+  if ((rc = make_map(&mb, B, (uint64_t)N, (uint64_t)K, (uint32_t)v.bn))) return rc;
+  const int wide = (((uintptr_t)C | (uintptr_t)z) & 15) == 0 && ldc % 8 == 0;
+  GemmArgs G{C, z, bias, ldc, epi, M, N, K, wide, err};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(N / v.bn), (unsigned)(M / GEMM_BM));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = v.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MK(cudaLaunchKernelEx(&cfg, v.kernel, ma, mb, G));
   return DCFR_OK;
 }
 
-// out[c][r] = in[r][c] (bf16), tiles of 32 x 32 through shared memory.
-__global__ void transpose_bf16(const bf16* __restrict__ in, bf16* __restrict__ out, int rows, int cols) {
-  __shared__ bf16 t[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    t[i][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * cols + c] : __float2bfloat16(0.0f);
+// out[c][r] = in[r][c] (bf16, rows and cols multiples of 64), tiles of 64 x 64
+// through shared memory with 16-byte accesses on both sides; one launch for
+// two matrices of the same rows (blockIdx.x runs over both matrices' columns).
+struct TransposePair {
+  const bf16* in[2];
+  bf16* out[2];
+  int cols[2];
+};
+__global__ void __launch_bounds__(256) transpose_bf16(TransposePair P, int rows) {
+  __shared__ uint16_t t[64][66];
+  const int split = P.cols[0] / 64, which = (int)blockIdx.x >= split ? 1 : 0;
+  const int c0 = ((int)blockIdx.x - which * split) * 64, r0 = blockIdx.y * 64, cols = which ? P.cols[1] : P.cols[0];
+  const uint16_t* in = reinterpret_cast<const uint16_t*>(which ? P.in[1] : P.in[0]);
+  uint16_t* out = reinterpret_cast<uint16_t*>(which ? P.out[1] : P.out[0]);
+  for (int i = threadIdx.x; i < 512; i += 256) {
+    const int r = i >> 3, c = (i & 7) * 8;
+    const uint4 v = *reinterpret_cast<const uint4*>(in + (size_t)(r0 + r) * cols + c0 + c);
+    uint32_t* d = reinterpret_cast<uint32_t*>(&t[r][c]);
+    d[0] = v.x;
+    d[1] = v.y;
+    d[2] = v.z;
+    d[3] = v.w;
   }
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < cols && r < rows) out[(size_t)c * rows + r] = t[threadIdx.x][i];
+  for (int i = threadIdx.x; i < 512; i += 256) {
+    // Neighbouring threads take neighbouring columns of t: no bank conflicts.
+    const int c = (i & 7) + ((i >> 6) << 3), r = ((i >> 3) & 7) * 8;
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = (uint32_t)t[r + 2 * k][c] | (uint32_t)t[r + 2 * k + 1][c] << 16;
+    *reinterpret_cast<uint4*>(out + (size_t)(c0 + c) * rows + r0 + r) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
-void transpose(const bf16* in, bf16* out, int rows, int cols, cudaStream_t s) {
-  transpose_bf16<<<dim3((cols + 31) / 32, (rows + 31) / 32), dim3(32, 8), 0, s>>>(in, out, rows, cols);
+void transpose(const bf16* in, bf16* out, int rows, int cols, cudaStream_t s, const bf16* in2 = nullptr,
+               bf16* out2 = nullptr, int cols2 = 0) {
+  const TransposePair P{{in, in2}, {out, out2}, {cols, cols2}};
+  transpose_bf16<<<dim3((cols + cols2) / 64, rows / 64), 256, 0, s>>>(P, rows);
 }
 
 // Row-major f32 [rows][cols] into a zero-padded bf16 [prow][pcol].
@@ -131,80 +184,120 @@ __global__ void pack_bf16(const float* __restrict__ in, int rows, int cols, bf16
   out[i] = __float2bfloat16(r < rows && c < cols ? in[(size_t)r * cols + c] : 0.0f);
 }
 
-// f32 -> bf16, same layout; and f32 W_t[n][k] -> bf16 W[k][n].
+// f32 -> bf16, same layout.
 __global__ void f32_to_bf16(const float* __restrict__ in, bf16* __restrict__ out, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = __float2bfloat16(in[i]);
 }
 
-__global__ void f32_transpose_bf16(const float* __restrict__ in, bf16* __restrict__ out, int rows, int cols) {
-  __shared__ float t[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    t[i][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * cols + c] : 0.0f;
-  }
+// Sum over the block (256 threads), added to *to by its first thread: one
+// atomic per block.
+__device__ __forceinline__ void block_add(float v, float* to) {
+  __shared__ float red[8];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < cols && r < rows) out[(size_t)c * rows + r] = __float2bfloat16(t[threadIdx.x][i]);
+  if (threadIdx.x == 0) {
+    float t = 0.0f;
+    for (int w = 0; w < 8; w++) t += red[w];
+    if (t != 0.0f) atomicAdd(to, t);
   }
 }
+// Blocks of the reductions: one atomic each on one address (an atomic per
+// warp of a thread per element cost 34 us a reduction of 0.7 M elements).
+constexpr int REDUCE_BLOCKS = 296;
 
 // count[0] = number of valid outputs (sum of the mask, or rows * cols).
-__global__ void mask_count(const float* __restrict__ mask, size_t n, float* __restrict__ count) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float c = i < n ? (mask ? mask[i] : 1.0f) : 0.0f;
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0 && c != 0.0f) atomicAdd(count, c);
+__global__ void __launch_bounds__(256) mask_count(const float* __restrict__ mask, size_t n, float* __restrict__ count) {
+  float c = 0.0f;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    c += mask ? mask[i] : 1.0f;
+  block_add(c, count);
 }
 
 // dY = 2 * mask * (Y - T) / count (bf16) and loss += mask * (Y - T)^2 / count,
 // over the padded [prow][pcol] output; T and mask are [rows][cols] f32.
-__global__ void loss_grad(const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ mask,
-                          int rows, int cols, int prow, int pcol, const float* __restrict__ count,
-                          bf16* __restrict__ dY, float* __restrict__ loss) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) loss_grad(const float* __restrict__ Y, const float* __restrict__ T,
+                                                 const float* __restrict__ mask, int rows, int cols, int prow, int pcol,
+                                                 const float* __restrict__ count, bf16* __restrict__ dY,
+                                                 float* __restrict__ loss) {
   const float inv_count = *count > 0.0f ? 1.0f / *count : 0.0f;
   float l = 0.0f;
-  if (i < (size_t)prow * pcol) {
-    const int r = (int)(i / pcol), c = (int)(i % pcol);
-    float g = 0.0f;
-    if (r < rows && c < cols) {
-      const size_t j = (size_t)r * cols + c;
-      const float m = mask ? mask[j] : 1.0f;
-      const float d = Y[i] - T[j];
-      g = 2.0f * m * d * inv_count;
-      l = m * d * d * inv_count;
+  for (int r = blockIdx.x; r < prow; r += gridDim.x)
+    for (int c = threadIdx.x; c < pcol; c += blockDim.x) {
+      float g = 0.0f;
+      if (r < rows && c < cols) {
+        const size_t j = (size_t)r * cols + c;
+        const float m = mask ? mask[j] : 1.0f;
+        const float d = Y[(size_t)r * pcol + c] - T[j];
+        g = 2.0f * m * d * inv_count;
+        l += m * d * d * inv_count;
+      }
+      dY[(size_t)r * pcol + c] = __float2bfloat16(g);
     }
-    dY[i] = __float2bfloat16(g);
+  block_add(l, loss);
+}
+
+// db[c] = sum over rows of dY[r][c]: 64 columns and 8 runs of rows a block.
+__global__ void __launch_bounds__(256) column_sums(const bf16* __restrict__ dY, int rows, int cols,
+                                                   float* __restrict__ db) {
+  __shared__ float2 part[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const __nv_bfloat162* in = reinterpret_cast<const __nv_bfloat162*>(dY + blockIdx.x * 64) + x;
+  float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll 8
+  for (int r = y; r < rows; r += 8) {
+    const float2 v = __bfloat1622float2(in[(size_t)r * (cols / 2)]);
+    acc.x += v.x;
+    acc.y += v.y;
   }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0 && l != 0.0f) atomicAdd(loss, l);
+  part[y][x] = acc;
+  __syncthreads();
+  if (y == 0) {
+    for (int k = 1; k < 8; k++) {
+      acc.x += part[k][x].x;
+      acc.y += part[k][x].y;
+    }
+    reinterpret_cast<float2*>(db + blockIdx.x * 64)[x] = acc;
+  }
 }
 
-// db[c] = sum over rows of dY[r][c].
-__global__ void column_sums(const bf16* __restrict__ dY, int rows, int cols, float* __restrict__ db) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float acc = 0.0f;
-  for (int r = 0; r < rows; r++) acc += __bfloat162float(dY[(size_t)r * cols + c]);
-  db[c] = acc;
-}
-
-// Adam on the f32 master copy; gradients of padded entries are zero by
-// construction (pmask marks the real entries).
-__global__ void adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                     const uint8_t* __restrict__ pmask, size_t n, float lr, float b1, float b2, float eps, float c1,
-                     float c2, float gscale) {
+// Adam on the f32 master copy, and its bf16 copy of the first nw (the
+// weights); gradients of padded entries are zero by construction (pmask marks
+// the real entries). n and nw are multiples of 4. Bound by memory: 33 bytes an
+// entry, 4 entries a thread.
+__global__ void __launch_bounds__(256) adam(float4* __restrict__ w, const float4* __restrict__ g,
+                                            float4* __restrict__ m, float4* __restrict__ v,
+                                            const uchar4* __restrict__ pmask, bf16* __restrict__ w16, size_t n4,
+                                            size_t nw4, float lr, float b1, float b2, float eps, float c1, float c2,
+                                            float gscale) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !pmask[i]) return;
-  const float gi = g[i] * gscale;
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+  if (i >= n4) return;
+  const uchar4 on = pmask[i];
+  float4 wi = w[i], mi = m[i], vi = v[i];
+  const float4 gi = g[i];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (!(&on.x)[k]) continue;
+    const float gk = (&gi.x)[k] * gscale;
+    const float mk = b1 * (&mi.x)[k] + (1.0f - b1) * gk;
+    const float vk = b2 * (&vi.x)[k] + (1.0f - b2) * gk * gk;
+    (&mi.x)[k] = mk;
+    (&vi.x)[k] = vk;
+    (&wi.x)[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+  }
+  w[i] = wi;
   m[i] = mi;
   v[i] = vi;
-  w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  if (i < nw4) {
+    union {
+      uint2 u;
+      __nv_bfloat162 h[2];
+    } o;
+    o.h[0] = __floats2bfloat162_rn(wi.x, wi.y);
+    o.h[1] = __floats2bfloat162_rn(wi.z, wi.w);
+    reinterpret_cast<uint2*>(w16)[i] = o.u;
+  }
 }
 
 __global__ void copy_rows_f32(const float* __restrict__ in, int pcol, int rows, int cols, float* __restrict__ out) {
@@ -224,18 +317,20 @@ struct dcfr_mlp {
   size_t nparams = 0, nw = 0;
   float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // flat: all W_t then all b
   uint8_t* pmask = nullptr;
-  std::vector<bf16*> wt_bf, w_bf;       // per layer: [N][K] and [K][N]
+  bf16* w16 = nullptr;                  // all W_t in bf16, laid out as w
+  std::vector<bf16*> wt_bf, w_bf;       // per layer: [N][K] (in w16) and [K][N]
   std::vector<bf16*> X, Z;              // activations [Mp][kin[l]] (X_0 = input) and pre-activations
   std::vector<bf16*> dY;                // [Mp][nout[l]]
   bf16 *tA = nullptr, *tB = nullptr;    // transposes for the weight-gradient GEMM
   float* Y = nullptr;                   // [Mp][nout[L]]
-  float* loss = nullptr;
-  int* err = nullptr;
+  float* loss = nullptr;                // [0] the loss, [1] the valid outputs, [2] err
+  int* err = nullptr;                   // set by a GEMM whose wait gave up
+  float* result = nullptr;              // page-locked copy of loss[0..2]
   int step = 0;
   cudaStream_t stream = nullptr;
   ~dcfr_mlp() {
-    for (void* p : std::vector<void*>{w, g, m, v, pmask, tA, tB, Y, loss, err}) cudaFree(p);
-    for (auto* p : wt_bf) cudaFree(p);
+    for (void* p : std::vector<void*>{w, g, m, v, pmask, w16, tA, tB, Y, loss}) cudaFree(p);
+    if (result) cudaFreeHost(result);
     for (auto* p : w_bf) cudaFree(p);
     for (auto* p : X) cudaFree(p);
     for (auto* p : Z) cudaFree(p);
@@ -246,21 +341,21 @@ struct dcfr_mlp {
 
 namespace {
 
-int refresh_bf16(dcfr_mlp* n) {
-  const int L = n->layers + 1;
-  for (int l = 0; l < L; l++) {
-    const size_t cnt = (size_t)n->nout[l] * n->kin[l];
-    f32_to_bf16<<<blocks_for(cnt, 256), 256, 0, n->stream>>>(n->w + n->woff[l], n->wt_bf[l], cnt);
-    f32_transpose_bf16<<<dim3((n->kin[l] + 31) / 32, (n->nout[l] + 31) / 32), dim3(32, 8), 0, n->stream>>>(
-        n->w + n->woff[l], n->w_bf[l], n->nout[l], n->kin[l]);
-  }
+// The transposed weights, from the bf16 copy.
+int refresh_transposed(dcfr_mlp* n) {
+  for (int l = 0; l <= n->layers; l++) transpose(n->wt_bf[l], n->w_bf[l], n->nout[l], n->kin[l], n->stream);
   MK(cudaGetLastError());
   return DCFR_OK;
 }
 
-int forward(dcfr_mlp* n, const float* x, int M, int Mp, cudaStream_t s) {
+int refresh_bf16(dcfr_mlp* n) {
+  f32_to_bf16<<<blocks_for(n->nw, 256), 256, 0, n->stream>>>(n->w, n->w16, n->nw);
+  return refresh_transposed(n);
+}
+
+// The layers on Mp packed input rows.
+int forward_packed(dcfr_mlp* n, int Mp, cudaStream_t s) {
   int rc;
-  pack_bf16<<<blocks_for((size_t)Mp * n->kin[0], 256), 256, 0, s>>>(x, M, n->in_dim, n->X[0], Mp, n->kin[0]);
   for (int l = 0; l < n->layers; l++)
     if ((rc = gemm(n->X[l], n->wt_bf[l], Mp, n->nout[l], n->kin[l], EPI_BIAS_GELU, n->X[l + 1], n->nout[l], n->Z[l],
                    n->w + n->boff[l], n->err, s)))
@@ -270,27 +365,28 @@ int forward(dcfr_mlp* n, const float* x, int M, int Mp, cudaStream_t s) {
               n->w + n->boff[L], n->err, s);
 }
 
-int forward(dcfr_mlp* n, const float* x, int M, int Mp) { return forward(n, x, M, Mp, n->stream); }
+int forward(dcfr_mlp* n, const float* x, int M, int Mp) {
+  pack_bf16<<<blocks_for((size_t)Mp * n->kin[0], 256), 256, 0, n->stream>>>(x, M, n->in_dim, n->X[0], Mp, n->kin[0]);
+  return forward_packed(n, Mp, n->stream);
+}
 
 // Gradients of the loss into n->g (and the loss into n->loss).
 int backward(dcfr_mlp* n, const float* target, const float* mask, int M, int Mp) {
   const int L = n->layers;
   // loss[0]: the loss; loss[1]: the number of valid outputs (the normaliser).
   MK(cudaMemsetAsync(n->loss, 0, 8, n->stream));
-  MK(cudaMemsetAsync(n->g, 0, n->nparams * 4, n->stream));
   const size_t nt = (size_t)M * n->out_dim;
-  mask_count<<<blocks_for(nt, 256), 256, 0, n->stream>>>(mask, nt, n->loss + 1);
-  loss_grad<<<blocks_for((size_t)Mp * n->nout[L], 256), 256, 0, n->stream>>>(
+  mask_count<<<REDUCE_BLOCKS, 256, 0, n->stream>>>(mask, nt, n->loss + 1);
+  loss_grad<<<std::min(Mp, REDUCE_BLOCKS), 256, 0, n->stream>>>(
       n->Y, target, mask, M, n->out_dim, Mp, n->nout[L], n->loss + 1, n->dY[L], n->loss);
   int rc;
   for (int l = L; l >= 0; l--) {
     const int K = n->kin[l], N = n->nout[l];
     // dW_t[l] [N][K] = dY_l^T X_l: operands dY_l^T [N][Mp] and X_l^T [K][Mp].
-    transpose(n->dY[l], n->tA, Mp, N, n->stream);
-    transpose(n->X[l], n->tB, Mp, K, n->stream);
+    transpose(n->dY[l], n->tA, Mp, N, n->stream, n->X[l], n->tB, K);
     if ((rc = gemm(n->tA, n->tB, N, K, Mp, EPI_F32, n->g + n->woff[l], K, nullptr, nullptr, n->err, n->stream)))
       return rc;
-    column_sums<<<blocks_for(N, 128), 128, 0, n->stream>>>(n->dY[l], Mp, N, n->g + n->boff[l]);
+    column_sums<<<N / 64, 256, 0, n->stream>>>(n->dY[l], Mp, N, n->g + n->boff[l]);
     if (l > 0) {
       // dY_{l-1} = (dY_l W_l) * gelu'(Z_{l-1}): B operand W_l as [K][N].
       if ((rc = gemm(n->dY[l], n->w_bf[l], Mp, K, N, EPI_GELU_GRAD, n->dY[l - 1], K, n->Z[l - 1], nullptr, n->err,
@@ -302,11 +398,15 @@ int backward(dcfr_mlp* n, const float* target, const float* mask, int M, int Mp)
   return DCFR_OK;
 }
 
-int check_err(dcfr_mlp* n) {
-  int e = 0;
-  MK(cudaMemcpyAsync(&e, n->err, 4, cudaMemcpyDeviceToHost, n->stream));
+// Waits for the stream; the loss and the GEMMs' error flag come back in one
+// copy.
+int check_err(dcfr_mlp* n, float* loss = nullptr) {
+  MK(cudaMemcpyAsync(n->result, n->loss, 12, cudaMemcpyDeviceToHost, n->stream));
   MK(cudaStreamSynchronize(n->stream));
+  int e = 0;
+  std::memcpy(&e, n->result + 2, 4);
   if (e) return fail(DCFR_ERR_DEVICE_TIMEOUT, "tensor-core GEMM: a bounded wait gave up (code " + std::to_string(e) + ")");
+  if (loss) *loss = n->result[0];
   return DCFR_OK;
 }
 
@@ -327,13 +427,20 @@ int mlp_shape(const dcfr_mlp* n, int* in_dim, int* out_dim, int* max_batch) {
   return DCFR_OK;
 }
 
-// The network's forward pass on stream s, nothing synchronised: a solver
-// enqueues it between its kernels (and captures it in its graphs). y is the
-// network's own padded output buffer, valid until its next forward pass.
-int mlp_enqueue_forward(dcfr_mlp* n, const float* x, int m, cudaStream_t s, const float** y, int* ldy) {
+// The rows that a forward pass reads: a solver writes its inputs there.
+bf16* mlp_input(dcfr_mlp* n, int* ldx) {
+  *ldx = n->kin[0];
+  return n->X[0];
+}
+
+// The network's forward pass on the first m packed input rows on stream s,
+// nothing synchronised: a solver enqueues it between its kernels (and captures
+// it in its graphs). y is the network's own padded output buffer, valid until
+// its next forward pass.
+int mlp_enqueue_forward(dcfr_mlp* n, int m, cudaStream_t s, const float** y, int* ldy) {
   int rc = batch_ok(n, m);
   if (rc) return rc;
-  if ((rc = forward(n, x, m, pad128(m), s))) return rc;
+  if ((rc = forward_packed(n, pad128(m), s))) return rc;
   *y = n->Y;
   *ldy = n->nout[n->layers];
   return DCFR_OK;
@@ -445,12 +552,12 @@ int dcfr_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, int32_t out_
   MK(cudaMemcpy(n->pmask, hm.data(), n->nparams, cudaMemcpyHostToDevice));
   MK(cudaMemset(n->m, 0, n->nparams * 4));
   MK(cudaMemset(n->v, 0, n->nparams * 4));
+  MK(cudaMalloc(&n->w16, n->nw * 2));
   size_t tmax = 0;
   for (int l = 0; l < L; l++) {
-    bf16 *a = nullptr, *b = nullptr;
-    MK(cudaMalloc(&a, (size_t)n->nout[l] * n->kin[l] * 2));
+    bf16* b = nullptr;
     MK(cudaMalloc(&b, (size_t)n->nout[l] * n->kin[l] * 2));
-    n->wt_bf.push_back(a);
+    n->wt_bf.push_back(n->w16 + n->woff[l]);
     n->w_bf.push_back(b);
     tmax = std::max(tmax, (size_t)std::max(n->kin[l], n->nout[l]));
   }
@@ -470,9 +577,10 @@ int dcfr_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, int32_t out_
   MK(cudaMalloc(&n->tA, (size_t)Mp * tmax * 2));
   MK(cudaMalloc(&n->tB, (size_t)Mp * tmax * 2));
   MK(cudaMalloc(&n->Y, (size_t)Mp * n->nout[layers] * 4));
-  MK(cudaMalloc(&n->loss, 8));
-  MK(cudaMalloc(&n->err, 4));
-  MK(cudaMemset(n->err, 0, 4));
+  MK(cudaMalloc(&n->loss, 12));
+  MK(cudaMemset(n->loss, 0, 12));
+  n->err = reinterpret_cast<int*>(n->loss + 2);
+  MK(cudaMallocHost(&n->result, 12));
   int rc = refresh_bf16(n.get());
   if (rc) return rc;
   MK(cudaStreamSynchronize(n->stream));
@@ -526,8 +634,7 @@ int dcfr_mlp_gradients(dcfr_mlp* n, const float* x, const float* target, const f
   const int Mp = pad128(M);
   if ((rc = forward(n, x, M, Mp))) return rc;
   if ((rc = backward(n, target, mask, M, Mp))) return rc;
-  if ((rc = check_err(n))) return rc;
-  if (loss) MK(cudaMemcpy(loss, n->loss, 4, cudaMemcpyDeviceToHost));
+  if ((rc = check_err(n, loss))) return rc;
   if (grads_host) MK(cudaMemcpy(grads_host, n->g, n->nparams * 4, cudaMemcpyDeviceToHost));
   return DCFR_OK;
 }
@@ -538,9 +645,11 @@ static int adam_step(dcfr_mlp* n, float lr, float gscale) {
   n->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f - std::pow(b1, (float)n->step), c2 = 1.0f - std::pow(b2, (float)n->step);
-  adam<<<blocks_for(n->nparams, 256), 256, 0, n->stream>>>(n->w, n->g, n->m, n->v, n->pmask, n->nparams, lr, b1, b2,
-                                                           1e-8f, c1, c2, gscale);
-  return refresh_bf16(n);
+  adam<<<blocks_for(n->nparams / 4, 256), 256, 0, n->stream>>>(
+      reinterpret_cast<float4*>(n->w), reinterpret_cast<const float4*>(n->g), reinterpret_cast<float4*>(n->m),
+      reinterpret_cast<float4*>(n->v), reinterpret_cast<const uchar4*>(n->pmask), n->w16, n->nparams / 4, n->nw / 4, lr,
+      b1, b2, 1e-8f, c1, c2, gscale);
+  return refresh_transposed(n);
 }
 
 int dcfr_mlp_train_step(dcfr_mlp* n, const float* x, const float* target, const float* mask, int32_t M, float lr,
@@ -552,8 +661,7 @@ int dcfr_mlp_train_step(dcfr_mlp* n, const float* x, const float* target, const 
   if ((rc = forward(n, x, M, Mp))) return rc;
   if ((rc = backward(n, target, mask, M, Mp))) return rc;
   if ((rc = adam_step(n, lr, 1.0f))) return rc;
-  if ((rc = check_err(n))) return rc;
-  if (loss) MK(cudaMemcpy(loss, n->loss, 4, cudaMemcpyDeviceToHost));
+  if ((rc = check_err(n, loss))) return rc;
   return DCFR_OK;
 }
 
@@ -568,10 +676,7 @@ int dcfr_mlp_backward(dcfr_mlp* n, const float* x, const float* target, const fl
   const int Mp = pad128(M);
   if ((rc = forward(n, x, M, Mp))) return rc;
   if ((rc = backward(n, target, mask, M, Mp))) return rc;
-  if ((rc = check_err(n))) return rc;
-  if (loss) MK(cudaMemcpy(loss, n->loss, 4, cudaMemcpyDeviceToHost));
-  MK(cudaStreamSynchronize(n->stream));
-  return DCFR_OK;
+  return check_err(n, loss);
 }
 
 int dcfr_mlp_gradients_device(dcfr_mlp* n, float** grads, uint64_t* count) {
@@ -585,9 +690,7 @@ int dcfr_mlp_adam_step(dcfr_mlp* n, float lr, float gscale) {
   if (!n) return fail(DCFR_ERR_INVALID_ARG, "NULL argument");
   int rc = adam_step(n, lr, gscale);
   if (rc) return rc;
-  if ((rc = check_err(n))) return rc;
-  MK(cudaStreamSynchronize(n->stream));
-  return DCFR_OK;
+  return check_err(n);
 }
 
 }  // extern "C"
