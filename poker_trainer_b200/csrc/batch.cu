@@ -870,7 +870,7 @@ void Batch::Impl::enqueue(int mode, const dcfr_batch_tuning& t) {
   const bool lpt = t.longest_first != 0;
   float* out = mode == M_CFR ? nullptr : root_out;
   launch_traversal_start(alive, (int)total_slots, alive + total_slots, (int)total_slots, reach, roots, 0,
-                         mode == M_CFR ? counter : nullptr, disc, disc_len, cur_disc, stream);
+                         mode == M_CFR ? counter : nullptr, disc, disc_len, cur_disc, nullptr, stream);
   enqueue_rows(mode, -1, 0, lpt, nullptr);
   enqueue_terminals(0, t);
   enqueue_rows(mode, 0, 1, lpt, out);

@@ -46,6 +46,9 @@ static void dfree(T*& p) {
   p = nullptr;
 }
 
+// Terminals per SM from which the tile kernel evaluates them.
+constexpr int TILE_TERMINALS_PER_SM = 384;
+
 static inline int pad8(int n) { return (n + 7) & ~7; }
 
 Plan::~Plan() {
@@ -53,6 +56,7 @@ Plan::~Plan() {
   dfree(d_up);
   dfree(d_fast);
   dfree(d_units);
+  dfree(d_jobs);
   dfree(d_panels);
   dfree(d_leaves);
   dfree(d_trees);
@@ -177,6 +181,7 @@ Engine::~Engine() {
   dfree(tables_);
   dfree(table_count_);
   dfree(term_counter_);
+  dfree(tile_claims_);
   dfree(fcat_);
   dfree(fseg_);
   dfree(frec_);
@@ -472,6 +477,18 @@ Status Engine::ensure_fast_layouts() {
   }
   term_group_ = want == "group" && group_groups_ > 0;
   term_group_auto_ = sel == nullptr && group_groups_ > 0;
+  // Tiles where the tree has many terminals per SM (their number is known
+  // from the count, before the plans, whose task order differs): a block then
+  // works through hundreds of tiles. us a traversal's terminals, tiles against
+  // two warps per terminal: flop 8300 against 10820 (23,800 terminals an SM,
+  // 470 hands), with sampled cards 521 against 589 (929 an SM); a turn's 79 an
+  // SM lose to staging and part tiles, 99 against 87 (816 hands) and 51 against
+  // 46 (470).
+  tile_T_ = 0;
+  if (fast_ && (want == "tile" || (sel == nullptr && g.stats.terminal >= (uint64_t)TILE_TERMINALS_PER_SM * sms)))
+    tile_T_ = tile_terminal_setup(g.n[0], g.n[1], hp_[0], hp_[1]);
+  if (want == "tile" && tile_T_ > 0) term_group_ = true;
+  if (tile_T_ > 0 && !(s = dalloc(tile_claims_, 2, "terminal counter")).ok()) return s;
   if (term_kernel_ == TK_PANEL) {
     const int o0 = 1, o1 = 0;  // opponent of traverser 0 and 1
     panel_T_ = panel_E_ = panel_blocks_ = 0;
@@ -927,7 +944,42 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   plan.h_panels.clear();
   const bool panels = fast_ && term_kernel_ == TK_PANEL;
   const size_t PT = panels ? (size_t)panel_T_ : 1;
-  for (uint32_t l = 0; l <= nb; l++) {
+  // With tiles a layout's tasks are ordered by class instead.
+  plan.h_units.clear();
+  for (uint32_t l = 0; l <= nb && tile_T_ > 0; l++)
+    for (uint32_t cls : {TILE_PLAIN, TILE_GENERAL, TILE_FOLD}) {
+      const uint32_t first = (uint32_t)plan.h_fast.size();
+      if (cls == TILE_FOLD) {
+        for (uint32_t i = f_off[l]; i < f_off[l + 1]; i++) plan.h_fast.push_back(fold_task(f_idx[i]));
+      } else {
+        for (uint32_t i = s_off[l]; i < s_off[l + 1]; i++) {
+          const SdLane& x = sd[s_idx[i]];
+          const bool plain = x.kind == T_SHOWDOWN_BATCH && x.lane.c == 0.0 && x.lane.frow == NONE32;
+          if (plain == (cls == TILE_PLAIN)) plan.h_fast.push_back(sd_task(s_idx[i]));
+        }
+      }
+      const uint32_t count = (uint32_t)plan.h_fast.size() - first;
+      if (count) plan.h_units.push_back(TermUnit{l, first, count, cls});
+    }
+  // Jobs of the tile kernel: whole windows first, the last quarter of the
+  // tasks in smaller and smaller ones, so that blocks finish together.
+  plan.h_jobs.clear();
+  if (tile_T_ > 0) {
+    const size_t all = plan.h_fast.size(), per_block = all / (size_t)std::max(term_sms_, 1) + 1;
+    size_t done = 0;
+    for (const TermUnit& U : plan.h_units)
+      for (uint32_t i = 0; i < U.count;) {
+        const size_t left = all - done;
+        size_t most = std::min<size_t>(TILE_THREADS, per_block / 4 + 1);
+        if (left * 4 < all) most = std::min(most, left / (2 * (size_t)term_sms_) + 1);
+        most = std::max<size_t>((most + tile_T_ - 1) / tile_T_ * tile_T_, 2 * (size_t)tile_T_);
+        const uint32_t c = (uint32_t)std::min<size_t>(most, U.count - i);
+        plan.h_jobs.push_back(TermUnit{U.layout, U.first + i, c, U.pad});
+        i += c;
+        done += c;
+      }
+  }
+  for (uint32_t l = 0; l <= nb && tile_T_ == 0; l++) {
     const size_t S0 = s_off[l], SN = s_off[l + 1] - S0, F0 = f_off[l], FN = f_off[l + 1] - F0;
     const size_t ns = (SN + PT - 1) / PT, nf = (FN + PT - 1) / PT;
     size_t i = 0, j = 0;
@@ -942,8 +994,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   }
   // Units of the warp terminal kernel: maximal runs of tasks on one layout
   // (h_fast is ordered by layout).
-  plan.h_units.clear();
-  for (size_t i = 0; i < plan.h_fast.size();) {
+  for (size_t i = 0; i < plan.h_fast.size() && tile_T_ == 0;) {
     size_t j = i;
     while (j < plan.h_fast.size() && plan.h_fast[j].board == plan.h_fast[i].board) j++;
     plan.h_units.push_back(TermUnit{plan.h_fast[i].board, (uint32_t)i, (uint32_t)(j - i), 0});
@@ -1009,6 +1060,9 @@ Status Engine::upload_plan(Plan& plan) {
   if (!(s = dalloc(plan.d_up, plan.h_up.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fast, plan.h_fast.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_units, plan.h_units.size(), "plan")).ok()) return s;
+  if (!(s = dalloc(plan.d_jobs, plan.h_jobs.size(), "plan")).ok()) return s;
+  if (!plan.h_jobs.empty())
+    CK(cudaMemcpy(plan.d_jobs, plan.h_jobs.data(), plan.h_jobs.size() * sizeof(TermUnit), cudaMemcpyHostToDevice));
   if (!(s = dalloc(plan.d_leaves, plan.h_leaves.size(), "plan")).ok()) return s;
   if (!plan.h_leaves.empty())
     CK(cudaMemcpy(plan.d_leaves, plan.h_leaves.data(), plan.h_leaves.size() * sizeof(LeafTask),
@@ -1250,7 +1304,10 @@ void Engine::enqueue_terminals(const Plan& plan) {
       // terminal for long rows.
       // Two warps per terminal (the default where there are enough tasks,
       // for short and long hand lists alike) comes first.
-      if (term_group_)
+      if (term_group_ && tile_T_ > 0)
+        launch_tile_terminal(F, plan.d_fast, plan.d_jobs, (int)plan.h_jobs.size(), tile_claims_ + p, tile_T_, term_sms_,
+                             stream_);
+      else if (term_group_)
         launch_group_terminal(F, plan.d_fast, plan.d_units, (int)plan.h_units.size(), (int)plan.h_fast.size(),
                               group_groups_, group_blocks_, stream_);
       else if (term_kernel_ == TK_PANEL)
@@ -1302,7 +1359,7 @@ void Engine::enqueue_up(const Plan& plan, int mode) {
 // up levels (deepest first); the root's value row is copied to root_out.
 void Engine::enqueue_traversal(const Plan& plan, int mode, const float* root_row, float* root_out, bool advance) {
   launch_traversal_start(alive(plan.p), (int)plan.nslots, nullptr, 0, reach_, root_row, stride_,
-                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, stream_);
+                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, tile_claims_, stream_);
   mark(DCFR_KERNEL_OTHER);
   if (plan.seg) enqueue_segment(nullptr, &plan, mode, root_row, nullptr);
   enqueue_down(plan, mode);
@@ -1327,7 +1384,7 @@ void Engine::enqueue_pair(int mode, float* root_out, bool advance) {
     return;
   }
   launch_traversal_start(alive(0), (int)a.nslots, alive(1), (int)b.nslots, reach_, root_rows_, stride_,
-                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, stream_);
+                         advance ? counter_ : nullptr, disc_table_, disc_len_, cur_disc_, tile_claims_, stream_);
   enqueue_segment(nullptr, &a, mode, root_rows_, nullptr);
   enqueue_down(a, mode);
   enqueue_terminals(a);

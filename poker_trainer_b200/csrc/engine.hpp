@@ -52,6 +52,9 @@ int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_s
 int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, bool multi);
 void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
                            int groups, int max_blocks, cudaStream_t s);
+int tile_terminal_setup(int n0, int n1, int hp0, int hp1);
+void launch_tile_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* jobs, int njobs, uint32_t* counter,
+                          int T, int max_blocks, cudaStream_t s);
 int panel_terminal_setup(int hpo, int hpp, int cstride, int tstride, int T, int& blocks_per_sm);
 int warp_terminal_dyn_setup(int stride, int cstride, int tstride, int max_warps, int& blocks_per_sm);
 void launch_fast_terminal_dyn(const FastArgs& A, const FastTask* tasks, int ntasks, int max_blocks, uint32_t* counter,
@@ -72,10 +75,11 @@ void launch_evaluate(const unsigned long long* masks, uint32_t* out, int n, cuda
 void launch_five_card_counts(unsigned long long* counts, cudaStream_t s);
 // counter non-null: also advance the DCFR iteration (t += 1, the discounts
 // of iteration t from the table into cur).
-// alive2 non-null: also clear the flags of another traversal.
+// alive2 non-null: also clear the flags of another traversal. claims
+// non-null: clear both traversals' job counters.
 void launch_traversal_start(uint32_t* alive, int nslots, uint32_t* alive2, int nslots2, float* reach, const float* root_row, int stride,
                             uint32_t* counter, const DiscountD* table, uint32_t table_len, DiscountD* cur,
-                            cudaStream_t s);
+                            uint32_t* claims, cudaStream_t s);
 // Storage blocks between the device layout and the reference's packed
 // layout; elem_bytes 4 (f32) or 2 (compressed storage).
 void launch_storage_pack(int elem_bytes, const void* dev, void* packed, const StorageBlockD* blocks, int nblocks,
@@ -108,6 +112,8 @@ struct Plan {
   std::vector<FastTask> h_fast;  // one task per terminal
   std::vector<TermUnit> h_units; // runs of h_fast on one layout (warp terminal kernel)
   TermUnit* d_units = nullptr;
+  std::vector<TermUnit> h_jobs;  // the same, in jobs of the tile terminal kernel
+  TermUnit* d_jobs = nullptr;
   std::vector<PanelD> h_panels;  // panels of h_fast (panel terminal kernel)
   PanelD* d_panels = nullptr;
   std::vector<LeafTask> h_leaves; // depth-limited solves: the leaves of this traversal
@@ -299,6 +305,9 @@ class Engine {
   // Short rows: two warps per terminal (terminal_group.cu) instead of one.
   bool term_group_ = false, term_group_auto_ = false;
   int group_groups_ = 0, group_blocks_ = 0, term_sms_ = 0;
+  // Terminals per tile (terminal_tile.cu), 0: no tiles.
+  int tile_T_ = 0;
+  uint32_t* tile_claims_ = nullptr;  // [2] jobs claimed per traverser
   uint32_t* term_counter_ = nullptr;
   // Depth-limited solves: the leaf-value network and its buffers.
   dcfr_mlp* net_ = nullptr;

@@ -378,8 +378,10 @@ void launch_five_card_counts(unsigned long long* counts, cudaStream_t s) {
 __global__ void traversal_start_kernel(uint32_t* __restrict__ alive, int nslots, uint32_t* __restrict__ alive2,
                                        int nslots2, float* __restrict__ reach,
                                        const float* __restrict__ root_row, int stride, uint32_t* counter,
-                                       const DiscountD* table, uint32_t table_len, DiscountD* cur) {
+                                       const DiscountD* table, uint32_t table_len, DiscountD* cur,
+                                       uint32_t* __restrict__ claims) {
   pdl_wait();
+  if (claims && blockIdx.x == 0 && threadIdx.x < 2) claims[threadIdx.x] = 0u;
   if (counter && blockIdx.x == 0 && threadIdx.x == 0) {
     const uint32_t t = *counter + 1;
     *counter = t;
@@ -449,13 +451,13 @@ void launch_storage_unpack(int elem_bytes, void* dev, const void* packed, const 
 
 void launch_traversal_start(uint32_t* alive, int nslots, uint32_t* alive2, int nslots2, float* reach,
                             const float* root_row, int stride, uint32_t* counter, const DiscountD* table, uint32_t table_len, DiscountD* cur,
-                            cudaStream_t s) {
+                            uint32_t* claims, cudaStream_t s) {
   const int threads = 256, rows = nslots > nslots2 ? nslots : nslots2, work = rows > stride / 4 ? rows : stride / 4;
   int blocks = (work + threads - 1) / threads;
   if (blocks > 1184) blocks = 1184;
   if (blocks < 1) blocks = 1;
   launch_dependent(traversal_start_kernel, (unsigned)blocks, (unsigned)threads, 0, s, alive, nslots, alive2, nslots2, reach,
-                   root_row, stride, counter, table, table_len, cur);
+                   root_row, stride, counter, table, table_len, cur, claims);
 }
 
 }  // namespace dcfr

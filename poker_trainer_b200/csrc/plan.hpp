@@ -137,8 +137,12 @@ struct TermUnit {
   uint32_t layout;  // FastTask::board of every task in the run
   uint32_t first;   // first task
   uint32_t count;   // tasks
-  uint32_t pad;
+  uint32_t pad;     // TileClass of its tasks, where the plan orders them by class
 };
+// Tasks that a tile of terminal_tile.cu evaluates alike: batched showdowns
+// with neither tie payoff nor paired fold, other showdowns, folds.
+constexpr int TILE_THREADS = 512;  // threads a block, and most tasks of a job
+enum TileClass : uint32_t { TILE_PLAIN = 0, TILE_GENERAL = 1, TILE_FOLD = 2 };
 
 // A panel of the panel terminal kernel (terminal_panel.cu): `count` (1..T)
 // consecutive fast terminal tasks, all on one layout and all showdowns or
