@@ -404,7 +404,7 @@ struct Batch::Impl {
   cudaGraphExec_t graph = nullptr;
   uint32_t graph_iters = 0;
   int sms = 148, optin = 0;
-  int max_groups = 0, block_blocks = 0;  // group kernel: groups per block; block kernel: blocks
+  int max_groups = 0, group_warps = 2, block_blocks = 0;  // group kernel: groups per block; block kernel: blocks
   uint64_t launches = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0.0;
@@ -756,7 +756,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
     return s;
   }
   int bps = 0;
-  max_groups = group_terminal_setup(stride, cstride, tstride, bps, true);
+  max_groups = group_terminal_setup(stride, cstride, tstride, group_warps, bps, true);
   const int fast_bps = fast_blocks_per_sm(stride, emax, cstride, tstride);
   if (max_groups <= 0 || fast_bps <= 0) {
     s.code = DCFR_ERR_UNSUPPORTED;
@@ -777,7 +777,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
 // Resident blocks per SM of the group terminal kernel with up to `warps`
 // terminals in flight in a block.
 int Batch::Impl::occupancy(int warps) const {
-  return std::max(1, group_terminal_occupancy(stride, cstride, tstride, std::min(warps, max_groups), true));
+  return std::max(1, group_terminal_occupancy(stride, cstride, tstride, std::min(warps, max_groups), group_warps, true));
 }
 
 // A row pass over all spots: the up pass of traverser up_p, then the down
@@ -839,7 +839,7 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
 // All spots' terminals of one traversal: a block per terminal while there
 // are few of them or hand lists so long that few groups fit a block, two warps
 // per terminal otherwise (1081 hands, five groups, us an iteration, block
-// against group kernel: 37 spots 126 against 152, 512 spots 1323 against 1350).
+// against group kernel: 37 spots 126 against 135, 512 spots 1148 against 1134).
 void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t) {
   FastArgs F;
   F.reach = reach;
@@ -861,7 +861,7 @@ void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t) {
     launch_fast_terminal(F, term[p], (int)ntasks[p], block_blocks, stream);
     return;
   }
-  launch_group_terminal(F, term[p], units[p], (int)nunits[p], (int)ntasks[p], std::min(t.warps, max_groups),
+  launch_group_terminal(F, term[p], units[p], (int)nunits[p], (int)ntasks[p], std::min(t.warps, max_groups), group_warps,
                         sms * std::max(t.blocks_per_sm, 1), stream);
 }
 

@@ -472,7 +472,7 @@ Status Engine::ensure_fast_layouts() {
   term_sms_ = sms;
   {
     int bps = 0;
-    group_groups_ = group_terminal_setup(stride_, fcstride_, tstride_, bps);
+    group_groups_ = group_terminal_setup(stride_, fcstride_, tstride_, group_warps_, bps);
     group_blocks_ = sms * bps;
   }
   term_group_ = want == "group" && group_groups_ > 0;
@@ -1309,7 +1309,7 @@ void Engine::enqueue_terminals(const Plan& plan) {
                              stream_);
       else if (term_group_)
         launch_group_terminal(F, plan.d_fast, plan.d_units, (int)plan.h_units.size(), (int)plan.h_fast.size(),
-                              group_groups_, group_blocks_, stream_);
+                              group_groups_, group_warps_, group_blocks_, stream_);
       else if (term_kernel_ == TK_PANEL)
         launch_panel_terminal(F, plan.d_fast, plan.d_panels, (int)plan.h_panels.size(), panel_T_, panel_E_,
                               panel_blocks_, stream_);

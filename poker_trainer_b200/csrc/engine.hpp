@@ -48,10 +48,10 @@ void launch_warp_terminal64(const FastArgs64& A, const FastTask* tasks, const Te
                             int warps,
                             int max_blocks, cudaStream_t s);
 int warp_terminal_setup(int stride, int cstride, int tstride, int rsize, int max_warps, int& blocks_per_sm);
-int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm, bool multi = false);
-int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, bool multi);
+int group_terminal_setup(int stride, int cstride, int tstride, int& warps, int& blocks_per_sm, bool multi = false);
+int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, int warps, bool multi);
 void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
-                           int groups, int max_blocks, cudaStream_t s);
+                           int groups, int warps, int max_blocks, cudaStream_t s);
 int tile_terminal_setup(int n0, int n1, int hp0, int hp1);
 void launch_tile_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* jobs, int njobs, uint32_t* counter,
                           int T, int max_blocks, cudaStream_t s);
@@ -304,7 +304,7 @@ class Engine {
   int dyn_warps_ = 0, dyn_blocks_ = 0;
   // Short rows: two warps per terminal (terminal_group.cu) instead of one.
   bool term_group_ = false, term_group_auto_ = false;
-  int group_groups_ = 0, group_blocks_ = 0, term_sms_ = 0;
+  int group_groups_ = 0, group_warps_ = 2, group_blocks_ = 0, term_sms_ = 0;
   // Terminals per tile (terminal_tile.cu), 0: no tiles.
   int tile_T_ = 0;
   uint32_t* tile_claims_ = nullptr;  // [2] jobs claimed per traverser

@@ -1,6 +1,6 @@
 // Group-per-terminal evaluation: the fixed-point prefix sums of
 // warp_terminal_task (warp_terminal.cuh) with every terminal evaluated by a
-// group of GROUP_WARPS warps instead of one.
+// group of GW warps (two, or four on long hand lists) instead of one.
 //
 // The warp-per-terminal kernel keeps one terminal in flight per warp, and
 // each terminal needs its own prefix array (8 bytes per layout element) and
@@ -31,19 +31,19 @@
 
 namespace dcfr {
 
-constexpr int GROUP_WARPS = 2;
-constexpr int GROUP_THREADS = 32 * GROUP_WARPS;
-// Groups per block (named barriers 1..GROUP_MAX). Twelve leave 80 registers a
-// thread with no spills; fourteen (72 registers, a few spills) measured 1.5%
-// slower on the flop.
-constexpr int GROUP_MAX = 12;
+// Groups per block (named barriers 1..group_max). 24 warps leave 80 registers a
+// thread with no spills; 28 (72 registers, a few spills) measured 1.5% slower
+// on the flop.
+// Groups of two per SM up to which a group takes four warps.
+constexpr int GROUP_WIDE_MAX = 8;
+constexpr int group_max(int warps) { return 24 / warps; }
 
 // Shared memory of a block: the staged layout (shared by the block's
 // groups), then per group two reach rows, the prefix array, the card-segment
 // start and end prefixes (16 bytes per card) and the warps' partial results.
 struct GroupSmem {
   size_t same, cat, rec, seg, group0, row_bytes, g_off, cst_off, red_off, group_bytes, total;
-  __host__ __device__ GroupSmem(int stride, int cstride, int tstride, int groups) {
+  __host__ __device__ GroupSmem(int stride, int cstride, int tstride, int groups, int warps) {
     auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     same = 0;
     cat = up16(same + (size_t)stride * 2);
@@ -56,51 +56,56 @@ struct GroupSmem {
     const size_t gn = (size_t)cstride + 2 > 56 ? (size_t)cstride + 2 : 56;
     cst_off = g_off + up16(gn * 8);
     red_off = cst_off + up16(52 * 16);
-    group_bytes = red_off + up16((size_t)GROUP_WARPS * 12);
+    group_bytes = red_off + up16((size_t)warps * 12);
     total = group0 + (size_t)groups * group_bytes;
   }
 };
 
+template <int GW>
 __device__ __forceinline__ void group_sync(int id) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(GROUP_THREADS) : "memory");
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(32 * GW) : "memory");
 }
 
 // The group's threads copy the row of `slot` in 16-byte chunks: thread gt
-// takes chunks gt, gt + GROUP_THREADS, ... (the same chunks it reads back
+// takes chunks gt, gt + GT, ... (the same chunks it reads back
 // for its part of the row maximum).
+template <int GW>
 __device__ __forceinline__ void group_row_prefetch(const FastArgs& A, int hpo, uint32_t slot, float* row, int gt) {
+  constexpr int GT = 32 * GW;
   const char* src = reinterpret_cast<const char*>(A.reach + (size_t)slot * A.stride);
   const uint32_t dst = (uint32_t)__cvta_generic_to_shared(row);
-  for (int i = gt; i < hpo / 4; i += GROUP_THREADS)
+  for (int i = gt; i < hpo / 4; i += GT)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 16 * (size_t)i)
                  : "memory");
 }
 
-// One terminal task evaluated by the GROUP_THREADS threads of a group (gt
+// One terminal task evaluated by the GT threads of a group (gt
 // = thread in the group). row: the group's copy of the task's reach row, its
 // own chunks waited for by every thread. next_slot / next_row: the row to
 // request after barrier (1) (NONE32: none), `fetch` entries of it. bfirst: the first segment
 // boundary b >= 1 with seg[b] >= this thread's first scan element.
+template <int GW>
 __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T, const WarpLayout& Y, int hpo, int hpp,
                                            int np, int fetch, const float* row, long long* G, long long* cst,
                                            long long* gsum, float* gmax, int gt, int bar, int bfirst,
                                            uint32_t next_slot, float* next_row) {
+  constexpr int GT = 32 * GW;
   const int lane = gt & 31, w = gt >> 5;
   const int L = Y.L;
   // 1. Row maximum: each thread's own copied chunks, then the group's.
   float mx = 0.0f;
-  for (int i = gt; i < hpo / 4; i += GROUP_THREADS) {
+  for (int i = gt; i < hpo / 4; i += GT) {
     const float4 v = reinterpret_cast<const float4*>(row)[i];
     mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   if (lane == 0) gmax[w] = mx;
-  group_sync(bar);  // (1)
-  if (next_slot != NONE32) group_row_prefetch(A, fetch, next_slot, next_row, gt);
+  group_sync<GW>(bar);  // (1)
+  if (next_slot != NONE32) group_row_prefetch<GW>(A, fetch, next_slot, next_row, gt);
   cp_async_commit();
 #pragma unroll
-  for (int k = 0; k < GROUP_WARPS; k++) mx = fmaxf(mx, gmax[k]);
+  for (int k = 0; k < GW; k++) mx = fmaxf(mx, gmax[k]);
   const int S = scale_exponent(mx);
   const double scale = pow2(S), inv = pow2(-S);
   const double pa = T.a * inv, pb = T.b * inv, pc = T.c * inv, pd = T.d * inv;
@@ -111,20 +116,20 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   if (fold) {
     // eval_fold (eval.rs:40-64): the total and each card's total.
     long long t0 = 0;
-    for (int k = gt; k < Y.seg[1]; k += GROUP_THREADS) t0 += fixed(row[Y.cat[k]], scale);
+    for (int k = gt; k < Y.seg[1]; k += GT) t0 += fixed(row[Y.cat[k]], scale);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) t0 += __shfl_xor_sync(0xffffffffu, t0, d);
     if (lane == 0) gsum[w] = t0;
-    for (int c = gt; c < 52; c += GROUP_THREADS) {
+    for (int c = gt; c < 52; c += GT) {
       long long tc = 0;
       for (int k = Y.seg[1 + c]; k < Y.seg[2 + c]; k++) tc += fixed(row[Y.cat[k]], scale);
       G[c] = tc;
     }
-    group_sync(bar);  // (2)
+    group_sync<GW>(bar);  // (2)
     t0 = 0;
 #pragma unroll
-    for (int k = 0; k < GROUP_WARPS; k++) t0 += gsum[k];
-    for (int h = gt; h < hpp; h += GROUP_THREADS) {
+    for (int k = 0; k < GW; k++) t0 += gsum[k];
+    for (int h = gt; h < hpp; h += GT) {
       float v = 0.0f;
       if (h < np) {
         const uint32_t q = Y.rec[h].w;
@@ -139,7 +144,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
     return;
   }
   // 2. Elements in layout order: E consecutive elements per thread.
-  const int E = ((L + GROUP_THREADS - 1) / GROUP_THREADS) | 1;
+  const int E = ((L + GT - 1) / GT) | 1;
   const int k0 = gt * E, k1 = min(L, k0 + E);
   long long local = 0;
   int k = k0;
@@ -165,10 +170,10 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
     if (lane >= d) inc += y;
   }
   if (lane == 31) gsum[w] = inc;
-  group_sync(bar);  // (2)
+  group_sync<GW>(bar);  // (2)
   long long acc = inc - local, total = 0;
 #pragma unroll
-  for (int q = 0; q < GROUP_WARPS; q++) {
+  for (int q = 0; q < GW; q++) {
     if (q < w) acc += gsum[q];
     total += gsum[q];
   }
@@ -200,7 +205,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
     G[L] = total;  // a card segment's end can be the layout's end
     for (int b = FAST_SEGS - 1; b >= 1 && Y.seg[b] >= L; b--) put(b, total);
   }
-  group_sync(bar);  // (3)
+  group_sync<GW>(bar);  // (3)
 
   // 3. Values in hand order. Boundary 1 closes the strength segment, so T0
   // is card 0's start.
@@ -241,18 +246,18 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   };
   // Two hands per step: both hands' loads are issued before the stores.
   int h = gt;
-  for (; h + GROUP_THREADS < hpp; h += 2 * GROUP_THREADS) {
+  for (; h + GT < hpp; h += 2 * GT) {
     float v0, f0, v1, f1;
     value(h, v0, f0);
-    value(h + GROUP_THREADS, v1, f1);
+    value(h + GT, v1, f1);
     out[h] = v0;
-    out[h + GROUP_THREADS] = v1;
+    out[h + GT] = v1;
     if (fout) {
       fout[h] = f0;
-      fout[h + GROUP_THREADS] = f1;
+      fout[h + GT] = f1;
     }
   }
-  for (; h < hpp; h += GROUP_THREADS) {
+  for (; h < hpp; h += GT) {
     float v0, f0;
     value(h, v0, f0);
     out[h] = v0;
@@ -268,25 +273,26 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
 // MULTI: a batch's spots, a unit each: the players' hand counts and the
 // identical-hand map change with the unit, and rows are fetched to their
 // common stride (a spot's entries past its own hands are zero).
-template <bool MULTI>
-__global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
+template <int GW, bool MULTI>
+__global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
     group_terminal_kernel(FastArgs A, const FastTask* __restrict__ tasks, const TermUnit* __restrict__ units,
                           int nunits, int ntasks) {
+  constexpr int GT = 32 * GW;
   extern __shared__ __align__(16) unsigned char smem_g[];
-  const int NG = (int)blockDim.x / GROUP_THREADS;
-  const GroupSmem L_(A.stride, A.cstride, A.tstride, NG);
+  const int NG = (int)blockDim.x / GT;
+  const GroupSmem L_(A.stride, A.cstride, A.tstride, NG, GW);
   uint16_t* ssame = reinterpret_cast<uint16_t*>(smem_g + L_.same);
   uint16_t* scat = reinterpret_cast<uint16_t*>(smem_g + L_.cat);
   uint4* srec = reinterpret_cast<uint4*>(smem_g + L_.rec);
   uint16_t* sseg = reinterpret_cast<uint16_t*>(smem_g + L_.seg);
-  const int tid = threadIdx.x, grp = tid / GROUP_THREADS, gt = tid - grp * GROUP_THREADS;
+  const int tid = threadIdx.x, grp = tid / GT, gt = tid - grp * GT;
   unsigned char* gb = smem_g + L_.group0 + (size_t)grp * L_.group_bytes;
   float* const row_a = reinterpret_cast<float*>(gb);
   float* const row_b = reinterpret_cast<float*>(gb + L_.row_bytes);
   long long* G = reinterpret_cast<long long*>(gb + L_.g_off);
   long long* cst = reinterpret_cast<long long*>(gb + L_.cst_off);
   long long* gsum = reinterpret_cast<long long*>(gb + L_.red_off);
-  float* gmax = reinterpret_cast<float*>(gb + L_.red_off + GROUP_WARPS * 8);
+  float* gmax = reinterpret_cast<float*>(gb + L_.red_off + GW * 8);
   const int bar = 1 + grp;
 
   const int p = A.p, o = p ^ 1;
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   bool live = false;
   if (next < t1) {
     live = A.alive[tasks[next].slot] != 0;
-    if (live) group_row_prefetch(A, fetch, tasks[next].slot, row_a, gt);
+    if (live) group_row_prefetch<GW>(A, fetch, tasks[next].slot, row_a, gt);
   }
   cp_async_commit();
   for (; u < nunits && (int)units[u].first < t1; u++) {
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
     __syncthreads();
     const WarpLayout Y{ssame, scat, srec, sseg, L};
     // This thread's first segment boundary at or after its first element.
-    const int k0 = gt * (((L + GROUP_THREADS - 1) / GROUP_THREADS) | 1);
+    const int k0 = gt * (((L + GT - 1) / GT) | 1);
     int bfirst = 1;
     while (bfirst < FAST_SEGS && sseg[bfirst] < k0) bfirst++;
     const int end = min(t1, (int)(U.first + U.count));
@@ -362,14 +368,14 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
       float* const nxt_row = buf ? row_a : row_b;
       // Dead subtree (cfr.rs:267-274): row untouched.
       if (live) {
-        group_task(A, tasks[next], Y, hpo, hpp, np, fetch, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
+        group_task<GW>(A, tasks[next], Y, hpo, hpp, np, fetch, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
                    nlive ? tasks[nx].slot : NONE32, nxt_row);
       } else {
         // The group's other warps may still read the previous task's row
         // from the buffer the next row goes to.
         if (nlive) {
-          group_sync(bar);
-          group_row_prefetch(A, fetch, tasks[nx].slot, nxt_row, gt);
+          group_sync<GW>(bar);
+          group_row_prefetch<GW>(A, fetch, tasks[nx].slot, nxt_row, gt);
         }
         cp_async_commit();
       }
@@ -380,39 +386,58 @@ __global__ void __launch_bounds__(GROUP_THREADS* GROUP_MAX, 1)
   cp_async_wait<0>();
 }
 
-size_t group_terminal_smem(int stride, int cstride, int tstride, int groups) {
-  return GroupSmem(stride, cstride, tstride, groups).total;
+size_t group_terminal_smem(int stride, int cstride, int tstride, int groups, int warps) {
+  return GroupSmem(stride, cstride, tstride, groups, warps).total;
 }
 
-// Resident blocks per SM of `groups` groups; 0 if none fits.
-int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, bool multi) {
+using GroupKernel = void (*)(FastArgs, const FastTask*, const TermUnit*, int, int);
+static GroupKernel group_kernel(int warps, bool multi) {
+  if (warps == 4) return multi ? group_terminal_kernel<4, true> : group_terminal_kernel<4, false>;
+  return multi ? group_terminal_kernel<2, true> : group_terminal_kernel<2, false>;
+}
+
+// Resident blocks per SM of `groups` groups of `warps` warps; 0 if none fits.
+int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, int warps, bool multi) {
   int b = 0;
-  const void* fn = multi ? (const void*)group_terminal_kernel<true> : (const void*)group_terminal_kernel<false>;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, groups * GROUP_THREADS,
-                                                    group_terminal_smem(stride, cstride, tstride, groups)) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, group_kernel(warps, multi), groups * warps * 32,
+                                                    group_terminal_smem(stride, cstride, tstride, groups, warps)) !=
+      cudaSuccess)
     return 0;
   return b;
 }
 
-// Groups per block (1..GROUP_MAX) that maximise resident groups per SM, and
-// the blocks per SM at that count; 0 if none fits.
-int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_sm, bool multi) {
+// Warps per terminal, and groups per block that maximise resident groups per
+// SM, and the blocks per SM at that count; 0 groups if none fits. Four warps
+// where shared memory holds no more than eight groups of two (long hand
+// lists): as many warps are resident as registers allow either way (turn, 816 hands,
+// us a traversal's terminals: 86.2 to 84.3).
+int group_terminal_setup(int stride, int cstride, int tstride, int& warps, int& blocks_per_sm, bool multi) {
   int dev = 0, optin = 0;
   blocks_per_sm = 0;
+  warps = 2;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return 0;
-  const void* fn = multi ? (const void*)group_terminal_kernel<true> : (const void*)group_terminal_kernel<false>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return 0;
+  for (int w : {2, 4})
+    if (cudaFuncSetAttribute((const void*)group_kernel(w, multi), cudaFuncAttributeMaxDynamicSharedMemorySize, optin) !=
+        cudaSuccess)
+      return 0;
   int best_g = 0, best_b = 0;
-  for (int g = 1; g <= GROUP_MAX; g++) {
-    const size_t smem = group_terminal_smem(stride, cstride, tstride, g);
-    if (smem > (size_t)optin) break;
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, g * GROUP_THREADS, smem) != cudaSuccess) return 0;
-    if (b > 0 && g * b >= best_g * best_b) {
-      best_g = g;
-      best_b = b;
+  for (int w : {2, 4}) {
+    if (w == 4 && best_g * best_b > GROUP_WIDE_MAX) break;
+    int wg = 0, wb = 0;
+    for (int g = 1; g <= group_max(w); g++) {
+      if (group_terminal_smem(stride, cstride, tstride, g, w) > (size_t)optin) break;
+      const int b = group_terminal_occupancy(stride, cstride, tstride, g, w, multi);
+      if (b > 0 && g * b >= wg * wb) {
+        wg = g;
+        wb = b;
+      }
+    }
+    if (wg > 0) {
+      best_g = wg;
+      best_b = wb;
+      warps = w;
     }
   }
   blocks_per_sm = best_b;
@@ -420,13 +445,13 @@ int group_terminal_setup(int stride, int cstride, int tstride, int& blocks_per_s
 }
 
 void launch_group_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
-                           int groups, int max_blocks, cudaStream_t s) {
+                           int groups, int warps, int max_blocks, cudaStream_t s) {
   if (nunits <= 0 || ntasks <= 0) return;
   // At most one block per task: every block's range is non-empty.
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
-  const size_t smem = group_terminal_smem(A.stride, A.cstride, A.tstride, groups);
-  launch_dependent(A.dims ? group_terminal_kernel<true> : group_terminal_kernel<false>, (unsigned)blocks,
-                   (unsigned)(groups * GROUP_THREADS), smem, s, A, tasks, units, nunits, ntasks);
+  const size_t smem = group_terminal_smem(A.stride, A.cstride, A.tstride, groups, warps);
+  launch_dependent(group_kernel(warps, A.dims != nullptr), dim3((unsigned)blocks), (unsigned)(groups * warps * 32), smem, s,
+                   A, tasks, units, nunits, ntasks);
 }
 
 }  // namespace dcfr
