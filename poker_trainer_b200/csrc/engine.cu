@@ -730,6 +730,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
       } else {
         DownTask t{D_CHANCE_SPLIT, sv, first_slot, nd.nchild, 0, cc_off_[nd.index], nd.factor};
         down[depth].push_back(t);
+        dmax[depth] = std::max<int>(dmax[depth], (int)nd.nchild);
         UpTask u{U_CHANCE_SUM, sv, v, nd.first, nd.nchild, first_slot, 0, cc_off_[nd.index], iso_first_[nd.index],
                  (uint32_t)g.chance[nd.index].ci.size(), 0};
         up[depth].push_back(u);
@@ -1286,8 +1287,8 @@ void Engine::enqueue_down(const Plan& plan, int mode) {
       for (const Plan::Level& lv : plan.seg_down[l])
         if (lv.count) launch_down(mode, lv.maxa, A, plan.d_down + lv.first, (int)lv.count, hp_[o], stream_);
     if (l < plan.down.size() && plan.down[l].count)
-      launch_down(mode, plan.down[l].maxa, A, plan.d_down + plan.down[l].first, (int)plan.down[l].count, hp_[o],
-                  stream_);
+      launch_chance_down(mode, A, plan.d_down + plan.down[l].first, (int)plan.down[l].count, plan.down[l].maxa, hp_[o],
+                         stream_);
   }
   mark(DCFR_KERNEL_DOWN);
 }
@@ -1343,7 +1344,7 @@ void Engine::enqueue_up(const Plan& plan, int mode) {
   const size_t layers = std::max({plan.tree_layers.size(), plan.down.size(), plan.seg_down.size()});
   for (size_t l = layers; l-- > 0;) {
     if (l < plan.up.size() && plan.up[l].count)
-      launch_up(mode, plan.up[l].maxa, A, plan.d_up + plan.up[l].first, (int)plan.up[l].count, hp_[p], stream_);
+      launch_chance_up(mode, A, plan.d_up + plan.up[l].first, (int)plan.up[l].count, hp_[p], stream_);
     if (l < plan.seg_up.size() && !(l == 0 && plan.seg))
       for (size_t d = plan.seg_up[l].size(); d-- > 0;) {
         const Plan::Level& lv = plan.seg_up[l][d];

@@ -22,6 +22,9 @@ struct RowArgs;
 // Kernel launchers (kernels.cu).
 void launch_down(int mode, int maxa, const RowArgs& A, const DownTask* tasks, int ntasks, int hp, cudaStream_t s);
 void launch_up(int mode, int maxa, const RowArgs& A, const UpTask* tasks, int ntasks, int hp, cudaStream_t s);
+void launch_chance_down(int mode, const RowArgs& A, const DownTask* tasks, int ntasks, int max_children, int hp,
+                        cudaStream_t s);
+void launch_chance_up(int mode, const RowArgs& A, const UpTask* tasks, int ntasks, int hp, cudaStream_t s);
 void launch_fused_down(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees,
                        const DownTask* tasks, int hp, cudaStream_t s);
 void launch_fused_up(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees, const UpTask* tasks,

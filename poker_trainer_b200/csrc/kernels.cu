@@ -52,6 +52,101 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) up_kernel(RowArgs A, const Up
   pdl_trigger();
 }
 
+// A layer's chance nodes where they are few (a turn has as many as its root
+// street has calls, about 15): a block per node leaves the GPU idle while each
+// thread writes 48 children one after another, or sums 4 hands over them a
+// batch of rows at a time; both are bound by the latency of those chains.
+// Splits take a block per `group` children of a node, sums a thread per hand.
+// A turn of 15 nodes, 48 children and 816 hands, us an iteration: 331, with
+// the splits 320, with both 300.
+__global__ void __launch_bounds__(ROW_MAX_THREADS) chance_down_kernel(RowArgs A, const DownTask* __restrict__ tasks,
+                                                                      int chunks, int groups, uint32_t group) {
+  const int t = blockIdx.x / (chunks * groups), r = blockIdx.x - t * chunks * groups, ch = r / groups, g = r - ch * groups;
+  const DownTask T = tasks[t];
+  pdl_wait();
+  pdl_trigger();
+  down_item<M_CFR, 1, D_CHANCE_SPLIT>(A, T, (ch * (int)blockDim.x + (int)threadIdx.x) * VEC, threadIdx.x & 31, nullptr,
+                                      (uint32_t)g * group, ((uint32_t)g + 1) * group);
+}
+
+// up_item<U_CHANCE_SUM>'s additions in its order. What does not change during
+// a solve (cards, isomorphic hands) is read before the wait, children's rows
+// together with their liveness after it.
+constexpr int CHANCE_SUM_THREADS = 64, DECK = 52;
+__global__ void __launch_bounds__(CHANCE_SUM_THREADS) chance_up_kernel(RowArgs A, const UpTask* __restrict__ tasks,
+                                                                       int chunks) {
+  constexpr uint16_t BLOCKED = 0xFFFFu;
+  __shared__ uint8_t cards[DECK], on[DECK], iso_child[DECK], iso_pair[DECK];
+  __shared__ uint16_t iso_hand[DECK][CHANCE_SUM_THREADS];
+  const int t = blockIdx.x / chunks, ch = blockIdx.x - t * chunks, tid = (int)threadIdx.x;
+  const UpTask T = tasks[t];
+  const int p = A.p, hp = pick(p, A.hp), np = pick(p, A.n), h = ch * CHANCE_SUM_THREADS + tid;
+  const size_t stride = (size_t)A.stride;
+  const uint8_t* hc1 = pick(p, A.hc1);
+  const uint8_t* hc2 = pick(p, A.hc2);
+  const int n = (int)T.nchild, niso = (int)T.iso_count;
+  if (tid < n) cards[tid] = A.chance_cards[T.cards + tid];
+  if (tid < niso) {
+    const IsoRefD ref = A.iso[T.iso_first + tid];
+    iso_child[tid] = (uint8_t)ref.ci;
+    iso_pair[tid] = ref.pair;
+  }
+  __syncthreads();
+  const int hi = min(h, hp - 1), hn = min(h, np - 1);
+  const uint8_t m1 = hc1[hi], m2 = hc2[hi];
+  constexpr int BI = 13;  // isomorphic cards at a time
+  for (int k0 = 0; k0 < niso; k0 += BI) {
+    uint16_t q[BI];
+    uint8_t q1[BI], q2[BI];
+#pragma unroll
+    for (int k = 0; k < BI; k++) q[k] = A.perm[(size_t)(p * 6 + iso_pair[min(k0 + k, niso - 1)]) * stride + hn];
+#pragma unroll
+    for (int k = 0; k < BI; k++) {
+      q1[k] = hc1[q[k]];
+      q2[k] = hc2[q[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < BI; k++)
+      if (k0 + k < niso) {
+        const uint8_t card = cards[iso_child[k0 + k]];
+        iso_hand[k0 + k][tid] = (q1[k] == card) | (q2[k] == card) | (h >= np) ? BLOCKED : q[k];
+      }
+  }
+  pdl_wait();
+  pdl_trigger();
+  const bool live = A.alive[T.slot] != 0;
+  if (tid < n) on[tid] = A.alive[T.child_slot + tid] != 0;
+  const float* rows = A.vals + (size_t)T.child * stride;
+  double acc = 0.0;
+  constexpr int B = 26;  // children at a time
+  for (int i0 = 0; i0 < n; i0 += B) {
+    float v[B];
+#pragma unroll
+    for (int i = 0; i < B; i++) v[i] = rows[(size_t)min(i0 + i, n - 1) * stride + hi];
+    if (i0 == 0) __syncthreads();  // on[]
+#pragma unroll
+    for (int i = 0; i < B; i++) {
+      const int c = min(i0 + i, n - 1), card = cards[c];
+      const bool add = (i0 + i < n) & (on[c] != 0) & (m1 != card) & (m2 != card);
+      acc += (double)(add ? v[i] : 0.0f);  // acc is never -0: adding 0 leaves it
+    }
+  }
+  for (int k0 = 0; k0 < niso; k0 += BI) {
+    float x[BI];
+    bool add[BI];
+#pragma unroll
+    for (int k = 0; k < BI; k++) {
+      const int r = min(k0 + k, niso - 1);
+      const uint16_t q = iso_hand[r][tid];
+      add[k] = (k0 + k < niso) & (q != BLOCKED) & (on[iso_child[r]] != 0);
+      x[k] = rows[(size_t)iso_child[r] * stride + (q != BLOCKED ? q : 0)];
+    }
+#pragma unroll
+    for (int k = 0; k < BI; k++) acc += (double)(add[k] ? x[k] : 0.0f);
+  }
+  if (live && h < hp) A.vals[(size_t)T.node * stride + h] = (float)acc;
+}
+
 // Fused river subtrees: one block per subtree walks its nodes (see
 // FusedTree). Every thread keeps the same 4 hands throughout, so a node's
 // rows are produced and consumed by the same threads; the barrier between
@@ -350,6 +445,32 @@ void launch_up(int mode, int maxa, const RowArgs& A, const UpTask* tasks, int nt
   if (mode == M_CFR) launch_up_m<M_CFR>(maxa, A, tasks, ntasks, hp, s);
   else if (mode == M_BR) launch_up_m<M_BR>(maxa, A, tasks, ntasks, hp, s);
   else launch_up_m<M_AVG>(maxa, A, tasks, ntasks, hp, s);
+}
+
+// Chance nodes of a layer up to which they take the kernels for few: four a
+// multiprocessor. A flop's second layer has more, and a block per node and 4
+// hands a thread is faster there (us an iteration, against the kernels for few
+// on both layers: 1472 nodes of 6 children, 1176 hands 1872 against 1908; 4356
+// nodes, 48 children 15365 against 15533).
+constexpr int CHANCE_FEW = 592;
+
+// A layer's chance nodes, their largest having max_children.
+void launch_chance_down(int mode, const RowArgs& A, const DownTask* tasks, int ntasks, int max_children, int hp,
+                        cudaStream_t s) {
+  if (ntasks <= 0) return;
+  if (ntasks > CHANCE_FEW) return launch_down(mode, 1, A, tasks, ntasks, hp, s);
+  const int threads = row_threads(hp), chunks = (hp + threads * VEC - 1) / (threads * VEC);
+  const uint32_t group = 4;
+  const int groups = (max_children + (int)group - 1) / (int)group;
+  launch_dependent(chance_down_kernel, dim3((unsigned)(ntasks * chunks * groups)), (unsigned)threads, 0, s, A, tasks,
+                   chunks, groups, group);
+}
+
+void launch_chance_up(int mode, const RowArgs& A, const UpTask* tasks, int ntasks, int hp, cudaStream_t s) {
+  if (ntasks <= 0) return;
+  if (ntasks > CHANCE_FEW) return launch_up(mode, 1, A, tasks, ntasks, hp, s);
+  const int chunks = (hp + CHANCE_SUM_THREADS - 1) / CHANCE_SUM_THREADS;
+  launch_dependent(chance_up_kernel, dim3((unsigned)(ntasks * chunks)), CHANCE_SUM_THREADS, 0, s, A, tasks, chunks);
 }
 
 void launch_strength(const uint8_t* boards, int nboards, const uint8_t* hc1_0, const uint8_t* hc2_0,

@@ -93,9 +93,10 @@ __device__ __forceinline__ float block_max(float v, int& phase) {
 // (cfr.rs:448-456).
 // One warp's item: hands [h0, h0 + 128) of one node, 4 per lane.
 // COMP: compressed storage (T.cards holds the node's scale slot); the whole
-// block takes part in every call.
+// block takes part in every call. A chance node's children [c0, c1) only.
 template <int MODE, int MAXA, int KIND, bool COMP = false>
-__device__ __forceinline__ void down_item(const RowArgs& A, const DownTask& T, int h0, int lane, int* phase = nullptr) {
+__device__ __forceinline__ void down_item(const RowArgs& A, const DownTask& T, int h0, int lane, int* phase = nullptr,
+                                          uint32_t c0 = 0, uint32_t c1 = NONE32) {
   const uint32_t live = A.alive[T.in_slot];
   if (live == 0) return;  // dead subtree: children stay dead
   const int o = A.p ^ 1;
@@ -222,7 +223,8 @@ __device__ __forceinline__ void down_item(const RowArgs& A, const DownTask& T, i
       oc2 = *reinterpret_cast<const uchar4*>(pick(o, A.hc2) + h0);
     }
     const uint8_t* cards = A.chance_cards + T.cards;
-    for (uint32_t i = 0; i < T.nchild; i++) {
+    const uint32_t end = min(c1, T.nchild);
+    for (uint32_t i = c0; i < end; i++) {
       const uint8_t card = cards[i];
       float4 c;
 #pragma unroll
