@@ -245,7 +245,11 @@ Status Engine::init() {
   CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ev0_));
   CK(cudaEventCreate(&ev1_));
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
   CK(segment_setup());
+  CK(fused_setup());
   hp_[0] = pad8(g.n[0]);
   hp_[1] = pad8(g.n[1]);
   stride_ = std::max(hp_[0], hp_[1]);
@@ -556,10 +560,10 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   };
   // A segment runs fused only where its layer has at least
   // FUSE_MIN_SEGMENTS segments (one block each fills the GPU) and it has at
-  // most FUSE_MAX_NODES decision nodes. Others (the traversal's root
+  // most FUSED_MAX_NODES decision nodes. Others (the traversal's root
   // segment, wide segments) run level by level: one launch per depth, with
   // many blocks per node.
-  constexpr uint32_t FUSE_MAX_NODES = 48, FUSE_MIN_SEGMENTS = 16;
+  constexpr uint32_t FUSE_MIN_SEGMENTS = 16;
   // The traversal's nodes in id order. build_game appends a node's children
   // after it, so ids grow from parent to child and a pass in id order visits
   // every parent before its children (the reverse pass, children first).
@@ -615,7 +619,7 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
     }
   }
   auto fused_segment = [&](uint32_t v, uint32_t layer) {
-    return seg_size[v] <= FUSE_MAX_NODES && layer < layer_segments.size() &&
+    return seg_size[v] <= (uint32_t)FUSED_MAX_NODES && layer < layer_segments.size() &&
            layer_segments[layer] >= FUSE_MIN_SEGMENTS;
   };
   std::vector<std::vector<std::vector<DownTask>>> sdown;  // wide segments: [layer][depth]
@@ -816,17 +820,21 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   plan.h_fup.reserve(fup.size());
   plan.h_trees.reserve(ntrees);
   plan.tree_layers.clear();
+  std::vector<uint16_t> local(next_slot, 0);  // slot within its segment
   for (uint32_t t : order) {
     const uint32_t l = tree_layer[t];
     if (plan.tree_layers.size() <= l) plan.tree_layers.resize(l + 1, {(uint32_t)plan.h_trees.size(), 0u});
     plan.tree_layers[l].second++;
     FusedTree F{(uint32_t)plan.h_fdown.size(), 0, (uint32_t)plan.h_fup.size(), 0};
     uint32_t prev = 0;
+    uint16_t nlocal = 1;
     for (uint32_t i = fd_off[t]; i < fd_off[t + 1]; i++) {
       const FDown& x = fdown[fd_idx[i]];
       DownTask T = x.t;
       if (i > fd_off[t] && x.depth != prev) T.kind |= LEVEL_BREAK;
       prev = x.depth;
+      T.kind |= (uint32_t)local[T.in_slot] << LOCAL_SHIFT;
+      for (uint32_t a = 0; a < T.nchild; a++) local[T.out_slot + a] = nlocal++;
       plan.h_fdown.push_back(T);
     }
     // Up tasks deepest level first, discovery order within a level: the
@@ -1207,6 +1215,7 @@ void Engine::row_args(int p, RowArgs& A) const {
   A.iso = iso_;
   A.disc = cur_disc_;
   A.stride = stride_;
+  A.sms = sms_;
   A.p = p;
 }
 

@@ -25,6 +25,7 @@ void launch_up(int mode, int maxa, const RowArgs& A, const UpTask* tasks, int nt
 void launch_chance_down(int mode, const RowArgs& A, const DownTask* tasks, int ntasks, int max_children, int hp,
                         cudaStream_t s);
 void launch_chance_up(int mode, const RowArgs& A, const UpTask* tasks, int ntasks, int hp, cudaStream_t s);
+cudaError_t fused_setup();
 void launch_fused_down(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees,
                        const DownTask* tasks, int hp, cudaStream_t s);
 void launch_fused_up(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees, const UpTask* tasks,
@@ -307,7 +308,7 @@ class Engine {
   int dyn_warps_ = 0, dyn_blocks_ = 0;
   // Short rows: two warps per terminal (terminal_group.cu) instead of one.
   bool term_group_ = false, term_group_auto_ = false;
-  int group_groups_ = 0, group_warps_ = 2, group_blocks_ = 0, term_sms_ = 0;
+  int group_groups_ = 0, group_warps_ = 2, group_blocks_ = 0, term_sms_ = 0, sms_ = 1;
   // Terminals per tile (terminal_tile.cu), 0: no tiles.
   int tile_T_ = 0;
   uint32_t* tile_claims_ = nullptr;  // [2] jobs claimed per traverser

@@ -147,42 +147,6 @@ __global__ void __launch_bounds__(CHANCE_SUM_THREADS) chance_up_kernel(RowArgs A
   if (live && h < hp) A.vals[(size_t)T.node * stride + h] = (float)acc;
 }
 
-// Fused river subtrees: one block per subtree walks its nodes (see
-// FusedTree). Every thread keeps the same 4 hands throughout, so a node's
-// rows are produced and consumed by the same threads; the barrier between
-// down levels publishes the children's liveness flags.
-template <int MODE, int MAXA, bool COMP>
-__global__ void __launch_bounds__(ROW_MAX_THREADS) fused_down_kernel(RowArgs A, const FusedTree* __restrict__ trees,
-                                                                     const DownTask* __restrict__ tasks) {
-  const FusedTree F = trees[blockIdx.x];
-  pdl_wait();
-  const int h0 = (int)threadIdx.x * VEC, lane = threadIdx.x & 31;
-  int phase = 0;  // block_max scratch row (compressed storage)
-#pragma unroll 1
-  for (uint32_t i = 0; i < F.down_count; i++) {
-    const DownTask T = tasks[F.down_first + i];
-    if (T.kind & LEVEL_BREAK) __syncthreads();
-    down_item<MODE, MAXA, D_OPP_SPLIT, COMP>(A, T, h0, lane, &phase);
-  }
-  pdl_trigger();
-}
-
-template <int MODE, int MAXA, bool COMP>
-__global__ void __launch_bounds__(ROW_MAX_THREADS) fused_up_kernel(RowArgs A, const FusedTree* __restrict__ trees,
-                                                                   const UpTask* __restrict__ tasks) {
-  const FusedTree F = trees[blockIdx.x];
-  pdl_wait();
-  const int h0 = (int)threadIdx.x * VEC;
-  int phase = 0;  // block_max scratch row (compressed storage)
-#pragma unroll 1
-  for (uint32_t i = 0; i < F.up_count; i++) {
-    const UpTask T = tasks[F.up_first + i];
-    if ((T.kind & KIND_MASK) == U_OWN) up_item<MODE, MAXA, U_OWN, COMP>(A, T, h0, &phase);
-    else up_item<MODE, MAXA, U_OPP_SUM>(A, T, h0);
-  }
-  pdl_trigger();
-}
-
 // ------------------------------------------------------------ setup kernels
 // 7-card strength (crates/holdem/src/eval.rs:104-198): category<<26 | payload.
 __device__ __forceinline__ uint32_t hb(uint32_t x) { return 31u - (uint32_t)__clz(x); }
@@ -386,51 +350,6 @@ static void launch_up_m(int maxa, const RowArgs& A, const UpTask* tasks, int nta
   if (maxa <= 4) return launch_level(up_kernel<MODE, 4, false>, A, tasks, ntasks, hp, s);
   if (maxa <= 8) return launch_level(up_kernel<MODE, 8, false>, A, tasks, ntasks, hp, s);
   launch_level(up_kernel<MODE, MAX_ACTIONS, false>, A, tasks, ntasks, hp, s);
-}
-
-template <typename K, typename Task>
-static void launch_fused(K kernel, const RowArgs& A, const FusedTree* trees, int ntrees, const Task* tasks, int hp,
-                         cudaStream_t s) {
-  launch_dependent(kernel, (unsigned)ntrees, (unsigned)row_threads(hp), 0, s, A, trees, tasks);
-}
-
-template <int MODE>
-static void launch_fused_m(bool up, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees,
-                           const DownTask* dt, const UpTask* ut, int hp, cudaStream_t s) {
-  if (A.compressed) {
-    if (up) {
-      if (maxa <= 4) return launch_fused(fused_up_kernel<MODE, 4, true>, A, trees, ntrees, ut, hp, s);
-      if (maxa <= 8) return launch_fused(fused_up_kernel<MODE, 8, true>, A, trees, ntrees, ut, hp, s);
-      return launch_fused(fused_up_kernel<MODE, MAX_ACTIONS, true>, A, trees, ntrees, ut, hp, s);
-    }
-    if (maxa <= 4) return launch_fused(fused_down_kernel<MODE, 4, true>, A, trees, ntrees, dt, hp, s);
-    if (maxa <= 8) return launch_fused(fused_down_kernel<MODE, 8, true>, A, trees, ntrees, dt, hp, s);
-    return launch_fused(fused_down_kernel<MODE, MAX_ACTIONS, true>, A, trees, ntrees, dt, hp, s);
-  }
-  if (up) {
-    if (maxa <= 4) return launch_fused(fused_up_kernel<MODE, 4, false>, A, trees, ntrees, ut, hp, s);
-    if (maxa <= 8) return launch_fused(fused_up_kernel<MODE, 8, false>, A, trees, ntrees, ut, hp, s);
-    return launch_fused(fused_up_kernel<MODE, MAX_ACTIONS, false>, A, trees, ntrees, ut, hp, s);
-  }
-  if (maxa <= 4) return launch_fused(fused_down_kernel<MODE, 4, false>, A, trees, ntrees, dt, hp, s);
-  if (maxa <= 8) return launch_fused(fused_down_kernel<MODE, 8, false>, A, trees, ntrees, dt, hp, s);
-  launch_fused(fused_down_kernel<MODE, MAX_ACTIONS, false>, A, trees, ntrees, dt, hp, s);
-}
-
-void launch_fused_down(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees,
-                       const DownTask* tasks, int hp, cudaStream_t s) {
-  if (ntrees <= 0) return;
-  if (mode == M_CFR) launch_fused_m<M_CFR>(false, maxa, A, trees, ntrees, tasks, nullptr, hp, s);
-  else if (mode == M_BR) launch_fused_m<M_BR>(false, maxa, A, trees, ntrees, tasks, nullptr, hp, s);
-  else launch_fused_m<M_AVG>(false, maxa, A, trees, ntrees, tasks, nullptr, hp, s);
-}
-
-void launch_fused_up(int mode, int maxa, const RowArgs& A, const FusedTree* trees, int ntrees, const UpTask* tasks,
-                     int hp, cudaStream_t s) {
-  if (ntrees <= 0) return;
-  if (mode == M_CFR) launch_fused_m<M_CFR>(true, maxa, A, trees, ntrees, nullptr, tasks, hp, s);
-  else if (mode == M_BR) launch_fused_m<M_BR>(true, maxa, A, trees, ntrees, nullptr, tasks, hp, s);
-  else launch_fused_m<M_AVG>(true, maxa, A, trees, ntrees, nullptr, tasks, hp, s);
 }
 
 void launch_down(int mode, int maxa, const RowArgs& A, const DownTask* tasks, int ntasks, int hp, cudaStream_t s) {

@@ -53,15 +53,18 @@ struct UpTask {
   uint32_t pad;
 };
 
-// Fused river subtree: the down and up tasks of all its decision nodes,
-// processed by one block (down: BFS order, LEVEL_BREAK on a level's first
-// task; up: deepest level first).
+// Fused segment: the down and up tasks of all its decision nodes, processed by
+// one block (down: BFS order, LEVEL_BREAK on a level's first task, the node's
+// slot counted in the segment above LOCAL_SHIFT: 0 for the root's, then the
+// tasks' children in order; up: deepest level first).
 struct FusedTree {
   uint32_t down_first, down_count;
   uint32_t up_first, up_count;
 };
 constexpr uint32_t LEVEL_BREAK = 0x100u;  // in DownTask::kind
 constexpr uint32_t KIND_MASK = 0xFFu;
+constexpr uint32_t LOCAL_SHIFT = 12;      // of DownTask::kind in a fused segment
+constexpr int FUSED_MAX_NODES = 48;       // decision nodes of a fused segment
 
 struct IsoRefD {
   uint16_t ci;    // canonical child index
@@ -213,6 +216,7 @@ struct RowArgs {
   int hp[2];
   int stride;
   int p;
+  int sms;                // the device's
 };
 
 // Segment passes (segment.cu). Tasks count slots, value rows and storage rows
