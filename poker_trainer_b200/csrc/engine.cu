@@ -389,7 +389,7 @@ Status Engine::init() {
     const size_t enough = (size_t)4 * (size_t)term_sms_;
     term_group_ = full_[0]->h_fast.size() >= enough && full_[1]->h_fast.size() >= enough;
   }
-  if (!(s = dalloc(cur_disc_, 1, "discounts")).ok()) return s;
+  if (!(s = dalloc(cur_disc_, 2, "discounts")).ok()) return s;
   if (!(s = dalloc(counter_, 1, "counter")).ok()) return s;
   CK(cudaMemsetAsync(counter_, 0, 4, stream_));
   if (!(s = ensure_discounts(1024)).ok()) return s;
@@ -486,7 +486,7 @@ Status Engine::ensure_fast_layouts() {
   // works through hundreds of tiles. us a traversal's terminals, tiles against
   // two warps per terminal: flop 8300 against 10820 (23,800 terminals an SM,
   // 470 hands), with sampled cards 521 against 589 (929 an SM); a turn's 79 an
-  // SM lose to staging and part tiles, 99 against 87 (816 hands) and 51 against
+  // SM lose to staging and part tiles, 99 against 87 (777 hands) and 51 against
   // 46 (470).
   tile_T_ = 0;
   if (fast_ && (want == "tile" || (sel == nullptr && g.stats.terminal >= (uint64_t)TILE_TERMINALS_PER_SM * sms)))
@@ -1251,7 +1251,7 @@ void Engine::drop_segment(Plan& plan) {
   plan.kernels += levels - 1;
 }
 
-SegPass Engine::segment_pass(const Plan* up, const Plan* down) const {
+SegPass Engine::segment_pass(const Plan* up, const Plan* down, bool next) const {
   SegPass P{};
   P.slices = (stride_ + SEG_SLICE - 1) / SEG_SLICE;
   const int q = up ? up->p : down->p ^ 1;
@@ -1264,6 +1264,7 @@ SegPass Engine::segment_pass(const Plan* up, const Plan* down) const {
   }
   if (down) {
     row_args(down->p, P.down);
+    if (next) P.down.disc = cur_disc_ + 1;
     P.D = down->res;
     P.down_deferred = down->d_deferred;
   }
@@ -1272,9 +1273,10 @@ SegPass Engine::segment_pass(const Plan* up, const Plan* down) const {
 
 // A segment pass: the up pass of `up`'s root segment (its value row to
 // root_out, if given), then the down pass of `down`'s from root_row; either
-// may be null.
-void Engine::enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out) {
-  SegPass P = segment_pass(up, down);
+// may be null. next: the down pass begins the next iteration.
+void Engine::enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out,
+                             bool next) {
+  SegPass P = segment_pass(up, down, next);
   P.root_out = root_out;
   P.roots = root_row;
   launch_segment(mode, std::max(up ? up->seg_maxa : 1, down ? down->seg_maxa : 1), P, stream_);
@@ -1283,10 +1285,11 @@ void Engine::enqueue_segment(const Plan* up, const Plan* down, int mode, const f
 // Down levels below the root segment pass (or all, without one): segment
 // layer l (fused segments, then wide ones level by level), then the chance
 // nodes of layer l.
-void Engine::enqueue_down(const Plan& plan, int mode) {
+void Engine::enqueue_down(const Plan& plan, int mode, bool next) {
   const int o = plan.p ^ 1;
   RowArgs A;
   row_args(plan.p, A);
+  if (next) A.disc = cur_disc_ + 1;
   const size_t layers = std::max({plan.tree_layers.size(), plan.down.size(), plan.seg_down.size()});
   for (size_t l = 0; l < layers; l++) {
     if (l < plan.tree_layers.size() && plan.tree_layers[l].second)
@@ -1303,12 +1306,13 @@ void Engine::enqueue_down(const Plan& plan, int mode) {
 }
 
 // Terminals and leaves of a traversal.
-void Engine::enqueue_terminals(const Plan& plan) {
+void Engine::enqueue_terminals(const Plan& plan, const PassTurn& turn) {
   const int p = plan.p;
   if (fast_) {
     if (!plan.h_fast.empty()) {
       FastArgs F;
       fast_args(p, F);
+      F.turn = turn;
       // Panels of T terminals per block; or (a selectable alternative) a
       // warp per terminal for short rows and one block-wide scan per
       // terminal for long rows.
@@ -1338,6 +1342,7 @@ void Engine::enqueue_terminals(const Plan& plan) {
   } else if (!plan.h_fast.empty()) {
     FastArgs F;
     fast_args(p, F);
+    F.turn = turn;
     launch_exact_terminal(F, plan.d_fast, (int)plan.h_fast.size(), (uint32_t)g.boards.size(), exact_blocks_, stream_);
   }
   enqueue_leaves(plan);
@@ -1404,6 +1409,54 @@ void Engine::enqueue_pair(int mode, float* root_out, bool advance) {
   enqueue_terminals(b);
   enqueue_up(b, mode);
   enqueue_segment(&b, nullptr, mode, nullptr, out1);
+}
+
+// Whether iterations may be chained as enqueue_rolled does: both root segments
+// run as passes, and the terminal kernels are ones that do a PassTurn.
+bool Engine::rolls() const {
+  const Plan &a = *full_[0], &b = *full_[1];
+  if (!a.seg || !b.seg || a.h_fast.empty() || b.h_fast.empty()) return false;
+  if (!fast_) return true;
+  if (term_group_) return tile_T_ == 0;
+  return term_kernel_ != TK_PANEL && term_kernel_ != TK_WARP && !term_dynamic_;
+}
+
+// n iterations in a row: the up pass that ends one and the down pass that
+// begins the next share a segment pass, and a start kernel runs only before
+// the first; the terminal kernels do what it would (PassTurn). An iteration is
+// four launches instead of six, which on a river take 3 to 5 us each whatever
+// its size. Solves against separate iterations, us: river of 1081 hands, 100
+// iterations 2678 to 2507; of 245 hands, 10 iterations 303 to 285; of 1081 in
+// exact precision, 10 iterations 623 to 590; turn of 440 hands, 40 iterations
+// 8876 to 8739.
+void Engine::enqueue_rolled(uint32_t n) {
+  const Plan &a = *full_[0], &b = *full_[1];
+  launch_traversal_start(alive(0), (int)a.nslots, alive(1), (int)b.nslots, reach_, root_rows_, stride_, counter_,
+                         disc_table_, disc_len_, cur_disc_, tile_claims_, stream_);
+  enqueue_segment(nullptr, &a, M_CFR, root_rows_, nullptr);
+  PassTurn turn;
+  turn.counter = counter_;
+  turn.table = disc_table_;
+  turn.table_len = disc_len_;
+  turn.cur = cur_disc_;
+  for (uint32_t i = 0; i < n; i++) {
+    const bool first = i == 0, last = i + 1 == n;
+    enqueue_down(a, M_CFR, !first);
+    turn.clear = alive(1);
+    turn.nclear = first ? 0 : b.nslots;
+    turn.step = first ? TURN_KEEP : TURN_BEGIN;
+    enqueue_terminals(a, turn);
+    enqueue_up(a, M_CFR);
+    enqueue_segment(&a, &b, M_CFR, root_rows_ + stride_, nullptr);
+    enqueue_down(b, M_CFR);
+    turn.clear = alive(0);
+    turn.nclear = last ? 0 : a.nslots;
+    turn.step = last ? TURN_KEEP : TURN_NEXT;
+    enqueue_terminals(b, turn);
+    enqueue_up(b, M_CFR);
+    if (last) enqueue_segment(&b, nullptr, M_CFR, nullptr, nullptr);
+    else enqueue_segment(&b, &a, M_CFR, root_rows_, nullptr, true);
+  }
 }
 
 // Kernels of enqueue_pair: the second start and one segment pass less than
@@ -1554,7 +1607,9 @@ Status Engine::capture_iterations(uint32_t n, cudaGraphExec_t& exec) {
   const auto t0 = std::chrono::steady_clock::now();
   cudaGraph_t graph;
   CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  for (uint32_t i = 0; i < n; i++) enqueue_pair(M_CFR, nullptr, true);
+  if (n > 1 && rolls()) enqueue_rolled(n);
+  else
+    for (uint32_t i = 0; i < n; i++) enqueue_pair(M_CFR, nullptr, true);
   CK(cudaStreamEndCapture(stream_, &graph));
   const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
@@ -1579,7 +1634,7 @@ Status Engine::launch_iterations(uint32_t most, uint32_t& done) {
   done = chunk ? ITER_CHUNK : 1;
   if (!chunk) singles_++;
   CK(cudaGraphLaunch(chunk ? chunk_graph_ : iter_graph_, stream_));
-  launches += (uint64_t)done * (uint64_t)iter_kernels_;
+  launches += (uint64_t)done * (uint64_t)iter_kernels_ - (chunk && rolls() ? 2u * (done - 1) : 0u);
   return Status();
 }
 

@@ -370,7 +370,7 @@ class Engine {
   Status build_plan(uint32_t root, int p, Plan& plan);
   Status upload_plan(Plan& plan);
   Status upload_segment(Plan& plan);
-  SegPass segment_pass(const Plan* up, const Plan* down) const;
+  SegPass segment_pass(const Plan* up, const Plan* down, bool next = false) const;
   static void drop_segment(Plan& plan);
   void row_args(int p, RowArgs& A) const;
   void fast_args(int p, FastArgs& A) const;
@@ -379,9 +379,12 @@ class Engine {
   // Both traversals of an iteration (or of an evaluation).
   void enqueue_pair(int mode, float* root_out, bool advance = false);
   int pair_launches() const;
-  void enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out);
-  void enqueue_down(const Plan& plan, int mode);
-  void enqueue_terminals(const Plan& plan);
+  void enqueue_segment(const Plan* up, const Plan* down, int mode, const float* root_row, float* root_out,
+                       bool next = false);
+  void enqueue_down(const Plan& plan, int mode, bool next = false);
+  void enqueue_terminals(const Plan& plan, const PassTurn& turn = PassTurn());
+  bool rolls() const;
+  void enqueue_rolled(uint32_t n);
   void enqueue_up(const Plan& plan, int mode);
   Status ensure_discounts(uint32_t max_t);
   Status capture_graphs();

@@ -4,14 +4,14 @@
 // down_item / up_item (row_items.cuh), in their order.
 //
 // With f32 storage and wide ranges the passes are bound by memory (a flop of
-// 2456M cells, 1176 hands: 6.3 TB/s of rows and storage); with 16-bit storage
+// 2456M cells, 468 hands: 6.3 TB/s of rows and storage); with 16-bit storage
 // or short hand lists by how many nodes an SM has in flight, each a chain of
 // task, liveness and storage reads. So a segment's tasks and liveness are kept
 // in shared memory, and storage is copied there asynchronously: its 2 x 4
-// rows of 4 cells a thread would take registers (80, two blocks of 320
-// threads an SM; now 56, three or more), and up passes copy the next node's
+// rows of 4 cells a thread would take registers (80, six blocks of 128
+// threads an SM; now at most 56, nine), and up passes copy the next node's
 // rows while they work on one. us an iteration against loads into registers:
-// flop of 873M cells, 16 bits, 1176 hands 15365 to 12014; 2456M cells, f32,
+// flop of 873M cells, 16 bits, 468 hands 15365 to 12014; 2456M cells, f32,
 // 34133 to 31082; 84M cells, sampled deals 1872 to 1762; turns of 14M and 6M
 // cells 300 to 300 and 197 to 184.
 #include <cuda_runtime.h>

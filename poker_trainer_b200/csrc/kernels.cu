@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(ROW_MAX_THREADS) up_kernel(RowArgs A, const Up
 // thread writes 48 children one after another, or sums 4 hands over them a
 // batch of rows at a time; both are bound by the latency of those chains.
 // Splits take a block per `group` children of a node, sums a thread per hand.
-// A turn of 15 nodes, 48 children and 816 hands, us an iteration: 331, with
+// A turn of 15 nodes, 48 children and 777 hands, us an iteration: 331, with
 // the splits 320, with both 300.
 __global__ void __launch_bounds__(ROW_MAX_THREADS) chance_down_kernel(RowArgs A, const DownTask* __restrict__ tasks,
                                                                       int chunks, int groups, uint32_t group) {
@@ -369,7 +369,7 @@ void launch_up(int mode, int maxa, const RowArgs& A, const UpTask* tasks, int nt
 // Chance nodes of a layer up to which they take the kernels for few: four a
 // multiprocessor. A flop's second layer has more, and a block per node and 4
 // hands a thread is faster there (us an iteration, against the kernels for few
-// on both layers: 1472 nodes of 6 children, 1176 hands 1872 against 1908; 4356
+// on both layers: 1472 nodes of 6 children, 468 hands 1872 against 1908; 4356
 // nodes, 48 children 15365 against 15533).
 constexpr int CHANCE_FEW = 592;
 

@@ -6,10 +6,27 @@
 
 #include <cuda_runtime.h>
 
+#include "plan.hpp"
+
 namespace dcfr {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
+
+// PassTurn's work, by one block (block 0 of every terminal kernel has tasks)
+// after its wait.
+__device__ __forceinline__ void turn_pass(const PassTurn& T) {
+  if (blockIdx.x != 0) return;
+  for (uint32_t i = threadIdx.x; i < T.nclear; i += blockDim.x) T.clear[i] = 0u;
+  if (threadIdx.x != 0) return;
+  if (T.step == TURN_NEXT) {
+    const uint32_t t = *T.counter + 1;
+    T.cur[1] = T.table[t < T.table_len ? t : T.table_len - 1];
+  } else if (T.step == TURN_BEGIN) {
+    *T.counter += 1;
+    T.cur[0] = T.cur[1];
+  }
+}
 
 template <typename... P, typename... A>
 inline void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,

@@ -169,6 +169,23 @@ constexpr int FAST_THREADS = 256;
 
 // R is the row type: float for the solve, double for the FP64 best-response
 // oracle (br64.cu).
+// Between two traversals that share a segment pass across the end of an
+// iteration (Engine::enqueue_rolled), a terminal kernel clears the other
+// traverser's liveness flags, whose last reader is done and whose next writer
+// has not begun, and steps the discounts: TURN_NEXT writes the coming
+// iteration's to cur[1], TURN_BEGIN counts that iteration and makes them
+// cur[0].
+enum TurnStep : uint32_t { TURN_KEEP = 0, TURN_NEXT = 1, TURN_BEGIN = 2 };
+struct PassTurn {
+  uint32_t* clear = nullptr;
+  uint32_t nclear = 0;
+  uint32_t step = TURN_KEEP;
+  uint32_t* counter = nullptr;
+  const DiscountD* table = nullptr;
+  uint32_t table_len = 0;
+  DiscountD* cur = nullptr;
+};
+
 template <typename R>
 struct FastArgsT {
   const R* reach;
@@ -181,6 +198,7 @@ struct FastArgsT {
   // A batch's spots (layout 2 * spot): {n0, n1, hp0, hp1} of each, and `same`
   // has rows of `stride` per (spot, traverser). Null: one game, n and hp.
   const int4* dims = nullptr;
+  PassTurn turn;
   int cstride;
   int tstride;
   int emax;              // elements per thread (odd) for the largest layout

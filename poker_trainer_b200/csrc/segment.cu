@@ -159,8 +159,11 @@ __global__ void __launch_bounds__(SEG_WARPS * 32, 2) segment_kernel(const __grid
       if (sl == 0) P.down.alive[ds[0]] = 1u;
     }
   }
-  DiscountD d{};
-  if (MODE == M_CFR) d = *AQ.disc;
+  DiscountD d{}, dd{};  // the up pass's and the down pass's
+  if (MODE == M_CFR) {
+    d = *AQ.disc;
+    dd = do_down ? *P.down.disc : d;
+  }
   copies_landed();
   if (do_up) {
     if (MODE == M_CFR) {
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(SEG_WARPS * 32, 2) segment_kernel(const __grid
               rch[(T.out_slot + a) * SEG_SLICE + lane] = c;
               if (valid) {
                 to[(size_t)a * stride] = c;
-                if (MODE == M_CFR) P.down.sums[T.gstore + (size_t)a * hp + h] = next_sum(s[a], x[a], r, d);
+                if (MODE == M_CFR) P.down.sums[T.gstore + (size_t)a * hp + h] = next_sum(s[a], x[a], r, dd);
               }
             }
           }

@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(EXACT_THREADS) exact_terminal_kernel(FastArgs 
   const int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
   pdl_wait();
   pdl_trigger();
+  turn_pass(A.turn);
   uint32_t staged = NONE32;
   int L = 0;
   for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {

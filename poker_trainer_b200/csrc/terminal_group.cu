@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
   stage(units[u].layout);
   pdl_wait();
   pdl_trigger();
+  turn_pass(A.turn);
   int buf = 0;
   int next = t0 + grp;  // this group's current task
   bool live = false;
@@ -409,7 +410,7 @@ int group_terminal_occupancy(int stride, int cstride, int tstride, int groups, i
 // Warps per terminal, and groups per block that maximise resident groups per
 // SM, and the blocks per SM at that count; 0 groups if none fits. Four warps
 // where shared memory holds no more than eight groups of two (long hand
-// lists): as many warps are resident as registers allow either way (turn, 816 hands,
+// lists): as many warps are resident as registers allow either way (turn, 777 hands,
 // us a traversal's terminals: 86.2 to 84.3).
 int group_terminal_setup(int stride, int cstride, int tstride, int& warps, int& blocks_per_sm, bool multi) {
   int dev = 0, optin = 0;
