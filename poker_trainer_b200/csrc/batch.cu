@@ -6,19 +6,18 @@
 // its tree, storage order and arithmetic are those of the reference solver
 // (crates/solver/src/tree.rs, cfr.rs, river.rs, eval.rs). The spots share one
 // numbering of reach slots, value rows and terminal tasks (rows of one stride,
-// entries past a spot's own hands zero), and an iteration is six launches
-// over all of them: the flags' reset, then for each traversal a row pass and
-// the terminals, the up pass of the first traversal being one launch with
-// the down pass of the second.
+// entries past a spot's own hands zero), and an iteration is four launches
+// over all of them: for each traversal a row pass and the terminals, the up
+// pass of a traversal being one launch with the down pass of the next.
 //   * Row passes (batch_row_kernel): everything is per hand, so a slice of 32
-//     hands of a spot goes through all its nodes on its own, taking each
+//     or 64 hands of a spot goes through all its nodes on its own, taking each
 //     node's rows from global memory; a slice's part in the dead-subtree
 //     rule is deferred as in segment.cu.
 //   * Terminals: the single solve's kernels over all spots' tasks, a unit of
 //     the scan layouts per spot (terminal_group.cu; terminal_fast.cu for few).
 // A persistent block per spot, for whole iterations, left a spot's 400 nodes
 // to 6 warps and the GPU to its longest spots: 37 spots of 1081 hands took
-// 1622 us an iteration where they now take 126, 512 spots 2078 us, now 1300.
+// 1622 us an iteration where they now take 105, 512 spots 2078 us, now 1011.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,7 +63,8 @@ struct BatchPass {
   float* reach;
   float* vals;
   uint32_t* alive[2];       // per traverser
-  const DiscountD* disc;
+  const DiscountD* disc;       // the up pass's
+  const DiscountD* down_disc;
   int up_p, down_p;         // traversers of the two passes, -1: not wanted
   const SegUp* up;
   const SegDown* fix;       // the up traversal's down tasks
@@ -84,6 +84,28 @@ template <bool SHARE>
 struct RowShape {
   static constexpr int WARPS = SHARE ? 8 : 4;
   static constexpr int SLICES = SHARE ? 1 : WARPS;
+  static constexpr int V = SHARE ? 1 : 2;  // hands a lane
+  static constexpr int SLICE = 32 * V;     // hands a slice
+};
+
+// A lane's V hands of a row, by one load or store.
+template <int V>
+struct Row {
+  float x[V];
+  __device__ __forceinline__ static Row load(const float* p) {
+    Row r;
+    if constexpr (V == 1) r.x[0] = *p;
+    else {
+      const float2 t = *reinterpret_cast<const float2*>(p);
+      r.x[0] = t.x;
+      r.x[1] = t.y;
+    }
+    return r;
+  }
+  __device__ __forceinline__ void store(float* p) const {
+    if constexpr (V == 1) *p = x[0];
+    else *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  }
 };
 
 struct RowSmem {
@@ -109,14 +131,18 @@ __device__ __forceinline__ void stage_records(T* dst, const T* src, uint32_t cou
 
 // Bound by the latency of a node's loads (value rows, then the next node's),
 // so the plan records and liveness flags are in shared memory, no load waits
-// for another, and as many warps run as the registers allow without spills
-// (512 spots, us an iteration: 28 warps an SM 1303, 40 with spills 1349; with
-// records and flags read from global memory at 24 warps 1440).
+// for another, a lane has two hands where that leaves enough slices, and as
+// many warps run as the registers allow without spills (512 spots, us an
+// iteration: two hands a lane 28 warps an SM 1193 with spills, 24 warps 1057,
+// 20 warps 1018, 16 warps 1021; four hands 12 warps 1038, 16 warps 1080; one
+// hand 28 warps 1140). A node's work is by its own number of actions, not the
+// batch's largest: 37 spots of up to 8 actions 126 to 113.
 template <int MODE, int MAXA, bool SHARE>
-__global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA <= 8 ? 7 : 6))
+__global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
     batch_row_kernel(const __grid_constant__ BatchPass P) {
   extern __shared__ __align__(16) unsigned char smem_b[];
-  constexpr int W = RowShape<SHARE>::WARPS, GS = RowShape<SHARE>::SLICES;
+  using R = Row<RowShape<SHARE>::V>;
+  constexpr int W = RowShape<SHARE>::WARPS, GS = RowShape<SHARE>::SLICES, V = RowShape<SHARE>::V;
   const RowSmem L(P.max_up, P.max_fix, P.max_down, P.max_slots, GS);
   SegUp* ut = reinterpret_cast<SegUp*>(smem_b + L.up);
   SegDown* ft = reinterpret_cast<SegDown*>(smem_b + L.fix);
@@ -131,7 +157,7 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA
   const int w0 = SHARE ? warp : 0;
   constexpr int WS = SHARE ? W : 1;
   const SpotD S = P.spots[sp];
-  const int h = sl * 32 + lane;
+  const int h = sl * RowShape<SHARE>::SLICE + lane * V;  // the lane's first; hand counts are padded to eights
   const size_t stride = (size_t)P.stride;
   const bool do_up = P.up_p >= 0, do_down = P.down_p >= 0;
   const BatchPart U = pick(do_up ? P.up_p : 0, S.part), D = pick(do_down ? P.down_p : 0, S.part);
@@ -155,8 +181,11 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA
     smem_b[L.any + (i / S.nslots) * P.max_slots + i % S.nslots] = 0;
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   pdl_wait();
-  DiscountD d{};
-  if (MODE == M_CFR) d = *P.disc;
+  DiscountD d{}, dd{};  // the up pass's and the down pass's
+  if (MODE == M_CFR) {
+    d = *P.disc;
+    dd = *P.down_disc;
+  }
   if (do_up)
     for (uint32_t i = threadIdx.x; i < S.nslots; i += W * 32) live[i] = pick(P.up_p, P.alive)[S.slot + i] != 0;
   __syncthreads();
@@ -172,17 +201,27 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA
         for (; m; m &= m - 1) {
           const SegDown& T = ft[b + __ffs(m) - 1];
           if (h >= hpo) continue;
-          const int na = (int)T.nchild;
-          float x[MAXA];
+          by_actions<MAXA>((int)T.nchild, [&](auto most, int na) {
+            constexpr int M = decltype(most)::value;
+            float x[V][M];
 #pragma unroll
-          for (int a = 0; a < MAXA; a++) x[a] = a < na ? P.regrets[T.gstore + (size_t)a * hpo + h] : 0.0f;
-          to_strategy<MAXA, true>(x, na, T.uniform);
+            for (int a = 0; a < M; a++) {
+              const R v = a < na ? R::load(P.regrets + T.gstore + (size_t)a * hpo + h) : R{};
 #pragma unroll
-          for (int a = 0; a < MAXA; a++)
-            if (a < na) {
-              float* s = P.sums + T.gstore + (size_t)a * hpo + h;
-              *s = next_sum(*s, x[a], 0.0f, d);
+              for (int j = 0; j < V; j++) x[j][a] = v.x[j];
             }
+#pragma unroll
+            for (int j = 0; j < V; j++) to_strategy<M, true>(x[j], na, T.uniform);
+#pragma unroll
+            for (int a = 0; a < M; a++)
+              if (a < na) {
+                float* at = P.sums + T.gstore + (size_t)a * hpo + h;
+                R q = R::load(at);
+#pragma unroll
+                for (int j = 0; j < V; j++) q.x[j] = next_sum(q.x[j], x[j][a], 0.0f, d);
+                q.store(at);
+              }
+          });
         }
       }
     }
@@ -192,58 +231,82 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA
       for (uint32_t i = (SHARE ? P.up_levs[U.up_lev + l] - u0 : 0u) + w0; i < e; i += WS) {
         const SegUp& T = ut[i];
         if (live[T.slot] == 0 || h >= hp) continue;  // dead subtree
-        const int na = (int)T.nchild;
         const float* vp = P.vals + (size_t)T.child * stride + h;
-        float v[MAXA], out = 0.0f;
-        if (T.kind == U_OPP_SUM) {
+        R out{};
+        by_actions<MAXA>((int)T.nchild, [&](auto most, int na) {
+          constexpr int M = decltype(most)::value;
+          R v[M];
+          if (T.kind == U_OPP_SUM) {
 #pragma unroll
-          for (int a = 0; a < MAXA; a++)
-            if (a < na) v[a] = vp[(size_t)a * stride];
+            for (int a = 0; a < M; a++)
+              if (a < na) v[a] = R::load(vp + (size_t)a * stride);
 #pragma unroll
-          for (int a = 0; a < MAXA; a++)
-            if (a < na && live[T.child_slot + a] != 0) out += v[a];
-        } else if (MODE == M_BR) {
+            for (int a = 0; a < M; a++)
+              if (a < na && live[T.child_slot + a] != 0)
 #pragma unroll
-          for (int a = 0; a < MAXA; a++)
-            if (a < na) v[a] = vp[(size_t)a * stride];
-          out = v[0];
+                for (int j = 0; j < V; j++) out.x[j] += v[a].x[j];
+          } else if (MODE == M_BR) {
 #pragma unroll
-          for (int a = 1; a < MAXA; a++)
-            if (a < na) out = v[a] > out ? v[a] : out;
-        } else {
-          float* to = (MODE == M_CFR ? P.regrets : P.sums) + T.gstore + h;
-          float r[MAXA];
+            for (int a = 0; a < M; a++)
+              if (a < na) v[a] = R::load(vp + (size_t)a * stride);
+            out = v[0];
 #pragma unroll
-          for (int a = 0; a < MAXA; a++) {
-            v[a] = a < na ? vp[(size_t)a * stride] : 0.0f;
-            r[a] = a < na ? to[(size_t)a * hp] : 0.0f;
-          }
-          if (MODE == M_AVG) {
-            to_strategy<MAXA, false>(r, na, T.uniform);
+            for (int a = 1; a < M; a++)
+              if (a < na)
 #pragma unroll
-            for (int a = 0; a < MAXA; a++) out = a < na ? out + r[a] * v[a] : out;
+                for (int j = 0; j < V; j++) out.x[j] = v[a].x[j] > out.x[j] ? v[a].x[j] : out.x[j];
           } else {
-            own_value<MAXA>(r, v, na, T.uniform, out);
+            float* to = (MODE == M_CFR ? P.regrets : P.sums) + T.gstore + h;
+            float c[V][M], r[V][M];  // child values; regrets or sums
 #pragma unroll
-            for (int a = 0; a < MAXA; a++)
-              if (a < na) to[(size_t)a * hp] = next_regret(r[a], v[a], out, d);
+            for (int a = 0; a < M; a++) {
+              const R x = a < na ? R::load(vp + (size_t)a * stride) : R{};
+              const R y = a < na ? R::load(to + (size_t)a * hp) : R{};
+#pragma unroll
+              for (int j = 0; j < V; j++) {
+                c[j][a] = x.x[j];
+                r[j][a] = y.x[j];
+              }
+            }
+            if (MODE == M_AVG) {
+#pragma unroll
+              for (int j = 0; j < V; j++) {
+                to_strategy<M, false>(r[j], na, T.uniform);
+#pragma unroll
+                for (int a = 0; a < M; a++) out.x[j] = a < na ? out.x[j] + r[j][a] * c[j][a] : out.x[j];
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < V; j++) own_value<M>(r[j], c[j], na, T.uniform, out.x[j]);
+#pragma unroll
+              for (int a = 0; a < M; a++)
+                if (a < na) {
+                  R q;
+#pragma unroll
+                  for (int j = 0; j < V; j++) q.x[j] = next_regret(r[j][a], c[j][a], out.x[j], d);
+                  q.store(to + (size_t)a * hp);
+                }
+            }
           }
-        }
-        P.vals[(size_t)T.gnode * stride + h] = out;
+        });
+        out.store(P.vals + (size_t)T.gnode * stride + h);
       }
       if (SHARE) __syncthreads();
     }
     if (P.root_out && w0 == 0 && h < P.stride)
-      P.root_out[((size_t)sp * 2 + P.up_p) * stride + h] = P.vals[(size_t)S.node * stride + h];
+      R::load(P.vals + (size_t)S.node * stride + h).store(P.root_out + ((size_t)sp * 2 + P.up_p) * stride + h);
   }
   if (do_down) {
     uint32_t* alive = pick(P.down_p, P.alive);
     const int hp = pick(P.down_p ^ 1, S.hp);
     const bool valid = h < hp;
     if (w0 == 0) {
-      const float r = h < P.stride ? P.roots[((size_t)sp * 2 + P.down_p) * stride + h] : 0.0f;
-      if (h < P.stride) P.reach[(size_t)S.slot * stride + h] = r;
-      const bool some = __any_sync(0xffffffffu, valid && r != 0.0f);
+      const R r = h < P.stride ? R::load(P.roots + ((size_t)sp * 2 + P.down_p) * stride + h) : R{};
+      if (h < P.stride) r.store(P.reach + (size_t)S.slot * stride + h);
+      bool some = false;
+#pragma unroll
+      for (int j = 0; j < V; j++) some |= valid && r.x[j] != 0.0f;
+      some = __any_sync(0xffffffffu, some);
       if (lane == 0) {
         any[0] = some ? 1 : 0;
         if (sl == 0) alive[S.slot] = 1u;
@@ -259,33 +322,44 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : (MAXA
         const bool some = any[T.in_slot] != 0;
         float* to = P.reach + (size_t)T.gslot * stride + h;
         if (some) {
-          const float r = valid ? P.reach[(size_t)(S.slot + T.in_slot) * stride + h] : 0.0f;
+          const R r = valid ? R::load(P.reach + (size_t)(S.slot + T.in_slot) * stride + h) : R{};
           const float* from = (MODE == M_CFR ? P.regrets : P.sums) + T.gstore + h;
           float* sums = P.sums + T.gstore + h;
-          float x[MAXA], s[MAXA];
+          uint32_t kids = 0;  // children that a hand of the lane reaches
+          by_actions<MAXA>(na, [&](auto most, int na) {
+            constexpr int M = decltype(most)::value;
+            float x[V][M];
+            R s[M];
 #pragma unroll
-          for (int a = 0; a < MAXA; a++) {
-            x[a] = a < na && valid ? from[(size_t)a * hp] : 0.0f;
-            s[a] = MODE == M_CFR && a < na && valid ? sums[(size_t)a * hp] : 0.0f;
-          }
-          to_strategy<MAXA, MODE == M_CFR>(x, na, T.uniform);
-          uint32_t kids = 0;
+            for (int a = 0; a < M; a++) {
+              const R v = a < na && valid ? R::load(from + (size_t)a * hp) : R{};
+              s[a] = MODE == M_CFR && a < na && valid ? R::load(sums + (size_t)a * hp) : R{};
 #pragma unroll
-          for (int a = 0; a < MAXA; a++)
-            if (a < na) {
-              const float c = x[a] * r;
-              kids |= (__any_sync(0xffffffffu, valid && c != 0.0f) ? 1u : 0u) << a;
-              if (valid) {
-                to[(size_t)a * stride] = c;
-                if (MODE == M_CFR) sums[(size_t)a * hp] = next_sum(s[a], x[a], r, d);
-              }
+              for (int j = 0; j < V; j++) x[j][a] = v.x[j];
             }
-          if (lane < na && (kids >> lane & 1u)) {
+#pragma unroll
+            for (int j = 0; j < V; j++) to_strategy<M, MODE == M_CFR>(x[j], na, T.uniform);
+#pragma unroll
+            for (int a = 0; a < M; a++)
+              if (a < na && valid) {
+                R c;
+#pragma unroll
+                for (int j = 0; j < V; j++) {
+                  c.x[j] = x[j][a] * r.x[j];
+                  kids |= c.x[j] != 0.0f ? 1u << a : 0u;
+                  if (MODE == M_CFR) s[a].x[j] = next_sum(s[a].x[j], x[j][a], r.x[j], dd);
+                }
+                c.store(to + (size_t)a * stride);
+                if (MODE == M_CFR) s[a].store(sums + (size_t)a * hp);
+              }
+          });
+          kids = __reduce_or_sync(0xffffffffu, kids);
+          if (kids >> lane & 1u) {
             any[T.out_slot + lane] = 1;
             alive[T.gslot + lane] = 1u;
           }
         } else if (valid) {
-          for (int a = 0; a < na; a++) to[(size_t)a * stride] = 0.0f;
+          for (int a = 0; a < na; a++) R{}.store(to + (size_t)a * stride);
         }
         if (MODE == M_CFR && lane == 0) P.down_deferred[(size_t)sl * P.n_down + d0 + i] = some ? 0 : 1;
         if (!SHARE) __syncwarp();
@@ -412,17 +486,18 @@ struct Batch::Impl {
   ~Impl();
   Status init(const dcfr_config* cfgs, int count);
   int occupancy(int warps) const;
-  void enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out);
-  void enqueue_terminals(int p, const dcfr_batch_tuning& t);
-  void enqueue(int mode, const dcfr_batch_tuning& t);
-  Status launch(int mode, uint32_t iters, const dcfr_batch_tuning& t);
+  void enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out, bool next = false);
+  void enqueue_terminals(int p, const dcfr_batch_tuning& t, const PassTurn& turn = PassTurn());
+  void enqueue_start(bool advance);
+  Status launch_evaluation(int mode, const dcfr_batch_tuning& t);
+  void enqueue_iteration(bool first, bool last);
   Status ensure_discounts(uint32_t max_t);
   Status capture(uint32_t iters);
   Status run(uint32_t n);
 };
 
-// Kernels of one iteration (or evaluation) of every spot.
-constexpr uint64_t BATCH_LAUNCHES = 6;
+// Kernels of one iteration of every spot, and those before the first.
+constexpr uint64_t BATCH_LAUNCHES = 4, BATCH_START = 2;
 
 Batch::Impl::~Impl() {
   if (stream) cudaStreamSynchronize(stream);
@@ -741,7 +816,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   }
   BK(cudaGetLastError());
   if (!(s = balloc(counter, 1, "batch counter")).ok()) return s;
-  if (!(s = balloc(cur_disc, 1, "batch counter")).ok()) return s;
+  if (!(s = balloc(cur_disc, 2, "batch counter")).ok()) return s;
   BK(cudaMemsetAsync(counter, 0, 4, stream));
   if (!(s = ensure_discounts(1024)).ok()) return s;
   BK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -785,12 +860,11 @@ int Batch::Impl::occupancy(int warps) const {
 // are too few slices to give every warp its own (us an iteration, shared
 // against not: 37 spots of 34 slices 152 against 334, 512 spots 2113 against
 // 1347).
-void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out) {
+void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out, bool next) {
   BatchPass P{};
   P.spots = d_spots;
   P.order = lpt ? order_lpt : order_nat;
   P.nspots = (int)spots.size();
-  P.slices = slices;
   P.stride = stride;
   P.max_slots = max_slots;
   P.regrets = regrets;
@@ -800,6 +874,7 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
   P.alive[0] = alive;
   P.alive[1] = alive + total_slots;
   P.disc = cur_disc;
+  P.down_disc = cur_disc + (next ? 1 : 0);
   P.up_p = up_p;
   P.down_p = down_p;
   if (up_p >= 0) {
@@ -820,7 +895,9 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
     P.max_down = max_down[down_p];
     P.n_down = (uint32_t)ndown[down_p];
   }
-  const bool share = P.nspots * P.slices <= BATCH_SHARE_ITEMS;
+  const bool share = P.nspots * slices <= BATCH_SHARE_ITEMS;
+  const int hands = share ? RowShape<true>::SLICE : RowShape<false>::SLICE;
+  P.slices = (stride + hands - 1) / hands;
   const int per = share ? RowShape<true>::SLICES : RowShape<false>::SLICES;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(P.nspots * ((P.slices + per - 1) / per)));
@@ -840,8 +917,9 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
 // are few of them or hand lists so long that few groups fit a block, two warps
 // per terminal otherwise (1081 hands, five groups, us an iteration, block
 // against group kernel: 37 spots 126 against 135, 512 spots 1148 against 1134).
-void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t) {
+void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t, const PassTurn& turn) {
   FastArgs F;
+  F.turn = turn;
   F.reach = reach;
   F.vals = vals;
   F.alive = alive + (size_t)p * total_slots;
@@ -866,25 +944,47 @@ void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t) {
 }
 
 // One iteration (M_CFR), best-response or average pair of every spot.
-void Batch::Impl::enqueue(int mode, const dcfr_batch_tuning& t) {
-  const bool lpt = t.longest_first != 0;
-  float* out = mode == M_CFR ? nullptr : root_out;
+void Batch::Impl::enqueue_start(bool advance) {
   launch_traversal_start(alive, (int)total_slots, alive + total_slots, (int)total_slots, reach, roots, 0,
-                         mode == M_CFR ? counter : nullptr, disc, disc_len, cur_disc, nullptr, stream);
-  enqueue_rows(mode, -1, 0, lpt, nullptr);
-  enqueue_terminals(0, t);
-  enqueue_rows(mode, 0, 1, lpt, out);
-  enqueue_terminals(1, t);
-  enqueue_rows(mode, 1, -1, lpt, out);
+                         advance ? counter : nullptr, disc, disc_len, cur_disc, nullptr, stream);
 }
 
-// `iters` CFR iterations of every spot (M_CFR), or one best-response or
-// average pair of traversals.
-Status Batch::Impl::launch(int mode, uint32_t iters, const dcfr_batch_tuning& t) {
-  for (uint32_t i = 0; i < iters; i++) enqueue(mode, t);
+// One best-response or average pair of traversals of every spot.
+Status Batch::Impl::launch_evaluation(int mode, const dcfr_batch_tuning& t) {
+  const bool lpt = t.longest_first != 0;
+  enqueue_start(false);
+  enqueue_rows(mode, -1, 0, lpt, nullptr);
+  enqueue_terminals(0, t);
+  enqueue_rows(mode, 0, 1, lpt, root_out);
+  enqueue_terminals(1, t);
+  enqueue_rows(mode, 1, -1, lpt, root_out);
   BK(cudaGetLastError());
-  launches += iters * BATCH_LAUNCHES;
+  launches += BATCH_START + 4;
   return Status();
+}
+
+// An iteration after its first traversal's down pass. The up pass of the
+// second traversal is one launch with the next iteration's first down pass,
+// and the terminal kernels do what a start kernel would (PassTurn), as in
+// Engine::enqueue_rolled (us an iteration against separate ones: 37 spots 113
+// to 105, 512 spots 1018 to 1011).
+void Batch::Impl::enqueue_iteration(bool first, bool last) {
+  const bool lpt = tuning.longest_first != 0;
+  PassTurn turn;
+  turn.counter = counter;
+  turn.table = disc;
+  turn.table_len = disc_len;
+  turn.cur = cur_disc;
+  turn.clear = alive + total_slots;
+  turn.nclear = first ? 0 : (uint32_t)total_slots;
+  turn.step = first ? TURN_KEEP : TURN_BEGIN;
+  enqueue_terminals(0, tuning, turn);
+  enqueue_rows(M_CFR, 0, 1, lpt, nullptr);
+  turn.clear = alive;
+  turn.nclear = last ? 0 : (uint32_t)total_slots;
+  turn.step = last ? TURN_KEEP : TURN_NEXT;
+  enqueue_terminals(1, tuning, turn);
+  enqueue_rows(M_CFR, 1, last ? -1 : 0, lpt, nullptr, !last);
 }
 
 Status Batch::Impl::capture(uint32_t iters) {
@@ -895,32 +995,37 @@ Status Batch::Impl::capture(uint32_t iters) {
   }
   cudaGraph_t g;
   BK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-  Status s = launch(M_CFR, iters, tuning);
-  cudaError_t e = cudaStreamEndCapture(stream, &g);
-  launches -= iters * BATCH_LAUNCHES;
-  if (!s.ok()) return s;
-  BK(e);
+  for (uint32_t i = 0; i < iters; i++) enqueue_iteration(false, false);
+  BK(cudaStreamEndCapture(stream, &g));
   BK(cudaGraphInstantiate(&graph, g, 0));
   cudaGraphDestroy(g);
   graph_iters = iters;
   return Status();
 }
 
+// n iterations: all but the first and the last, and fewer than a graph's left
+// over, in graphs.
 Status Batch::Impl::run(uint32_t n) {
   Status s;
   if (!(s = ensure_discounts(iterations + n + 1)).ok()) return s;
   const uint32_t k = std::max<uint32_t>(tuning.iterations_per_launch, 1);
   if (!(s = capture(k)).ok()) return s;
   BK(cudaEventRecord(ev0, stream));
-  uint32_t done = 0;
-  while (n - done >= k) {
-    BK(cudaGraphLaunch(graph, stream));
-    launches += k * BATCH_LAUNCHES;
-    done += k;
+  if (n > 0) {
+    enqueue_start(true);
+    enqueue_rows(M_CFR, -1, 0, tuning.longest_first != 0, nullptr);
+    launches += BATCH_START + (uint64_t)n * BATCH_LAUNCHES;
   }
-  if (done < n) {
-    if (!(s = launch(M_CFR, n - done, tuning)).ok()) return s;
+  for (uint32_t i = 0; i < n;) {
+    if (i > 0 && n - 1 - i >= k) {
+      BK(cudaGraphLaunch(graph, stream));
+      i += k;
+    } else {
+      enqueue_iteration(i == 0, i + 1 == n);
+      i++;
+    }
   }
+  BK(cudaGetLastError());
   BK(cudaEventRecord(ev1, stream));
   BK(cudaEventSynchronize(ev1));
   float ms = 0.0f;
@@ -1046,7 +1151,7 @@ Status Batch::autotune(uint32_t trial_iterations, dcfr_batch_tuning& best) {
 Status Batch::root_values(int mode, std::vector<double>& out) {
   Impl& I = *impl_;
   Status s;
-  if (!(s = I.launch(mode, 1, I.tuning)).ok()) return s;
+  if (!(s = I.launch_evaluation(mode, I.tuning)).ok()) return s;
   std::vector<float> rows(I.spots.size() * 2 * I.stride);
   BK(cudaMemcpyAsync(rows.data(), I.root_out, rows.size() * 4, cudaMemcpyDeviceToHost, I.stream));
   BK(cudaStreamSynchronize(I.stream));

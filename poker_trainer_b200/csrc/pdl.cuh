@@ -13,12 +13,12 @@ namespace dcfr {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
-// PassTurn's work, by one block (block 0 of every terminal kernel has tasks)
-// after its wait.
-__device__ __forceinline__ void turn_pass(const PassTurn& T) {
-  if (blockIdx.x != 0) return;
-  for (uint32_t i = threadIdx.x; i < T.nclear; i += blockDim.x) T.clear[i] = 0u;
-  if (threadIdx.x != 0) return;
+// PassTurn's work, by the first `blocks` blocks (those with tasks) of a
+// terminal kernel, after their wait.
+__device__ __forceinline__ void turn_pass(const PassTurn& T, uint32_t blocks = 1) {
+  if (blockIdx.x >= blocks) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T.nclear; i += blocks * blockDim.x) T.clear[i] = 0u;
+  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   if (T.step == TURN_NEXT) {
     const uint32_t t = *T.counter + 1;
     T.cur[1] = T.table[t < T.table_len ? t : T.table_len - 1];

@@ -4,10 +4,22 @@
 // are left out of every sum by selection, with no branch per action.
 #pragma once
 
+#include <type_traits>
+
 #include "plan.hpp"
 #include "row_items.cuh"
 
 namespace dcfr {
+
+// f(most, na): a node's work with arrays of `most` entries. The usual action
+// counts are exact, so that their arrays have no entries to leave out.
+template <int MAXA, typename F>
+__device__ __forceinline__ void by_actions(int na, F&& f) {
+  if (na == 2) f(std::integral_constant<int, 2>(), 2);
+  else if (na == 3) f(std::integral_constant<int, 3>(), 3);
+  else if (MAXA <= 4 || na == 4) f(std::integral_constant<int, 4>(), MAXA <= 4 ? na : 4);
+  else f(std::integral_constant<int, MAXA>(), na);
+}
 
 // Strategy from regrets (regret_match_into, cfr.rs:161-192) or from strategy
 // sums (normalize_in_place, cfr.rs:124-154), in place.

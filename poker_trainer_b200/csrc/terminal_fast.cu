@@ -224,7 +224,10 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   pdl_wait();
   pdl_trigger();
   prefetch(t0, 0);
-  turn_pass(A.turn);
+  if constexpr (!DYN) {
+    const int per = (ntasks + gridDim.x - 1) / gridDim.x;
+    turn_pass(A.turn, (ntasks + per - 1) / per);
+  }
 
   // Three block barriers per terminal: after the row maxima (1), after the
   // scan's warp totals (2) and after the prefixes are written (3). The next

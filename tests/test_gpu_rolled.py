@@ -10,7 +10,7 @@ import pytest
 
 from oracle_api import OracleSolver
 from poker_trainer_b200 import abi, workloads
-from poker_trainer_b200.solver import Solver
+from poker_trainer_b200.solver import BatchSolver, Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +81,16 @@ def test_chained_iterations_equal_single_ones(gpu, board, counts, kernel, monkey
     assert a.exploitability() == b.exploitability()
     a.close()
     b.close()
+
+
+def test_chained_batch_iterations_equal_single_ones(gpu):
+    cfgs = [config(board, counts, "fast") for board, counts in
+            (("Ks7s2dTh4c", (90, 61)), ("AhAd8c3s3h", (300, 33)), ("5h6h7hTcJd", (1, 400)))]
+    a, b = BatchSolver.new(cfgs), BatchSolver.new(cfgs)
+    for its in (1, 2, 3, 27, 60):
+        a.iterate(its)
+        for _ in range(its):
+            b.iterate(1)
+        for k in range(len(cfgs)):
+            assert all(bits_equal(x, y) for x, y in zip(a.download_storage(k), b.download_storage(k)))
+    assert np.array_equal(a.exploitability(), b.exploitability())
