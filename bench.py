@@ -59,8 +59,8 @@ WORKLOADS = {
                     "beta 0 gamma 2"),
     "river": ("river subgame Ks7s2dTh4c: pot 20bb, stacks 90bb, bets 50%/100%/all-in + 2.5x raise, seeded class "
               "ranges (seeds 1000/1001), f32 storage, DCFR alpha 1.5 beta 0 gamma 2"),
-    "batch": ("512 independent river spots in one persistent launch per block of iterations under a captured CUDA "
-              "graph: 5-card boards from seed 3000, pots U[400,6000] chips, stacks U[2000,15000], menus of 1-3 sizes from "
+    "batch": ("512 independent river spots solved together, a few launches an iteration over all spots under captured "
+              "CUDA graphs: 5-card boards from seed 3000, pots U[400,6000] chips, stacks U[2000,15000], menus of 1-3 sizes from "
               "{33,50,75,100,150}% plus all-in for bets and raises, trees of 15-400 nodes, seeded class ranges, f32, "
               "DCFR alpha 1.5 beta 0 gamma 2, 500 iterations each, autotuned launch shape"),
     "learned": ("learned depth-limited flop solve: the flop workload's tree cut at the turn deal, leaves valued by "

@@ -60,7 +60,7 @@ enum { DCFR_STORAGE_F32 = 0, DCFR_STORAGE_COMPRESSED = 1, DCFR_STORAGE_AUTO = 2 
 /* GpuPrecision (crates/solver/src/gpu/mod.rs:51-63). FAST (the default, as
  * in the reference) evaluates terminals with exact 64-bit fixed-point sums of
  * the f32 reach, which agree with the CPU's sequential f64 sums except for
- * rare one-rounding-step differences; EXACT sweeps in the CPU's f64
+ * rare one-rounding-step differences; EXACT sums in the CPU's f64
  * operation order and is bit-identical to the CPU solver. */
 enum { DCFR_PRECISION_FAST = 0, DCFR_PRECISION_EXACT = 1 };
 
@@ -399,8 +399,8 @@ int dcfr_last_solve_ms(const dcfr_solver* s, double* ms);
 int dcfr_setup_profile_get(const dcfr_solver* s, dcfr_setup_profile* out);
 
 /* Measurement hook, no counterpart in the reference: the terminal kernel
- * this handle's f32 traversals launch (DCFR_TERMINAL_*; GROUP: two warps per
- * terminal), and for the panel kernel the terminals evaluated together per
+ * this handle's f32 traversals launch (DCFR_TERMINAL_*; GROUP: two or four
+ * warps per terminal, tiles of terminals in large trees), and for the panel kernel the terminals evaluated together per
  * panel (0 otherwise). */
 enum {
   DCFR_TERMINAL_PANEL = 0,

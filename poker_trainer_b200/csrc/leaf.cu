@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(PREPARE_WARPS * 32) leaf_prepare_kernel(LeafAr
 }
 
 // Block (leaf task, card index): one input row, as the network packs it (bf16,
-// zeros past the network.s inputs).
+// zeros past the network's inputs).
 __global__ void __launch_bounds__(256) leaf_inputs_kernel(LeafArgs A, const LeafTask* __restrict__ tasks,
                                                           const uint8_t* __restrict__ hc1_0,
                                                           const uint8_t* __restrict__ hc2_0,

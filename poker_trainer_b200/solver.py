@@ -480,8 +480,8 @@ class Solver:
 
     def terminal_kernel(self) -> tuple:
         """(kernel name, terminals per panel) of this handle's f32 terminal
-        evaluation: "panel", "warp", "block", "group" (two warps per
-        terminal) or "exact"."""
+        evaluation: "panel", "warp", "block", "group" (two or
+        four warps per terminal, tiles of terminals in large trees) or "exact"."""
         k = C.c_int32()
         t = C.c_int32()
         check(lib().dcfr_terminal_kernel(self._h, C.byref(k), C.byref(t)))
