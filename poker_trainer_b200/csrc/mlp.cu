@@ -643,6 +643,7 @@ int dcfr_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, int32_t out_
   MK(cudaMemset(n->loss, 0, 12));
   n->err = reinterpret_cast<int*>(n->loss + 2);
   MK(cudaMallocHost(&n->result, 12));
+  MK(cudaStreamSynchronize(cudaStreamLegacy));  // the copies and memsets above
   int rc = refresh_bf16(n.get());
   if (rc) return rc;
   MK(cudaStreamSynchronize(n->stream));
@@ -668,7 +669,9 @@ int dcfr_mlp_get_params(const dcfr_mlp* n, float* host) {
 
 int dcfr_mlp_set_params(dcfr_mlp* n, const float* host) {
   if (!n || !host) return fail(DCFR_ERR_INVALID_ARG, "NULL argument");
-  MK(cudaMemcpy(n->w, host, n->nparams * 4, cudaMemcpyHostToDevice));
+  // On the stream that reads them next: a copy from pageable memory may still
+  // be on its way to the device when cudaMemcpy returns.
+  MK(cudaMemcpyAsync(n->w, host, n->nparams * 4, cudaMemcpyHostToDevice, n->stream));
   int rc = refresh_bf16(n);
   if (rc) return rc;
   MK(cudaStreamSynchronize(n->stream));
