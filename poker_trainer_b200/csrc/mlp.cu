@@ -510,9 +510,9 @@ extern "C" {
 int dcfr_gemm_bf16(const void* a, const void* b, void* c, int32_t m, int32_t n, int32_t k, int32_t epi,
                    const float* bias, void* z, int32_t ldc, void* stream) {
   int* err = nullptr;
-  MK(cudaMalloc(&err, 4));
-  MK(cudaMemset(err, 0, 4));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  MK(cudaMalloc(&err, 4));
+  MK(cudaMemsetAsync(err, 0, 4, s));
   int rc = gemm_setup();
   if (!rc)
     rc = gemm(static_cast<const bf16*>(a), static_cast<const bf16*>(b), m, n, k, epi, c, ldc, static_cast<bf16*>(z),
@@ -535,10 +535,10 @@ int dcfr_gemm_bf16_timed(const void* a, const void* b, void* c, int32_t m, int32
   int* err = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   MK(cudaMalloc(&err, 4));
-  MK(cudaMemset(err, 0, 4));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  MK(cudaMemsetAsync(err, 0, 4, s));
   MK(cudaEventCreate(&e0));
   MK(cudaEventCreate(&e1));
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc = gemm_setup(), e = 0;
   MK(cudaEventRecord(e0, s));
   for (int r = 0; r < reps && !rc; r++)
