@@ -235,7 +235,9 @@ def ncu_traffic(kernel: str, workload: str):
 KERNEL_NAMES = {"terminal": "fast_terminal_kernel", "down": "down_kernel", "up": "up_kernel", "other": "other"}
 # The CUDA kernel behind each terminal kernel name of dcfr_terminal_kernel.
 TERMINAL_FN = {"panel": "panel_terminal_kernel", "warp": "warp_terminal_kernel", "block": "fast_terminal_kernel",
-               "group": "group_terminal_kernel", "exact": "terminal_kernel"}
+               "group": "group_terminal_kernel", "exact": "exact_terminal_kernel"}
+# "group" on a flop (384 terminals a multiprocessor and more): tiles of terminals.
+FLOP_TERMINAL_FN = dict(TERMINAL_FN, group="tile_terminal_kernel")
 
 
 def spawn_ranks(n: int) -> int:
@@ -581,7 +583,7 @@ def run_flop(args, world, rank, local):
     per_launch_ms = dc["ms"] / max(dc["launches"], 1)
     per_launch_bytes = dc["bytes"] / max(dc["launches"], 1)
     achieved = per_launch_bytes / (per_launch_ms / 1000.0) / 1e9 if per_launch_ms > 0 else 0.0
-    kfull = TERMINAL_FN[kname] if dom == "terminal" else KERNEL_NAMES[dom]
+    kfull = FLOP_TERMINAL_FN[kname] if dom == "terminal" else KERNEL_NAMES[dom]
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
