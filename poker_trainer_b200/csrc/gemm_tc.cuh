@@ -6,8 +6,8 @@
 // A and B are row-major with K contiguous (both operands "K-major"). One CTA
 // computes a 128 x BN tile of C:
 //   * warp 0, one thread: TMA loads of 128 x 64 tiles of A and BN x 64 tiles of
-//     B into a ring of STAGES in shared memory (128-byte swizzle, the canonical
-//     K-major layout the tensor core reads);
+//     B, DEPTH of each a step, into a ring of STAGES steps in shared memory
+//     (128-byte swizzle, the canonical K-major layout the tensor core reads);
 //   * warp 1, one thread: tcgen05.mma (M=128, N=BN, K=16 per instruction,
 //     FP32 accumulator in tensor memory), a tcgen05.commit per stage frees
 //     the stage, a last commit marks the accumulator complete;
@@ -24,6 +24,14 @@
 // 896 x 1024 x 1024 37.1 to 10.9, 256 x 1024 x 2816 41.3 to 17.4, 256 x 1024 x
 // 1024 33.0 to 9.4, 896 x 2688 x 1024 with bias 18.2 to 12.4; 8192 x 1024 x 2816
 // with GELU 105.7 to 60.0, plain 4096 x 1024 x 2816 28.4 to 27.6.
+// In one CTA alone on an SM a step of the ring costs about 0.14 us of barriers,
+// commit and polling, whatever the tile, and 0.14 us for each 64 of K: steps of
+// 128 or 192 there, and one warp that polls instead of eight. us a launch at
+// steps of 64 and now: 256 x 1024 x 2816 with GELU 17.4 to 12.2, 256 x 1024 x 1024
+// 9.6 to 7.2, 896 x 1024 x 2816 19.1 to 15.1, 896 x 1024 x 1024 10.9 to 9.9, 896 x
+// 2688 x 1024 15.6 to 14.7. Two CTAs on an SM hide each other's steps (256 x 2688 x
+// 1024: 10.1, one CTA with long steps 13.3; 4096 x 1024 x 2816: one polling warp
+// 28.4 against 27.9).
 // Every wait on an mbarrier is bounded; a wait that gives up records an error
 // code and the CTA skips the rest of its work, frees its tensor memory and
 // returns.
@@ -41,8 +49,8 @@ namespace dcfr {
 
 constexpr int GEMM_BM = 128, GEMM_BK = 64, GEMM_THREADS = 256;
 constexpr uint32_t GEMM_A_BYTES = GEMM_BM * GEMM_BK * 2;  // one 128 x 64 bf16 tile
-constexpr size_t gemm_smem(int bn, int stages) {
-  return 1024 + (size_t)stages * (GEMM_A_BYTES + (size_t)bn * GEMM_BK * 2) + 256;
+constexpr size_t gemm_smem(int bn, int stages, int depth) {
+  return 1024 + (size_t)stages * depth * (GEMM_A_BYTES + (size_t)bn * GEMM_BK * 2) + 256;
 }
 constexpr long long GEMM_WAIT_LIMIT = 1ll << 22;  // polls before a wait gives up (well over a second)
 
@@ -144,7 +152,7 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.3989422804014327f * expf(-0.5f * x * x);
 }
 
-template <int BN, int STAGES, int CTAS>
+template <int BN, int STAGES, int CTAS, int DEPTH>
 __global__ void __launch_bounds__(GEMM_THREADS, CTAS)
     gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                         GemmArgs G) {
@@ -152,8 +160,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, CTAS)
   constexpr uint32_t B_BYTES = BN * GEMM_BK * 2;
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)gemm_smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sa = smem;
-  unsigned char* sb = smem + STAGES * GEMM_A_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sb + STAGES * B_BYTES);
+  unsigned char* sb = smem + STAGES * DEPTH * GEMM_A_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sb + STAGES * DEPTH * B_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* accf = empty + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accf + 1);
@@ -161,7 +169,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, CTAS)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * GEMM_BM, n0 = blockIdx.x * BN;
-  const int nk = G.K / GEMM_BK;
+  const int nb = G.K / GEMM_BK, nk = (nb + DEPTH - 1) / DEPTH;  // 64-wide blocks of K, steps
 
   if (tid == 0) {
     failed = 0;
@@ -193,9 +201,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, CTAS)
         failed = 1;
         break;
       }
-      mbar_expect_tx(&full[s], GEMM_A_BYTES + B_BYTES);
-      tma_load_2d(sa + s * GEMM_A_BYTES, &map_a, &full[s], kb * GEMM_BK, m0);
-      tma_load_2d(sb + s * B_BYTES, &map_b, &full[s], kb * GEMM_BK, n0);
+      const int d1 = min(DEPTH, nb - kb * DEPTH);
+      mbar_expect_tx(&full[s], d1 * (GEMM_A_BYTES + B_BYTES));
+#pragma unroll
+      for (int d = 0; d < DEPTH; d++) {
+        if (d >= d1) break;
+        const int at = s * DEPTH + d, x = (kb * DEPTH + d) * GEMM_BK;
+        tma_load_2d(sa + at * GEMM_A_BYTES, &map_a, &full[s], x, m0);
+        tma_load_2d(sb + at * B_BYTES, &map_b, &full[s], x, n0);
+      }
     }
   } else if (warp == 1 && lane == 0) {
     // Tensor-core issue.
@@ -207,22 +221,36 @@ __global__ void __launch_bounds__(GEMM_THREADS, CTAS)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t da = sw128_desc(sa + s * GEMM_A_BYTES), db = sw128_desc(sb + s * B_BYTES);
+      const int d1 = min(DEPTH, nb - kb * DEPTH);
 #pragma unroll
-      for (int k = 0; k < GEMM_BK / 16; k++)  // K = 16 per instruction: 32 bytes along the swizzled row
-        umma_bf16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+      for (int d = 0; d < DEPTH; d++) {
+        if (d >= d1) break;
+        const int at = s * DEPTH + d;
+        const uint64_t da = sw128_desc(sa + at * GEMM_A_BYTES), db = sw128_desc(sb + at * B_BYTES);
+#pragma unroll
+        for (int k = 0; k < GEMM_BK / 16; k++)  // K = 16 per instruction: 32 bytes along the swizzled row
+          umma_bf16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || d > 0 || k > 0) ? 1u : 0u);
+      }
       umma_commit(&empty[s]);
     }
     umma_commit(accf);
   }
   __syncwarp();
   // Epilogue: every thread owns half a row of the tile.
-  const bool ok = mbar_wait(accf, 0);
-  if (!ok && lane == 0) atomicExch(&failed, 3);
-  __syncwarp();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // tcgen05.ld is warp-collective: decide once per warp.
-  const bool go = __all_sync(0xffffffffu, ok && *(volatile int*)&failed == 0);
+  bool go;  // the same for a warp at least: tcgen05.ld is warp-collective
+  if constexpr (CTAS == 1) {
+    // One warp polls, the others wait at the barrier.
+    if (warp == 0 && !mbar_wait(accf, 0) && lane == 0) atomicExch(&failed, 3);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    go = *(volatile int*)&failed == 0;
+  } else {
+    const bool ok = mbar_wait(accf, 0);
+    if (!ok && lane == 0) atomicExch(&failed, 3);
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    go = __all_sync(0xffffffffu, ok && *(volatile int*)&failed == 0);
+  }
   if (go) {
     constexpr int HALF = BN / 2, STEP = HALF < 32 ? HALF : 32;
     const int quarter = warp & 3;

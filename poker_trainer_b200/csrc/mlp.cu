@@ -91,28 +91,29 @@ struct GemmShape {
   int bn;
   size_t smem;
 };
-template <int BN, int STAGES, int CTAS>
+template <int BN, int STAGES, int CTAS, int DEPTH = 1>
 GemmShape gemm_variant() {
-  return GemmShape{(GemmKernel)gemm_bf16_tc_kernel<BN, STAGES, CTAS>, BN, gemm_smem(BN, STAGES)};
+  return GemmShape{(GemmKernel)gemm_bf16_tc_kernel<BN, STAGES, CTAS, DEPTH>, BN, gemm_smem(BN, STAGES, DEPTH)};
 }
 
 // The tile of an [M][N] output. 128 x 128 where that gives three fifths of the
 // SMs a CTA: two to an SM with 3-stage rings once there are more CTAs than
-// SMs (one's epilogue runs under the other's MMAs), else one with 6 stages.
-// Narrower tiles below (M = 896: 64 wide, M = 256: 32 wide; a 9-stage ring
-// there gains 3%).
+// SMs (one's epilogue runs under the other's MMAs), else one with long steps.
+// Narrower tiles below (M = 896: 64 wide, M = 256: 32 wide), two to an SM only
+// where there are more CTAs than SMs.
 GemmShape gemm_shape(int M, int N) {
   const int rows = M / GEMM_BM;
   if (rows * (N / 128) > 148) return gemm_variant<128, 3, 2>();
-  if (rows * (N / 128) >= 90) return gemm_variant<128, 6, 1>();
-  if (rows * (N / 64) >= 90) return gemm_variant<64, 8, 1>();
-  return gemm_variant<32, 5, 2>();
+  if (rows * (N / 128) >= 90) return gemm_variant<128, 3, 1, 2>();
+  if (rows * (N / 64) >= 90) return gemm_variant<64, 3, 1, 3>();
+  if (rows * (N / 32) > 148) return gemm_variant<32, 5, 2>();
+  return gemm_variant<32, 3, 1, 3>();
 }
 
 // Before a context's first gemm().
 int gemm_setup() {
-  for (const GemmShape& v : {gemm_variant<128, 3, 2>(), gemm_variant<128, 6, 1>(), gemm_variant<64, 8, 1>(),
-                             gemm_variant<32, 5, 2>()})
+  for (const GemmShape& v : {gemm_variant<128, 3, 2>(), gemm_variant<128, 3, 1, 2>(), gemm_variant<64, 3, 1, 3>(),
+                             gemm_variant<32, 5, 2>(), gemm_variant<32, 3, 1, 3>()})
     MK(cudaFuncSetAttribute((const void*)v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
   return DCFR_OK;
 }

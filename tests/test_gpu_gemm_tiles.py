@@ -38,6 +38,15 @@ def test_tiles(gpu, m, n, k, epi):
         assert float((z.double() - pre).abs().max()) <= 1e-2 * float(pre.abs().max())
 
 
+# Steps of 64, 128 and 192 of K: a last step that is partly empty, and rings that
+# go round; 256 x 2688: tiles 32 wide, two to an SM.
+@pytest.mark.parametrize("m,n", SHAPES + [(256, 2688)])
+@pytest.mark.parametrize("k", [256, 1344])
+@pytest.mark.parametrize("epi", [0, 2])
+def test_steps(gpu, m, n, k, epi):
+    test_tiles(gpu, m, n, k, epi)
+
+
 @pytest.mark.parametrize("rows", [1, 129, 300])
 @pytest.mark.parametrize("masked", [False, True])
 def test_gradients_with_padded_rows(gpu, rows, masked):
