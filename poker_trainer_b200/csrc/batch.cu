@@ -417,11 +417,12 @@ void bfree(T*& p) {
 }
 
 template <class T>
-Status upload(cudaStream_t stream, T*& d, const std::vector<T>& h, const char* what) {
+Status upload(T*& d, const std::vector<T>& h, const char* what) {
   Status s = balloc(d, h.size(), what);
   if (!s.ok()) return s;
-  // On the stream that reads it (see Engine::upload_plan).
-  if (!h.empty()) BK(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
+  if (h.empty()) return Status();
+  BK(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  BK(cudaStreamSynchronize(cudaStreamLegacy));  // see copies_done (engine.cu)
   return Status();
 }
 
@@ -556,7 +557,7 @@ Status Batch::Impl::ensure_discounts(uint32_t max_t) {
     graph = nullptr;
   }
   bfree(disc);
-  Status s = upload(stream, disc, tab, "discounts");
+  Status s = upload(disc, tab, "discounts");
   disc_len = len;
   return s;
 }
@@ -771,31 +772,31 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   if (!(s = balloc(alive, 2 * total_slots, "batch liveness flags")).ok()) return s;
   BK(cudaMemsetAsync(vals, 0, std::max<uint64_t>(nodes * stride, 1) * 4, stream));
   BK(cudaMemsetAsync(reach, 0, std::max<uint64_t>(total_slots * stride, 1) * 4, stream));
-  if (!(s = upload(stream, hc1, h1, "batch hands")).ok()) return s;
-  if (!(s = upload(stream, hc2, h2, "batch hands")).ok()) return s;
-  if (!(s = upload(stream, same, hs, "batch hands")).ok()) return s;
-  if (!(s = upload(stream, dims, hdims, "batch hands")).ok()) return s;
-  if (!(s = upload(stream, roots, hroot, "batch root rows")).ok()) return s;
+  if (!(s = upload(hc1, h1, "batch hands")).ok()) return s;
+  if (!(s = upload(hc2, h2, "batch hands")).ok()) return s;
+  if (!(s = upload(same, hs, "batch hands")).ok()) return s;
+  if (!(s = upload(dims, hdims, "batch hands")).ok()) return s;
+  if (!(s = upload(roots, hroot, "batch root rows")).ok()) return s;
   if (!(s = balloc(root_out, hroot.size(), "batch root rows")).ok()) return s;
-  if (!(s = upload(stream, boards, hb, "batch boards")).ok()) return s;
+  if (!(s = upload(boards, hb, "batch boards")).ok()) return s;
   for (int p = 0; p < 2; p++) {
     ntasks[p] = hterm[p].size();
     nunits[p] = hunits[p].size();
     ndown[p] = hdown[p].size();
-    if (!(s = upload(stream, down[p], hdown[p], "batch plan")).ok()) return s;
-    if (!(s = upload(stream, up[p], hup[p], "batch plan")).ok()) return s;
-    if (!(s = upload(stream, levs[p], hlevs[p], "batch plan")).ok()) return s;
-    if (!(s = upload(stream, term[p], hterm[p], "batch plan")).ok()) return s;
-    if (!(s = upload(stream, units[p], hunits[p], "batch plan")).ok()) return s;
+    if (!(s = upload(down[p], hdown[p], "batch plan")).ok()) return s;
+    if (!(s = upload(up[p], hup[p], "batch plan")).ok()) return s;
+    if (!(s = upload(levs[p], hlevs[p], "batch plan")).ok()) return s;
+    if (!(s = upload(term[p], hterm[p], "batch plan")).ok()) return s;
+    if (!(s = upload(units[p], hunits[p], "batch plan")).ok()) return s;
     if (!(s = balloc(deferred[p], hdown[p].size() * slices, "batch plan")).ok()) return s;
   }
-  if (!(s = upload(stream, d_spots, spots, "batch plan")).ok()) return s;
+  if (!(s = upload(d_spots, spots, "batch plan")).ok()) return s;
   std::vector<uint32_t> nat(count), lpt(count);
   std::iota(nat.begin(), nat.end(), 0u);
   lpt = nat;
   std::stable_sort(lpt.begin(), lpt.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
-  if (!(s = upload(stream, order_nat, nat, "batch order")).ok()) return s;
-  if (!(s = upload(stream, order_lpt, lpt, "batch order")).ok()) return s;
+  if (!(s = upload(order_nat, nat, "batch order")).ok()) return s;
+  if (!(s = upload(order_lpt, lpt, "batch order")).ok()) return s;
   // Strength tables and scan layouts, per spot (its board and fold layouts).
   if (!(s = balloc(tables, (size_t)count * 2 * tstride, "batch strength tables")).ok()) return s;
   if (!(s = balloc(tcount, (size_t)count * 2, "batch strength tables")).ok()) return s;
@@ -1218,7 +1219,7 @@ Status Batch::download(int spot, float* regrets, float* sums) {
     I.block_first.push_back((uint32_t)blk.size());
     if (!(s = balloc(I.staging, 2 * most, "batch transfer buffer")).ok()) return s;
     BK(cudaMallocHost((void**)&I.pinned, 2 * most * sizeof(float)));
-    if (!(s = upload(I.stream, I.blocks, blk, "batch transfer table")).ok()) return s;
+    if (!(s = upload(I.blocks, blk, "batch transfer table")).ok()) return s;
   }
   const uint32_t f = I.block_first[spot];
   const int nb = (int)(I.block_first[spot + 1] - f);

@@ -49,6 +49,16 @@ static void dfree(T*& p) {
 // Terminals per SM from which the tile kernel evaluates them.
 constexpr int TILE_TERMINALS_PER_SM = 384;
 
+// To be called between cudaMemcpy from host arrays and work on a handle's stream
+// that reads them: the copy from pageable memory may still be on its way when
+// cudaMemcpy returns, and a non-blocking stream does not wait for it. (Copies
+// queued on the handle's stream wait for its memsets: creating a turn solver
+// took 2.5 ms longer.)
+static Status copies_done() {
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  return Status();
+}
+
 static inline int pad8(int n) { return (n + 7) & ~7; }
 
 Plan::~Plan() {
@@ -280,9 +290,9 @@ Status Engine::init() {
     if (!(s = dalloc(hc1_[q], hp_[q], "hands")).ok()) return s;
     if (!(s = dalloc(hc2_[q], hp_[q], "hands")).ok()) return s;
     if (!(s = dalloc(same_[q], hp_[q], "hands")).ok()) return s;
-    CK(cudaMemcpyAsync(hc1_[q], a.data(), hp_[q], cudaMemcpyHostToDevice, stream_));
-    CK(cudaMemcpyAsync(hc2_[q], b.data(), hp_[q], cudaMemcpyHostToDevice, stream_));
-    CK(cudaMemcpyAsync(same_[q], sm.data(), hp_[q] * 4, cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(hc1_[q], a.data(), hp_[q], cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(hc2_[q], b.data(), hp_[q], cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(same_[q], sm.data(), hp_[q] * 4, cudaMemcpyHostToDevice));
   }
   {
     std::vector<uint16_t> perm((size_t)12 * stride_, 0);
@@ -290,7 +300,7 @@ Status Engine::init() {
       for (int pr = 0; pr < 6; pr++)
         for (size_t h = 0; h < g.perm[q][pr].size(); h++) perm[(size_t)(q * 6 + pr) * stride_ + h] = g.perm[q][pr][h];
     if (!(s = dalloc(perm_, perm.size(), "perm")).ok()) return s;
-    CK(cudaMemcpyAsync(perm_, perm.data(), perm.size() * 2, cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(perm_, perm.data(), perm.size() * 2, cudaMemcpyHostToDevice));
   }
   // Chance cards and isomorphic references.
   {
@@ -308,10 +318,9 @@ Status Engine::init() {
       for (size_t r = 0; r < ci.ci.size(); r++) iso.push_back(IsoRefD{ci.ci[r], ci.pair[r], 0});
     }
     if (!(s = dalloc(chance_cards_, cc.size(), "chance cards")).ok()) return s;
-    if (!cc.empty()) CK(cudaMemcpyAsync(chance_cards_, cc.data(), cc.size(), cudaMemcpyHostToDevice, stream_));
+    if (!cc.empty()) CK(cudaMemcpy(chance_cards_, cc.data(), cc.size(), cudaMemcpyHostToDevice));
     if (!(s = dalloc(iso_, iso.size(), "iso refs")).ok()) return s;
-    if (!iso.empty()) CK(cudaMemcpyAsync(iso_, iso.data(), iso.size() * sizeof(IsoRefD),
-                                         cudaMemcpyHostToDevice, stream_));
+    if (!iso.empty()) CK(cudaMemcpy(iso_, iso.data(), iso.size() * sizeof(IsoRefD), cudaMemcpyHostToDevice));
   }
   phase(setup.device_ms);
   // Strength tables, built on the device.
@@ -325,7 +334,8 @@ Status Engine::init() {
         for (int k = 0; k < 5; k++) bc[(size_t)b * 5 + k] = (uint8_t)g.boards[b][k];
       uint8_t* d_boards = nullptr;
       if (!(s = dalloc(d_boards, bc.size(), "boards")).ok()) return s;
-      CK(cudaMemcpyAsync(d_boards, bc.data(), bc.size(), cudaMemcpyHostToDevice, stream_));
+      CK(cudaMemcpy(d_boards, bc.data(), bc.size(), cudaMemcpyHostToDevice));
+      if (!(s = copies_done()).ok()) return s;
       launch_strength(d_boards, nb, hc1_[0], hc2_[0], hc1_[1], hc2_[1], g.n[0], g.n[1], tables_, table_count_,
                       tstride_, stream_);
       CK(cudaGetLastError());
@@ -364,7 +374,7 @@ Status Engine::init() {
     for (int p = 0; p < 2; p++)
       for (int i = 0; i < g.n[p ^ 1]; i++) rr[(size_t)p * stride_ + i] = g.weights[p ^ 1][i];
     if (!(s = dalloc(root_rows_, rr.size(), "root rows")).ok()) return s;
-    CK(cudaMemcpyAsync(root_rows_, rr.data(), rr.size() * 4, cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(root_rows_, rr.data(), rr.size() * 4, cudaMemcpyHostToDevice));
     if (!(s = dalloc(root_out_, rr.size(), "root rows")).ok()) return s;
   }
   phase(setup.rows_ms);
@@ -1064,9 +1074,6 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   return Status();
 }
 
-// Host arrays go up on the stream whose kernels read them (everywhere in this
-// file): cudaMemcpy may return before its copy from pageable memory has reached
-// the device, and a non-blocking stream does not wait for it.
 Status Engine::upload_plan(Plan& plan) {
   Status s;
   if (!(s = dalloc(plan.d_down, plan.h_down.size(), "plan")).ok()) return s;
@@ -1075,43 +1082,36 @@ Status Engine::upload_plan(Plan& plan) {
   if (!(s = dalloc(plan.d_units, plan.h_units.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_jobs, plan.h_jobs.size(), "plan")).ok()) return s;
   if (!plan.h_jobs.empty())
-    CK(cudaMemcpyAsync(plan.d_jobs, plan.h_jobs.data(), plan.h_jobs.size() * sizeof(TermUnit),
-                       cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_jobs, plan.h_jobs.data(), plan.h_jobs.size() * sizeof(TermUnit), cudaMemcpyHostToDevice));
   if (!(s = dalloc(plan.d_leaves, plan.h_leaves.size(), "plan")).ok()) return s;
   if (!plan.h_leaves.empty())
-    CK(cudaMemcpyAsync(plan.d_leaves, plan.h_leaves.data(), plan.h_leaves.size() * sizeof(LeafTask),
-                  cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_leaves, plan.h_leaves.data(), plan.h_leaves.size() * sizeof(LeafTask),
+                  cudaMemcpyHostToDevice));
   if (!plan.h_units.empty())
-    CK(cudaMemcpyAsync(plan.d_units, plan.h_units.data(), plan.h_units.size() * sizeof(TermUnit),
-                       cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_units, plan.h_units.data(), plan.h_units.size() * sizeof(TermUnit), cudaMemcpyHostToDevice));
   if (!(s = dalloc(plan.d_panels, plan.h_panels.size(), "plan")).ok()) return s;
   if (!plan.h_panels.empty())
-    CK(cudaMemcpyAsync(plan.d_panels, plan.h_panels.data(), plan.h_panels.size() * sizeof(PanelD),
-                  cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_panels, plan.h_panels.data(), plan.h_panels.size() * sizeof(PanelD),
+                  cudaMemcpyHostToDevice));
   if (plan.seg && !(s = upload_segment(plan)).ok()) return s;
   if (!(s = dalloc(plan.d_trees, plan.h_trees.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fdown, plan.h_fdown.size(), "plan")).ok()) return s;
   if (!(s = dalloc(plan.d_fup, plan.h_fup.size(), "plan")).ok()) return s;
   if (!plan.h_trees.empty()) {
-    CK(cudaMemcpyAsync(plan.d_trees, plan.h_trees.data(), plan.h_trees.size() * sizeof(FusedTree),
-                       cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_trees, plan.h_trees.data(), plan.h_trees.size() * sizeof(FusedTree), cudaMemcpyHostToDevice));
     if (!plan.h_fdown.empty())
-      CK(cudaMemcpyAsync(plan.d_fdown, plan.h_fdown.data(), plan.h_fdown.size() * sizeof(DownTask),
-                    cudaMemcpyHostToDevice, stream_));
+      CK(cudaMemcpy(plan.d_fdown, plan.h_fdown.data(), plan.h_fdown.size() * sizeof(DownTask),
+                    cudaMemcpyHostToDevice));
     if (!plan.h_fup.empty())
-      CK(cudaMemcpyAsync(plan.d_fup, plan.h_fup.data(), plan.h_fup.size() * sizeof(UpTask),
-                         cudaMemcpyHostToDevice, stream_));
+      CK(cudaMemcpy(plan.d_fup, plan.h_fup.data(), plan.h_fup.size() * sizeof(UpTask), cudaMemcpyHostToDevice));
   }
   if (!plan.h_fast.empty())
-    CK(cudaMemcpyAsync(plan.d_fast, plan.h_fast.data(), plan.h_fast.size() * sizeof(FastTask),
-                       cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_fast, plan.h_fast.data(), plan.h_fast.size() * sizeof(FastTask), cudaMemcpyHostToDevice));
   if (!plan.h_down.empty())
-    CK(cudaMemcpyAsync(plan.d_down, plan.h_down.data(), plan.h_down.size() * sizeof(DownTask),
-                       cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(plan.d_down, plan.h_down.data(), plan.h_down.size() * sizeof(DownTask), cudaMemcpyHostToDevice));
   if (!plan.h_up.empty())
-    CK(cudaMemcpyAsync(plan.d_up, plan.h_up.data(), plan.h_up.size() * sizeof(UpTask),
-                       cudaMemcpyHostToDevice, stream_));
-  return Status();
+    CK(cudaMemcpy(plan.d_up, plan.h_up.data(), plan.h_up.size() * sizeof(UpTask), cudaMemcpyHostToDevice));
+  return copies_done();
 }
 
 // The root segment in its own numbering (SegRes): value row 0 is the root's,
@@ -1197,7 +1197,7 @@ Status Engine::upload_segment(Plan& plan) {
   uint32_t o_own[2];
   for (int q = 0; q < 2; q++) o_own[q] = put(own[q].data(), own[q].size() * 8);
   CK(cudaMalloc(&plan.d_res, h.size()));
-  CK(cudaMemcpyAsync(plan.d_res, h.data(), h.size(), cudaMemcpyHostToDevice, stream_));
+  CK(cudaMemcpy(plan.d_res, h.data(), h.size(), cudaMemcpyHostToDevice));
   R.blob = static_cast<const unsigned char*>(plan.d_res);
   for (int q = 0; q < 2; q++) R.own[q] = reinterpret_cast<const uint64_t*>(R.blob + o_own[q]);
   const size_t slices = (size_t)((stride_ + SEG_SLICE - 1) / SEG_SLICE);
@@ -1506,12 +1506,13 @@ Status Engine::init_leaves() {
     std::vector<uint16_t> cb(hp_[q], 0);
     for (int i = 0; i < g.n[q]; i++) cb[i] = g.combos[q][i];
     if (!(s = dalloc(combos_[q], cb.size(), "leaf combos")).ok()) return s;
-    CK(cudaMemcpyAsync(combos_[q], cb.data(), cb.size() * 2, cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(combos_[q], cb.data(), cb.size() * 2, cudaMemcpyHostToDevice));
   }
   if (!(s = dalloc(leaf_mass_, (size_t)std::max(L, 1) * 2, "leaf masses")).ok()) return s;
   if (!(s = dalloc(leaf_shift_, (size_t)std::max(L, 1) * leaf_nc_, "leaf masses")).ok()) return s;
   if (!(s = dalloc(leaf_cards_, cards.size(), "leaf cards")).ok()) return s;
-  CK(cudaMemcpyAsync(leaf_cards_, cards.data(), cards.size(), cudaMemcpyHostToDevice, stream_));
+  CK(cudaMemcpy(leaf_cards_, cards.data(), cards.size(), cudaMemcpyHostToDevice));
+  if (!(s = copies_done()).ok()) return s;
   for (int p = 0; p < 2; p++)
     enqueue_traversal(*full_[p], M_AVG, root_rows_ + (size_t)p * stride_, nullptr);
   CK(cudaGetLastError());
@@ -1606,9 +1607,9 @@ Status Engine::ensure_discounts(uint32_t max_t) {
   dfree(disc_table_);
   Status s;
   if (!(s = dalloc(disc_table_, len, "discounts")).ok()) return s;
-  CK(cudaMemcpyAsync(disc_table_, tab.data(), len * sizeof(DiscountD), cudaMemcpyHostToDevice, stream_));
+  CK(cudaMemcpy(disc_table_, tab.data(), len * sizeof(DiscountD), cudaMemcpyHostToDevice));
   disc_len_ = len;
-  return Status();
+  return copies_done();
 }
 
 // n DCFR iterations: t += 1, then player 0's and player 1's traversals with
@@ -1817,7 +1818,8 @@ Status Engine::fp64_root_values(int mode, double out[2]) {
     std::vector<double> rr((size_t)2 * stride_, 0.0);
     for (int p = 0; p < 2; p++)
       for (int i = 0; i < g.n[p ^ 1]; i++) rr[(size_t)p * stride_ + i] = (double)g.weights[p ^ 1][i];
-    CK(cudaMemcpyAsync(root_rows64_, rr.data(), rr.size() * 8, cudaMemcpyHostToDevice, stream_));
+    CK(cudaMemcpy(root_rows64_, rr.data(), rr.size() * 8, cudaMemcpyHostToDevice));
+    if (!(s = copies_done()).ok()) return s;
     CK(cudaMemsetAsync(reach64_, 0, (size_t)max_slots_ * stride_ * 8, stream_));
     CK(cudaMemsetAsync(vals64_, 0, N * (size_t)stride_ * 8, stream_));
   }
@@ -2072,10 +2074,10 @@ Status Engine::storage_chunks() {
   if (c.count > 0) chunks.push_back(c);
   Status s;
   if (!(s = dalloc(sblk_, blk.size(), "storage transfer table")).ok()) return s;
-  CK(cudaMemcpyAsync(sblk_, blk.data(), blk.size() * sizeof(StorageBlockD), cudaMemcpyHostToDevice, stream_));
+  CK(cudaMemcpy(sblk_, blk.data(), blk.size() * sizeof(StorageBlockD), cudaMemcpyHostToDevice));
   stage_len_ = stage;
   schunks_ = std::move(chunks);
-  return Status();
+  return copies_done();
 }
 
 namespace {
