@@ -342,6 +342,7 @@ Status Engine::init() {
       CK(cudaStreamSynchronize(stream_));
       cudaFree(d_boards);
     }
+    if (nb == 0 && !(s = copies_done()).ok()) return s;
     if (!(s = ensure_fast_layouts()).ok()) return s;
   }
   phase(setup.tables_ms);
