@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -426,6 +427,55 @@ Status upload(T*& d, const std::vector<T>& h, const char* what) {
   return Status();
 }
 
+// A page-locked block of host memory that kernels can write, for the time of a
+// transfer. Page-locking takes 1 to 5 ms whatever the size, so up to
+// POOL_MOST blocks that are not in use are kept for the process's later
+// transfers, of any batch, thread or device.
+struct PinnedBlock {
+  static constexpr size_t BYTES = 2 << 20, POOL_MOST = 4;
+  void* p = nullptr;
+  PinnedBlock() {
+    {
+      std::lock_guard<std::mutex> hold(pool().lock);
+      if (!pool().free.empty()) {
+        p = pool().free.back();
+        pool().free.pop_back();
+      }
+    }
+    if (!p && cudaHostAlloc(&p, BYTES, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~PinnedBlock() {
+    if (!p) return;
+    {
+      std::lock_guard<std::mutex> hold(pool().lock);
+      if (pool().free.size() < POOL_MOST) {
+        pool().free.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+  PinnedBlock(const PinnedBlock&) = delete;
+  PinnedBlock& operator=(const PinnedBlock&) = delete;
+
+ private:
+  struct Pool {
+    std::mutex lock;
+    std::vector<void*> free;
+    Pool() { free.reserve(POOL_MOST); }
+  };
+  // Never destroyed: a batch may be closed while the process exits.
+  static Pool& pool() {
+    static Pool* const the = new Pool();
+    return *the;
+  }
+};
+// A node has at most 16 actions of 1326 hands.
+static_assert(sizeof(StorageBlockD) + 2 * 16 * DCFR_NUM_COMBOS * sizeof(float) <= PinnedBlock::BYTES, "a node fits");
+
 // Slices (spot x 32 hands) up to which a block's warps share one; terminals
 // per SM, and groups per block, up to which each terminal takes a block.
 constexpr int BATCH_SHARE_ITEMS = 148 * 24;
@@ -470,11 +520,6 @@ struct Batch::Impl {
   DiscountD* cur_disc = nullptr;
   uint32_t disc_len = 0;
   uint32_t* counter = nullptr;
-  // Transfers (built on the first): every spot's storage blocks, and room
-  // for the largest spot's regrets and sums on both sides.
-  StorageBlockD* blocks = nullptr;
-  std::vector<uint32_t> block_first;
-  float *staging = nullptr, *pinned = nullptr;
   uint32_t iterations = 0;
   dcfr_batch_tuning tuning{};
   cudaGraphExec_t graph = nullptr;
@@ -530,9 +575,6 @@ Batch::Impl::~Impl() {
     bfree(units[p]);
   }
   bfree(cur_disc);
-  bfree(blocks);
-  bfree(staging);
-  if (pinned) cudaFreeHost(pinned);
   bfree(d_spots);
   bfree(order_lpt);
   bfree(order_nat);
@@ -1192,45 +1234,44 @@ Status Batch::storage_len(int spot, uint64_t& len) const {
   return Status();
 }
 
-// One spot's storage: packed on the device into the reference's layout, both
-// kinds in one copy to a page-locked buffer, then into the caller's arrays
-// (before, two pageable copies of the padded blocks and a copy per row on the
-// host: 0.42 ms a spot of 80,000 cells, now 0.30, most of it the caller's
-// fresh pages).
+// One spot's storage, in the reference's layout: its decision nodes' records go
+// into a page-locked block, the pack kernel reads them there and writes the
+// nodes' cells beside them, and the host copies those to the caller's arrays;
+// a large spot takes several rounds of whole nodes. Nothing of this belongs to
+// the batch, so several threads may read spots of one batch, and the first
+// read costs what a later one does. ms, a batch's first and later reads of a
+// spot of 86,000 cells: with a table of all spots and buffers of the batch's own,
+// made on the first read, 2.2 to 3.9 (512 spots: 3.8 to 86) and 0.11; now 0.12
+// and 0.11.
 Status Batch::download(int spot, float* regrets, float* sums) {
   Impl& I = *impl_;
   if (spot < 0 || spot >= count()) return Status{DCFR_ERR_INVALID_ARG, "spot index out of range"};
   const Game& g = I.games[spot];
-  Status s;
-  if (!I.blocks) {
-    std::vector<StorageBlockD> blk;
-    uint64_t most = 1;
-    for (size_t i = 0; i < I.games.size(); i++) {
-      const Game& gi = I.games[i];
-      I.block_first.push_back((uint32_t)blk.size());
-      for (uint32_t v = 0; v < gi.nodes.size(); v++) {
-        const GNode& nd = gi.nodes[v];
-        if (nd.kind == N_PLAYER)
-          blk.push_back(StorageBlockD{I.store[i] + I.node_off[i][v], nd.ref_offset, nd.nchild, (uint32_t)gi.n[nd.player],
-                                      (uint32_t)I.spots[i].hp[nd.player], 0});
-      }
-      most = std::max<uint64_t>(most, gi.storage_len);
+  const std::vector<uint32_t> players = players_in_storage_order(g);
+  const PinnedBlock lease;
+  if (!lease.p) return Status{DCFR_ERR_OUT_OF_MEMORY, "page-locked transfer block"};
+  for (size_t i = 0; i < players.size();) {
+    // The nodes that fit: a record and both kinds of cells of each.
+    StorageBlockD* rec = static_cast<StorageBlockD*>(lease.p);
+    const uint64_t from = g.nodes[players[i]].ref_offset;
+    uint64_t len = 0;
+    int nb = 0;
+    for (; i < players.size(); i++, nb++) {
+      const GNode& nd = g.nodes[players[i]];
+      const uint64_t cells = (uint64_t)nd.nchild * (uint64_t)g.n[nd.player];
+      if (nb > 0 && (nb + 1) * sizeof(StorageBlockD) + 2 * (len + cells) * sizeof(float) > PinnedBlock::BYTES) break;
+      rec[nb] = StorageBlockD{I.store[spot] + I.node_off[spot][players[i]], nd.ref_offset - from, nd.nchild,
+                              (uint32_t)g.n[nd.player], (uint32_t)I.spots[spot].hp[nd.player], 0};
+      len += cells;
     }
-    I.block_first.push_back((uint32_t)blk.size());
-    if (!(s = balloc(I.staging, 2 * most, "batch transfer buffer")).ok()) return s;
-    BK(cudaMallocHost((void**)&I.pinned, 2 * most * sizeof(float)));
-    if (!(s = upload(I.blocks, blk, "batch transfer table")).ok()) return s;
+    float* out[2] = {reinterpret_cast<float*>(rec + nb), reinterpret_cast<float*>(rec + nb) + len};
+    if (regrets) launch_storage_pack(4, I.regrets, out[0], rec, nb, I.stream);
+    if (sums) launch_storage_pack(4, I.sums, out[1], rec, nb, I.stream);
+    BK(cudaGetLastError());
+    BK(cudaStreamSynchronize(I.stream));
+    if (regrets) std::memcpy(regrets + from, out[0], len * sizeof(float));
+    if (sums) std::memcpy(sums + from, out[1], len * sizeof(float));
   }
-  const uint32_t f = I.block_first[spot];
-  const int nb = (int)(I.block_first[spot + 1] - f);
-  const size_t len = (size_t)g.storage_len;
-  launch_storage_pack(4, I.regrets, I.staging, I.blocks + f, nb, I.stream);
-  launch_storage_pack(4, I.sums, I.staging + len, I.blocks + f, nb, I.stream);
-  BK(cudaGetLastError());
-  BK(cudaMemcpyAsync(I.pinned, I.staging, 2 * len * sizeof(float), cudaMemcpyDeviceToHost, I.stream));
-  BK(cudaStreamSynchronize(I.stream));
-  if (regrets) std::memcpy(regrets, I.pinned, len * sizeof(float));
-  if (sums) std::memcpy(sums, I.pinned + len, len * sizeof(float));
   return Status();
 }
 
