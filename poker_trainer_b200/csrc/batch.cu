@@ -5,8 +5,9 @@
 // and bet menu) built by the same host code as a single solve (game.cpp), so
 // its tree, storage order and arithmetic are those of the reference solver
 // (crates/solver/src/tree.rs, cfr.rs, river.rs, eval.rs). The spots share one
-// numbering of reach slots, value rows and terminal tasks (rows of one stride,
-// entries past a spot's own hands zero), and an iteration is four launches
+// numbering of reach slots, value rows and terminal tasks (rows of one stride;
+// a traversal writes its opponent's hands, and past them a reach row may hold
+// the other traversal's), and an iteration is four launches
 // over all of them: for each traversal a row pass and the terminals, the up
 // pass of a traversal being one launch with the down pass of the next.
 //   * Row passes (batch_row_kernel): everything is per hand, so a slice of 32
@@ -706,6 +707,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
     uint64_t work_units = 0;
     for (int p = 0; p < 2; p++) {
       const int o = p ^ 1;
+      const uint32_t entries = (uint32_t)S.hp[o];
       std::vector<uint32_t> slot(N, 0), depth(N, 0);
       std::vector<std::vector<SegUp>> ups;
       std::vector<std::vector<SegDown>> downs;
@@ -747,11 +749,11 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
             if (paired) continue;
             const int f = nd.player;
             const double val = f == p ? -(hpot + (double)nd.invest[p]) : hpot + (double)nd.invest[f] - (double)nd.rake;
-            folds.push_back(FastTask{T_FOLD_BATCH, layout, S.slot + sv, S.node + v, NONE32, {0, 0, 0}, val * norm, 0.0,
-                                     0.0, 0.0});
+            folds.push_back(FastTask{T_FOLD_BATCH, layout, S.slot + sv, S.node + v, NONE32, entries, {0, 0}, val * norm,
+                                     0.0, 0.0, 0.0});
           } else {
             const double rake = (double)nd.rake;
-            FastTask t{T_SHOWDOWN_BATCH, layout, S.slot + sv, S.node + v, NONE32, {0, 0, 0},
+            FastTask t{T_SHOWDOWN_BATCH, layout, S.slot + sv, S.node + v, NONE32, entries, {0, 0},
                        (hpot + (double)nd.invest[o] - rake) * norm, -(hpot + (double)nd.invest[p]) * norm,
                        0.5 * ((double)(nd.invest[o] - nd.invest[p]) - rake) * norm, 0.0};
             if (par.player == p)

@@ -113,7 +113,8 @@ struct FastTask {
   uint32_t slot;   // reach slot
   uint32_t row;    // value row (node id)
   uint32_t frow;   // paired fold's value row, or NONE32
-  uint32_t pad[3];
+  uint32_t entries;  // a batch's task: entries of its reach row (its opponent's hands, padded)
+  uint32_t pad[2];
   double a, b, c, d;  // as TermLane
 };
 

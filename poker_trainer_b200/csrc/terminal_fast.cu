@@ -168,7 +168,6 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   const int p = A.p, o = p ^ 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
   const bool multi = sizeof(R) == 4 && A.dims != nullptr;  // a batch's spots (FastArgsT::dims)
-  const int fetch = multi ? A.stride : hpo;
   __shared__ int s_claim[2];  // DYN: the first chunk, then the chunk after the current one
   int t0, t1;
   if constexpr (DYN) {
@@ -191,10 +190,15 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     }
   };
   if (!multi) stage_same(A.same);
-  auto prefetch = [&](int ti, int buf) {
-    const R* src = A.reach + (size_t)tasks[ti].slot * A.stride;
+  // A task's row: its opponent's hands and no more. Past them a batch's row may
+  // hold the other traversal's reach, which must not set the scale below; and
+  // the layout staged here may still be another spot's.
+  auto entries = [&](const FastTask& t) { return multi ? (int)t.entries : hpo; };
+  auto prefetch = [&](const FastTask& t, int buf) {
+    const R* src = A.reach + (size_t)t.slot * A.stride;
     R* dst = rbuf + (size_t)buf * A.stride;
-    for (int i = tid; i < fetch / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
+    const int n = entries(t);
+    for (int i = tid; i < n / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
     cp_async_commit();
   };
   uint32_t board = NONE32;
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   stage(T.board);
   pdl_wait();
   pdl_trigger();
-  prefetch(t0, 0);
+  prefetch(T, 0);
   if constexpr (!DYN) {
     const int per = (ntasks + gridDim.x - 1) / gridDim.x;
     turn_pass(A.turn, (ntasks + per - 1) / per);
@@ -240,6 +244,9 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     const bool first = DYN && ti == cbeg;
     if (first && tid == 0) s_claim[1] = (int)atomicAdd(counter, (uint32_t)FAST_DYN_CHUNK);
     const R* r = rbuf + (size_t)buf * A.stride;
+    const FastTask cur = T;
+    // The next task's record: its row is requested after barrier (1).
+    if (!DYN && ti + 1 < t1) T = tasks[ti + 1];
     // Row ti landed (own copies), partial maxima published.
     cp_async_wait_all();
     R mx = 0;
@@ -249,7 +256,8 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
         mx = row_max(mx, row_max(v.x, v.y));
       }
     } else {
-      for (int i = tid; i < fetch / 4; i += FAST_THREADS) {
+      const int n = entries(cur);
+      for (int i = tid; i < n / 4; i += FAST_THREADS) {
         const float4 v = reinterpret_cast<const float4*>(r)[i];
         mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
       }
@@ -267,9 +275,8 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     } else {
       next = ti + 1;
     }
-    if (next < t1) prefetch(next, buf ^ 1);
-    const FastTask cur = T;
-    if (next < t1) T = tasks[next];  // next task's record, loaded early
+    if (DYN && next < t1) T = tasks[next];
+    if (next < t1) prefetch(T, buf ^ 1);
     if (DYN && next != ti + 1) {
       cbeg = next;
       cend = min(t1, next + FAST_DYN_CHUNK);

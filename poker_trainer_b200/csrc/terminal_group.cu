@@ -272,7 +272,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
 // crosses from one unit to the next.
 // MULTI: a batch's spots, a unit each: the players' hand counts and the
 // identical-hand map change with the unit, and rows are fetched to their
-// common stride (a spot's entries past its own hands are zero).
+// common stride (the entries past the opponent's hands are not looked at).
 template <int GW, bool MULTI>
 __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
     group_terminal_kernel(FastArgs A, const FastTask* __restrict__ tasks, const TermUnit* __restrict__ units,
