@@ -139,16 +139,15 @@ __device__ __forceinline__ void stage_records(T* dst, const T* src, uint32_t cou
 // 20 warps 1018, 16 warps 1021; four hands 12 warps 1038, 16 warps 1080; one
 // hand 28 warps 1140). A node's work is by its own number of actions, not the
 // batch's largest: 37 spots of up to 8 actions 126 to 113.
-template <int MODE, int MAXA, bool SHARE>
+// STAGED: shared memory holds the plan records of the batch's largest spot; a
+// larger one's are read where they are (trees of 8,000 nodes and more).
+template <int MODE, int MAXA, bool SHARE, bool STAGED>
 __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
     batch_row_kernel(const __grid_constant__ BatchPass P) {
   extern __shared__ __align__(16) unsigned char smem_b[];
   using R = Row<RowShape<SHARE>::V>;
   constexpr int W = RowShape<SHARE>::WARPS, GS = RowShape<SHARE>::SLICES, V = RowShape<SHARE>::V;
   const RowSmem L(P.max_up, P.max_fix, P.max_down, P.max_slots, GS);
-  SegUp* ut = reinterpret_cast<SegUp*>(smem_b + L.up);
-  SegDown* ft = reinterpret_cast<SegDown*>(smem_b + L.fix);
-  SegDown* dt = reinterpret_cast<SegDown*>(smem_b + L.down);
   uint8_t* live = smem_b + L.live;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint8_t* any = smem_b + L.any + (SHARE ? 0 : (size_t)warp * P.max_slots);
@@ -167,18 +166,21 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
   if (do_up) {
     u0 = P.up_levs[U.up_lev];
     un = P.up_levs[U.up_lev + U.nup] - u0;
-    stage_records(ut, P.up + u0, un);
+    if constexpr (STAGED) stage_records(reinterpret_cast<SegUp*>(smem_b + L.up), P.up + u0, un);
     if (MODE == M_CFR) {
       f0 = P.up_levs[U.down_lev];
       fn = P.up_levs[U.down_lev + U.ndown] - f0;
-      stage_records(ft, P.fix + f0, fn);
+      if constexpr (STAGED) stage_records(reinterpret_cast<SegDown*>(smem_b + L.fix), P.fix + f0, fn);
     }
   }
   if (do_down) {
     d0 = P.down_levs[D.down_lev];
     dn = P.down_levs[D.down_lev + D.ndown] - d0;
-    stage_records(dt, P.down + d0, dn);
+    if constexpr (STAGED) stage_records(reinterpret_cast<SegDown*>(smem_b + L.down), P.down + d0, dn);
   }
+  const SegUp* const ut = STAGED ? reinterpret_cast<const SegUp*>(smem_b + L.up) : P.up + u0;
+  const SegDown* const ft = STAGED ? reinterpret_cast<const SegDown*>(smem_b + L.fix) : P.fix + f0;
+  const SegDown* const dt = STAGED ? reinterpret_cast<const SegDown*>(smem_b + L.down) : P.down + d0;
   for (uint32_t i = threadIdx.x; i < S.nslots * GS; i += W * 32)
     smem_b[L.any + (i / S.nslots) * P.max_slots + i % S.nslots] = 0;
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
@@ -372,14 +374,17 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
 }
 
 template <int MODE, bool SHARE>
-const void* row_fn(int maxa) {
-  if (maxa <= 4) return (const void*)batch_row_kernel<MODE, 4, SHARE>;
-  if (maxa <= 8) return (const void*)batch_row_kernel<MODE, 8, SHARE>;
-  return (const void*)batch_row_kernel<MODE, MAX_ACTIONS, SHARE>;
+const void* row_fn(int maxa, bool staged) {
+  if (!staged) return (const void*)batch_row_kernel<MODE, MAX_ACTIONS, SHARE, false>;
+  if (maxa <= 4) return (const void*)batch_row_kernel<MODE, 4, SHARE, true>;
+  if (maxa <= 8) return (const void*)batch_row_kernel<MODE, 8, SHARE, true>;
+  return (const void*)batch_row_kernel<MODE, MAX_ACTIONS, SHARE, true>;
 }
 template <bool SHARE>
-const void* row_fn(int mode, int maxa) {
-  return mode == M_CFR ? row_fn<M_CFR, SHARE>(maxa) : mode == M_BR ? row_fn<M_BR, SHARE>(maxa) : row_fn<M_AVG, SHARE>(maxa);
+const void* row_fn(int mode, int maxa, bool staged) {
+  return mode == M_CFR  ? row_fn<M_CFR, SHARE>(maxa, staged)
+         : mode == M_BR ? row_fn<M_BR, SHARE>(maxa, staged)
+                        : row_fn<M_AVG, SHARE>(maxa, staged);
 }
 
 // Shared memory of `warps` terminals in flight, one a warp, on the largest
@@ -495,6 +500,7 @@ struct Batch::Impl {
   std::vector<double> cost;
   int maxa = 1, max_slots = 1, stride = 8, slices = 1, tstride = 1, cstride = 8, emax = 1;
   uint64_t total_store = 0, total_slots = 0;
+  bool staged = true;  // row passes: plan records in shared memory
   size_t ntasks[2] = {0, 0}, nunits[2] = {0, 0}, ndown[2] = {0, 0};
   int max_up[2] = {0, 0}, max_down[2] = {0, 0};
   // Device.
@@ -866,16 +872,12 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   BK(cudaMemsetAsync(counter, 0, 4, stream));
   if (!(s = ensure_discounts(1024)).ok()) return s;
   BK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  staged = RowSmem(std::max(max_up[0], max_up[1]), std::max(max_down[0], max_down[1]), std::max(max_down[0], max_down[1]),
+                   max_slots, RowShape<false>::SLICES)
+               .total <= (size_t)optin;
   for (int mode : {M_CFR, M_BR, M_AVG})
-    for (const void* fn : {row_fn<true>(mode, maxa), row_fn<false>(mode, maxa)})
+    for (const void* fn : {row_fn<true>(mode, maxa, staged), row_fn<false>(mode, maxa, staged)})
       BK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  const size_t row_smem = RowSmem(std::max(max_up[0], max_up[1]), std::max(max_down[0], max_down[1]),
-                                  std::max(max_down[0], max_down[1]), max_slots, RowShape<false>::SLICES).total;
-  if (row_smem > (size_t)optin) {
-    s.code = DCFR_ERR_UNSUPPORTED;
-    s.msg = "a spot's tree needs more plan records than shared memory holds";
-    return s;
-  }
   int bps = 0;
   max_groups = group_terminal_setup(stride, cstride, tstride, group_warps, bps, true);
   const int fast_bps = fast_blocks_per_sm(stride, emax, cstride, tstride);
@@ -928,8 +930,8 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
     P.fix = down[up_p];
     P.up_levs = levs[up_p];
     P.up_deferred = deferred[up_p];
-    P.max_up = max_up[up_p];
-    P.max_fix = mode == M_CFR ? max_down[up_p] : 0;
+    P.max_up = staged ? max_up[up_p] : 0;
+    P.max_fix = staged && mode == M_CFR ? max_down[up_p] : 0;
     P.n_fix = (uint32_t)ndown[up_p];
     P.root_out = out;
   }
@@ -938,7 +940,7 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
     P.down_levs = levs[down_p];
     P.down_deferred = deferred[down_p];
     P.roots = roots;
-    P.max_down = max_down[down_p];
+    P.max_down = staged ? max_down[down_p] : 0;
     P.n_down = (uint32_t)ndown[down_p];
   }
   const bool share = P.nspots * slices <= BATCH_SHARE_ITEMS;
@@ -956,7 +958,8 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void* params[] = {(void*)&P};
-  cudaLaunchKernelExC(&cfg, share ? row_fn<true>(mode, maxa) : row_fn<false>(mode, maxa), params);
+  cudaLaunchKernelExC(&cfg, share ? row_fn<true>(mode, maxa, staged) : row_fn<false>(mode, maxa, staged),
+                      params);
 }
 
 // All spots' terminals of one traversal: a block per terminal while there
