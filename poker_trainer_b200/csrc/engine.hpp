@@ -43,7 +43,10 @@ void launch_strength(const uint8_t* boards, int nboards, const uint8_t* hc1_0, c
 void launch_fast_layouts(const EntryD* tables, const uint32_t* count, int tstride, int nboards, const uint8_t* hc1_0,
                          const uint8_t* hc2_0, const uint8_t* hc1_1, const uint8_t* hc2_1, int n0, int n1,
                          uint16_t* cat, uint16_t* seg, uint4* rec, int cstride, cudaStream_t s);
-void launch_fast_terminal(const FastArgs& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s);
+// settled: no kernel queued just before on s writes the tasks or layouts, so
+// they may be read while it runs (reach rows and flags are read after it).
+void launch_fast_terminal(const FastArgs& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s,
+                          bool settled = true);
 void launch_fast_terminal64(const FastArgs64& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s);
 void launch_warp_terminal(const FastArgs& A, const FastTask* tasks, const TermUnit* units, int nunits, int ntasks,
                           int warps,

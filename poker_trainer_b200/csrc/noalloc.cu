@@ -271,7 +271,8 @@ extern "C" int dcfr_showdown_values_noalloc(const uint8_t board[5], const uint8_
   A.hp[1] = (n_opp + 7) & ~7;
   A.stride = NA_HP;
   A.p = 0;
-  launch_fast_terminal(A, AT(FastTask, task), 1, 1, s);
+  // The kernels above write the task and its layout.
+  launch_fast_terminal(A, AT(FastTask, task), 1, 1, s, false);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(DCFR_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   e = cudaMemcpyAsync(out, AT(float, vals), (size_t)n_hero * sizeof(float), cudaMemcpyDeviceToDevice, s);

@@ -773,14 +773,17 @@ void launch_fast_layouts(const EntryD* tables, const uint32_t* count, int tstrid
 
 template <typename R>
 static void launch_fast_terminal_t(const FastArgsT<R>& A, const FastTask* tasks, int ntasks, int max_blocks,
-                                   cudaStream_t s) {
+                                   cudaStream_t s, bool settled) {
   if (ntasks <= 0) return;
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
   const size_t smem = fast_smem_bytes(A.stride, A.emax, A.cstride, A.tstride, (int)sizeof(R));
   switch (A.emax) {
-#define FAST_E(e_)                                                                     \
-  case e_:                                                                             \
-    launch_dependent(fast_terminal_kernel<e_, R>, (unsigned)blocks, FAST_THREADS, smem, s, A, tasks, ntasks, nullptr); \
+#define FAST_E(e_)                                                                                             \
+  case e_:                                                                                                     \
+    if (settled)                                                                                               \
+      launch_dependent(fast_terminal_kernel<e_, R>, (unsigned)blocks, FAST_THREADS, smem, s, A, tasks, ntasks, \
+                       nullptr);                                                                               \
+    else fast_terminal_kernel<e_, R><<<blocks, FAST_THREADS, smem, s>>>(A, tasks, ntasks);                     \
     break;
     FAST_E(1) FAST_E(3) FAST_E(5) FAST_E(7) FAST_E(9) FAST_E(11) FAST_E(13) FAST_E(15) FAST_E(17)
 #undef FAST_E
@@ -804,12 +807,13 @@ void launch_fast_terminal_dyn(const FastArgs& A, const FastTask* tasks, int ntas
   }
 }
 
-void launch_fast_terminal(const FastArgs& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s) {
-  launch_fast_terminal_t(A, tasks, ntasks, max_blocks, s);
+void launch_fast_terminal(const FastArgs& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s,
+                          bool settled) {
+  launch_fast_terminal_t(A, tasks, ntasks, max_blocks, s, settled);
 }
 
 void launch_fast_terminal64(const FastArgs64& A, const FastTask* tasks, int ntasks, int max_blocks, cudaStream_t s) {
-  launch_fast_terminal_t(A, tasks, ntasks, max_blocks, s);
+  launch_fast_terminal_t(A, tasks, ntasks, max_blocks, s, true);
 }
 
 }  // namespace dcfr
