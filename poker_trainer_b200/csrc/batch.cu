@@ -5,9 +5,9 @@
 // and bet menu) built by the same host code as a single solve (game.cpp), so
 // its tree, storage order and arithmetic are those of the reference solver
 // (crates/solver/src/tree.rs, cfr.rs, river.rs, eval.rs). The spots share one
-// numbering of reach slots, value rows and terminal tasks (rows of one stride;
-// a traversal writes its opponent's hands, and past them a reach row may hold
-// the other traversal's), and an iteration is four launches
+// numbering of reach slots, rows (each spot's as long as its own longer range; a
+// traversal writes its opponent's hands, and past them a reach row may hold the
+// other traversal's) and terminal tasks, and an iteration is four launches
 // over all of them: for each traversal a row pass and the terminals, the up
 // pass of a traversal being one launch with the down pass of the next.
 //   * Row passes (batch_row_kernel): everything is per hand, so a slice of 32
@@ -45,19 +45,26 @@ struct BatchPart {
 };
 struct SpotD {
   uint32_t slot;    // reach slot 0 of the spot (its root's)
-  uint32_t node;    // value row of its root
   uint32_t nslots;  // slots of its larger traversal
+  uint32_t reach;   // reach row of slot 0, and value row of the root (ROW_UNITs)
+  uint32_t vals;
+  int32_t stride;   // entries of its rows
   uint32_t pad;
   int32_t hp[2];
   BatchPart part[2];
 };
 
-// SegUp / SegDown (plan.hpp) with global value rows and slots counted from the
-// spot's first (gslot: global).
+// A block's work: a spot, and its slice or the first of its warps' slices.
+struct RowItem {
+  uint32_t spot, slice;
+};
+
+// SegUp / SegDown (plan.hpp) with slots counted from the spot's first, and rows
+// (node, child, gnode; gslot: the first child's reach row) in ROW_UNITs.
 struct BatchPass {
   const SpotD* spots;
-  const uint32_t* order;
-  int nspots, slices, stride;
+  const RowItem* items;
+  int stride;               // of roots and root_out
   int max_up, max_fix, max_down, max_slots;  // largest spot: records staged, slots
   uint32_t n_fix, n_down;   // down tasks of the up and of the down traversal
   float* regrets;
@@ -152,14 +159,14 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint8_t* any = smem_b + L.any + (SHARE ? 0 : (size_t)warp * P.max_slots);
   pdl_trigger();
-  const int per_spot = (P.slices + GS - 1) / GS;
-  const uint32_t sp = P.order[blockIdx.x / per_spot];
-  const int sl = (int)(blockIdx.x % per_spot) * GS + (SHARE ? 0 : warp);
+  const RowItem item = P.items[blockIdx.x];
+  const uint32_t sp = item.spot;
+  const int sl = (int)item.slice + (SHARE ? 0 : warp);
   const int w0 = SHARE ? warp : 0;
   constexpr int WS = SHARE ? W : 1;
   const SpotD S = P.spots[sp];
   const int h = sl * RowShape<SHARE>::SLICE + lane * V;  // the lane's first; hand counts are padded to eights
-  const size_t stride = (size_t)P.stride;
+  const size_t stride = (size_t)S.stride;
   const bool do_up = P.up_p >= 0, do_down = P.down_p >= 0;
   const BatchPart U = pick(do_up ? P.up_p : 0, S.part), D = pick(do_down ? P.down_p : 0, S.part);
   uint32_t u0 = 0, un = 0, f0 = 0, fn = 0, d0 = 0, dn = 0;
@@ -193,7 +200,7 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
   if (do_up)
     for (uint32_t i = threadIdx.x; i < S.nslots; i += W * 32) live[i] = pick(P.up_p, P.alive)[S.slot + i] != 0;
   __syncthreads();
-  if (!SHARE && sl >= P.slices) return;
+  if (!SHARE && sl * RowShape<SHARE>::SLICE >= S.stride) return;
   if (do_up) {
     const int hp = pick(P.up_p, S.hp), hpo = pick(P.up_p ^ 1, S.hp);
     if (MODE == M_CFR) {
@@ -235,7 +242,7 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
       for (uint32_t i = (SHARE ? P.up_levs[U.up_lev + l] - u0 : 0u) + w0; i < e; i += WS) {
         const SegUp& T = ut[i];
         if (live[T.slot] == 0 || h >= hp) continue;  // dead subtree
-        const float* vp = P.vals + (size_t)T.child * stride + h;
+        const float* vp = P.vals + (size_t)T.child * ROW_UNIT + h;
         R out{};
         by_actions<MAXA>((int)T.nchild, [&](auto most, int na) {
           constexpr int M = decltype(most)::value;
@@ -293,27 +300,27 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
             }
           }
         });
-        out.store(P.vals + (size_t)T.gnode * stride + h);
+        out.store(P.vals + (size_t)T.gnode * ROW_UNIT + h);
       }
       if (SHARE) __syncthreads();
     }
-    if (P.root_out && w0 == 0 && h < P.stride)
-      R::load(P.vals + (size_t)S.node * stride + h).store(P.root_out + ((size_t)sp * 2 + P.up_p) * stride + h);
+    if (P.root_out && w0 == 0 && h < S.stride)
+      R::load(P.vals + (size_t)S.vals * ROW_UNIT + h).store(P.root_out + ((size_t)sp * 2 + P.up_p) * P.stride + h);
   }
   if (do_down) {
-    uint32_t* alive = pick(P.down_p, P.alive);
+    uint32_t* alive = pick(P.down_p, P.alive) + S.slot;
     const int hp = pick(P.down_p ^ 1, S.hp);
     const bool valid = h < hp;
     if (w0 == 0) {
-      const R r = h < P.stride ? R::load(P.roots + ((size_t)sp * 2 + P.down_p) * stride + h) : R{};
-      if (h < P.stride) r.store(P.reach + (size_t)S.slot * stride + h);
+      const R r = h < S.stride ? R::load(P.roots + ((size_t)sp * 2 + P.down_p) * P.stride + h) : R{};
+      if (h < S.stride) r.store(P.reach + (size_t)S.reach * ROW_UNIT + h);
       bool some = false;
 #pragma unroll
       for (int j = 0; j < V; j++) some |= valid && r.x[j] != 0.0f;
       some = __any_sync(0xffffffffu, some);
       if (lane == 0) {
         any[0] = some ? 1 : 0;
-        if (sl == 0) alive[S.slot] = 1u;
+        if (sl == 0) alive[0] = 1u;
       }
     }
     if (SHARE) __syncthreads();
@@ -324,9 +331,9 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
         const SegDown& T = dt[i];
         const int na = (int)T.nchild;
         const bool some = any[T.in_slot] != 0;
-        float* to = P.reach + (size_t)T.gslot * stride + h;
+        float* to = P.reach + (size_t)T.gslot * ROW_UNIT + h;
         if (some) {
-          const R r = valid ? R::load(P.reach + (size_t)(S.slot + T.in_slot) * stride + h) : R{};
+          const R r = valid ? R::load(P.reach + (size_t)S.reach * ROW_UNIT + T.in_slot * stride + h) : R{};
           const float* from = (MODE == M_CFR ? P.regrets : P.sums) + T.gstore + h;
           float* sums = P.sums + T.gstore + h;
           uint32_t kids = 0;  // children that a hand of the lane reaches
@@ -360,7 +367,7 @@ __global__ void __launch_bounds__(RowShape<SHARE>::WARPS * 32, SHARE ? 3 : 5)
           kids = __reduce_or_sync(0xffffffffu, kids);
           if (kids >> lane & 1u) {
             any[T.out_slot + lane] = 1;
-            alive[T.gslot + lane] = 1u;
+            alive[T.out_slot + lane] = 1u;
           }
         } else if (valid) {
           for (int a = 0; a < na; a++) R{}.store(to + (size_t)a * stride);
@@ -498,7 +505,9 @@ struct Batch::Impl {
   std::vector<std::vector<uint64_t>> node_off;  // per spot, per node: float offset of a player block in the spot
   std::vector<uint64_t> spot_len;               // storage floats per spot
   std::vector<double> cost;
-  int maxa = 1, max_slots = 1, stride = 8, slices = 1, tstride = 1, cstride = 8, emax = 1;
+  int maxa = 1, max_slots = 1, stride = 8, tstride = 1, cstride = 8, emax = 1;
+  bool share = false;       // row passes: RowShape
+  int row_blocks = 0;
   uint64_t total_store = 0, total_slots = 0;
   bool staged = true;  // row passes: plan records in shared memory
   size_t ntasks[2] = {0, 0}, nunits[2] = {0, 0}, ndown[2] = {0, 0};
@@ -522,7 +531,7 @@ struct Batch::Impl {
   FastTask* term[2] = {nullptr, nullptr};
   TermUnit* units[2] = {nullptr, nullptr};
   SpotD* d_spots = nullptr;
-  uint32_t *order_lpt = nullptr, *order_nat = nullptr;
+  RowItem *items_lpt = nullptr, *items_nat = nullptr;
   DiscountD* disc = nullptr;
   DiscountD* cur_disc = nullptr;
   uint32_t disc_len = 0;
@@ -583,8 +592,8 @@ Batch::Impl::~Impl() {
   }
   bfree(cur_disc);
   bfree(d_spots);
-  bfree(order_lpt);
-  bfree(order_nat);
+  bfree(items_lpt);
+  bfree(items_nat);
   bfree(disc);
   bfree(counter);
   if (ev0) cudaEventDestroy(ev0);
@@ -661,7 +670,8 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   std::vector<uint32_t> hs;
   std::vector<float> hroot;
   std::vector<int4> hdims;
-  uint64_t nodes = 0;
+  uint64_t vals_len = 0, reach_len = 0;  // entries
+  int slices = 0;                         // of 32 hands
   spots.resize(count);
   store.resize(count);
   node_off.resize(count);
@@ -670,7 +680,6 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   for (int i = 0; i < count; i++) tstride = std::max(tstride, std::max(games[i].n[0], games[i].n[1]));
   cstride = (3 * tstride + 7) / 8 * 8;
   stride = std::max(8, pad8(tstride));
-  slices = (stride + 31) / 32;
   emax = fast_emax(tstride);
   for (int i = 0; i < count; i++) {
     const Game& g = games[i];
@@ -704,8 +713,12 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
     for (int p = 0; p < 2; p++)
       for (int h = 0; h < stride; h++) hroot.push_back(h < g.n[p ^ 1] ? g.weights[p ^ 1][h] : 0.0f);
     for (int k = 0; k < 5; k++) hb.push_back((uint8_t)g.board[k]);
+    S.stride = std::max(ROW_UNIT, std::max(hp0, hp1));
     S.slot = (uint32_t)total_slots;
-    S.node = (uint32_t)nodes;
+    S.reach = (uint32_t)(reach_len / ROW_UNIT);
+    S.vals = (uint32_t)(vals_len / ROW_UNIT);
+    const uint32_t units = (uint32_t)(S.stride / ROW_UNIT);  // of a row
+    slices += (S.stride + 31) / 32;
     const uint32_t layout = (uint32_t)(2 * i);
     // Traversal plans: slots, down tasks (breadth first), up tasks (deepest
     // first), terminals (showdowns with paired folds, and folds on the same
@@ -736,9 +749,9 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
           if (ups.size() <= depth[v]) ups.resize(depth[v] + 1), downs.resize(depth[v] + 1);
           const uint64_t at = store[i] + node_off[i][v];
           const float uniform = 1.0f / (float)nd.nchild;
-          if (!own) downs[depth[v]].push_back(SegDown{sv, first_slot, nd.nchild, 0, at, S.slot + first_slot, uniform});
-          ups[depth[v]].push_back(SegUp{own ? (uint32_t)U_OWN : (uint32_t)U_OPP_SUM, nd.nchild, sv, S.node + v,
-                                        S.node + nd.first, first_slot, 0, S.node + v, at, uniform, 0});
+          if (!own) downs[depth[v]].push_back(SegDown{sv, first_slot, nd.nchild, 0, at, S.reach + first_slot * units, uniform});
+          ups[depth[v]].push_back(SegUp{own ? (uint32_t)U_OWN : (uint32_t)U_OPP_SUM, nd.nchild, sv, S.vals + v * units,
+                                        S.vals + nd.first * units, first_slot, 0, S.vals + v * units, at, uniform, 0});
           work_units += nd.nchild;
         } else if (nd.kind == N_FOLD || nd.kind == N_SHOWDOWN) {
           // Every terminal of a river spot sits below a river decision node:
@@ -755,11 +768,11 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
             if (paired) continue;
             const int f = nd.player;
             const double val = f == p ? -(hpot + (double)nd.invest[p]) : hpot + (double)nd.invest[f] - (double)nd.rake;
-            folds.push_back(FastTask{T_FOLD_BATCH, layout, S.slot + sv, S.node + v, NONE32, entries, {0, 0}, val * norm,
-                                     0.0, 0.0, 0.0});
+            folds.push_back(FastTask{T_FOLD_BATCH, layout, S.slot + sv, S.vals + v * units, NONE32, S.reach + sv * units,
+                                     entries, 0, val * norm, 0.0, 0.0, 0.0});
           } else {
             const double rake = (double)nd.rake;
-            FastTask t{T_SHOWDOWN_BATCH, layout, S.slot + sv, S.node + v, NONE32, entries, {0, 0},
+            FastTask t{T_SHOWDOWN_BATCH, layout, S.slot + sv, S.vals + v * units, NONE32, S.reach + sv * units, entries, 0,
                        (hpot + (double)nd.invest[o] - rake) * norm, -(hpot + (double)nd.invest[p]) * norm,
                        0.5 * ((double)(nd.invest[o] - nd.invest[p]) - rake) * norm, 0.0};
             if (par.player == p)
@@ -769,7 +782,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
                   const int f = fn.player;
                   const double val =
                       f == p ? -(hpot + (double)fn.invest[p]) : hpot + (double)fn.invest[f] - (double)fn.rake;
-                  t.frow = S.node + c;
+                  t.frow = S.vals + c * units;
                   t.d = val * norm;
                 }
             sds.push_back(t);
@@ -804,12 +817,18 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
     }
     max_slots = std::max<int>(max_slots, (int)S.nslots);
     total_slots += S.nslots;
-    nodes += N;
-    cost[i] = (double)work_units * (double)stride;
+    vals_len += N * S.stride;
+    reach_len += (uint64_t)S.nslots * S.stride;
+    cost[i] = (double)work_units * (double)S.stride;
   }
   if (max_slots > BATCH_MAX_SLOTS) {
     s.code = DCFR_ERR_UNSUPPORTED;
     s.msg = "a spot's tree needs more than " + std::to_string(BATCH_MAX_SLOTS) + " reach slots";
+    return s;
+  }
+  if (std::max(vals_len, reach_len) / ROW_UNIT >= NONE32) {
+    s.code = DCFR_ERR_UNSUPPORTED;
+    s.msg = "the batch's rows pass what a 32-bit row number counts";
     return s;
   }
   // Device arrays.
@@ -817,11 +836,11 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
   if (!(s = balloc(sums, total_store, "batch storage")).ok()) return s;
   BK(cudaMemsetAsync(regrets, 0, std::max<uint64_t>(total_store, 1) * 4, stream));
   BK(cudaMemsetAsync(sums, 0, std::max<uint64_t>(total_store, 1) * 4, stream));
-  if (!(s = balloc(vals, nodes * stride, "batch value rows")).ok()) return s;
-  if (!(s = balloc(reach, total_slots * stride, "batch reach rows")).ok()) return s;
+  if (!(s = balloc(vals, vals_len, "batch value rows")).ok()) return s;
+  if (!(s = balloc(reach, reach_len, "batch reach rows")).ok()) return s;
   if (!(s = balloc(alive, 2 * total_slots, "batch liveness flags")).ok()) return s;
-  BK(cudaMemsetAsync(vals, 0, std::max<uint64_t>(nodes * stride, 1) * 4, stream));
-  BK(cudaMemsetAsync(reach, 0, std::max<uint64_t>(total_slots * stride, 1) * 4, stream));
+  BK(cudaMemsetAsync(vals, 0, std::max<uint64_t>(vals_len, 1) * 4, stream));
+  BK(cudaMemsetAsync(reach, 0, std::max<uint64_t>(reach_len, 1) * 4, stream));
   if (!(s = upload(hc1, h1, "batch hands")).ok()) return s;
   if (!(s = upload(hc2, h2, "batch hands")).ok()) return s;
   if (!(s = upload(same, hs, "batch hands")).ok()) return s;
@@ -838,15 +857,28 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
     if (!(s = upload(levs[p], hlevs[p], "batch plan")).ok()) return s;
     if (!(s = upload(term[p], hterm[p], "batch plan")).ok()) return s;
     if (!(s = upload(units[p], hunits[p], "batch plan")).ok()) return s;
-    if (!(s = balloc(deferred[p], hdown[p].size() * slices, "batch plan")).ok()) return s;
+    if (!(s = balloc(deferred[p], hdown[p].size() * ((stride + 31) / 32), "batch plan")).ok()) return s;
   }
   if (!(s = upload(d_spots, spots, "batch plan")).ok()) return s;
-  std::vector<uint32_t> nat(count), lpt(count);
-  std::iota(nat.begin(), nat.end(), 0u);
-  lpt = nat;
-  std::stable_sort(lpt.begin(), lpt.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
-  if (!(s = upload(order_nat, nat, "batch order")).ok()) return s;
-  if (!(s = upload(order_lpt, lpt, "batch order")).ok()) return s;
+  // The row passes' blocks, spots in input order and longest first. A block's
+  // warps share a slice while there are too few slices to give every warp its
+  // own (us an iteration, shared against not: 37 spots of 34 slices 152 against
+  // 334, 512 spots 2113 against 1347).
+  share = slices <= BATCH_SHARE_ITEMS;
+  std::vector<uint32_t> order(count);
+  std::iota(order.begin(), order.end(), 0u);
+  auto items = [&] {
+    const int hands = share ? RowShape<true>::SLICE : RowShape<false>::SLICE;
+    const int per = share ? RowShape<true>::SLICES : RowShape<false>::SLICES;
+    std::vector<RowItem> v;
+    for (uint32_t i : order)
+      for (int sl = 0; sl * hands < spots[i].stride; sl += per) v.push_back(RowItem{i, (uint32_t)sl});
+    return v;
+  };
+  row_blocks = (int)items().size();
+  if (!(s = upload(items_nat, items(), "batch order")).ok()) return s;
+  std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
+  if (!(s = upload(items_lpt, items(), "batch order")).ok()) return s;
   // Strength tables and scan layouts, per spot (its board and fold layouts).
   if (!(s = balloc(tables, (size_t)count * 2 * tstride, "batch strength tables")).ok()) return s;
   if (!(s = balloc(tcount, (size_t)count * 2, "batch strength tables")).ok()) return s;
@@ -880,7 +912,7 @@ Status Batch::Impl::init(const dcfr_config* cfgs, int count) {
       BK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   int bps = 0;
   max_groups = group_terminal_setup(stride, cstride, tstride, group_warps, bps, true);
-  const int fast_bps = fast_blocks_per_sm(stride, emax, cstride, tstride);
+  const int fast_bps = fast_blocks_per_sm(stride, emax, cstride, tstride, true);
   if (max_groups <= 0 || fast_bps <= 0) {
     s.code = DCFR_ERR_UNSUPPORTED;
     s.msg = "batched kernel: a spot's layout does not fit in shared memory";
@@ -904,15 +936,11 @@ int Batch::Impl::occupancy(int warps) const {
 }
 
 // A row pass over all spots: the up pass of traverser up_p, then the down
-// pass of down_p (-1: not wanted). A block's warps share a slice while there
-// are too few slices to give every warp its own (us an iteration, shared
-// against not: 37 spots of 34 slices 152 against 334, 512 spots 2113 against
-// 1347).
+// pass of down_p (-1: not wanted).
 void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out, bool next) {
   BatchPass P{};
   P.spots = d_spots;
-  P.order = lpt ? order_lpt : order_nat;
-  P.nspots = (int)spots.size();
+  P.items = lpt ? items_lpt : items_nat;
   P.stride = stride;
   P.max_slots = max_slots;
   P.regrets = regrets;
@@ -943,12 +971,9 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
     P.max_down = staged ? max_down[down_p] : 0;
     P.n_down = (uint32_t)ndown[down_p];
   }
-  const bool share = P.nspots * slices <= BATCH_SHARE_ITEMS;
-  const int hands = share ? RowShape<true>::SLICE : RowShape<false>::SLICE;
-  P.slices = (stride + hands - 1) / hands;
   const int per = share ? RowShape<true>::SLICES : RowShape<false>::SLICES;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(P.nspots * ((P.slices + per - 1) / per)));
+  cfg.gridDim = dim3((unsigned)row_blocks);
   cfg.blockDim = dim3((unsigned)((share ? RowShape<true>::WARPS : RowShape<false>::WARPS) * 32));
   cfg.dynamicSmemBytes = RowSmem(P.max_up, P.max_fix, P.max_down, P.max_slots, per).total;
   cfg.stream = stream;

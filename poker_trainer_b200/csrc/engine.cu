@@ -949,13 +949,13 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
   auto sd_task = [&](uint32_t i) {
     const SdLane& x = sd[i];
     const TermLane& L = x.lane;
-    return FastTask{x.kind, x.board, L.slot, L.row, L.frow, 0, {0, 0}, L.a, L.b, L.c, L.d};
+    return FastTask{x.kind, x.board, L.slot, L.row, L.frow, 0, 0, 0, L.a, L.b, L.c, L.d};
   };
   auto fold_task = [&](uint32_t i) {
     const bool b = i >= folds[0].size();
     const TermLane& L = b ? folds[1][i - folds[0].size()] : folds[0][i];
     return FastTask{b ? (uint32_t)T_FOLD_BATCH : (uint32_t)T_FOLD_SCALAR, fold_layout[i], L.slot, L.row, NONE32,
-                    0, {0, 0}, L.a, 0.0, 0.0, 0.0};
+                    0, 0, 0, L.a, 0.0, 0.0, 0.0};
   };
   // Within a layout, showdowns and folds are interleaved evenly in chunks of
   // PT tasks (after k chunks, about k |S| / (|S| + |F|) showdown chunks).

@@ -77,7 +77,7 @@ void launch_fused_down64(const Row64Args& A, const FusedTree* trees, int ntrees,
 void launch_fused_up64(int mode, const Row64Args& A, const FusedTree* trees, int ntrees, const UpTask* tasks,
                        cudaStream_t s);
 int fast_emax(int tstride);
-int fast_blocks_per_sm(int stride, int emax, int cstride, int tstride);
+int fast_blocks_per_sm(int stride, int emax, int cstride, int tstride, bool multi = false);
 void launch_evaluate(const unsigned long long* masks, uint32_t* out, int n, cudaStream_t s);
 void launch_five_card_counts(unsigned long long* counts, cudaStream_t s);
 // counter non-null: also advance the DCFR iteration (t += 1, the discounts

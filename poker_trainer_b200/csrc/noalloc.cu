@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(1024) noalloc_prep_kernel(Scratch* S, const __
     t.slot = 0;
     t.row = 0;
     t.frow = NONE32;
-    t.entries = t.pad[0] = t.pad[1] = 0;
+    t.reach = t.entries = t.pad = 0;
     t.a = P.win;
     t.b = P.lose;
     t.c = P.tie;

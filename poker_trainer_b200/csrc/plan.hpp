@@ -113,8 +113,11 @@ struct FastTask {
   uint32_t slot;   // reach slot
   uint32_t row;    // value row (node id)
   uint32_t frow;   // paired fold's value row, or NONE32
-  uint32_t entries;  // a batch's task: entries of its reach row (its opponent's hands, padded)
-  uint32_t pad[2];
+  // A batch's task, whose spot has rows of its own length: its reach row, which
+  // like row and frow counts ROW_UNITs there, and the row's entries (the
+  // opponent's hands, padded).
+  uint32_t reach, entries;
+  uint32_t pad;
   double a, b, c, d;  // as TermLane
 };
 
@@ -165,6 +168,7 @@ struct PanelD {
 // aw | as << 16, bw | bs << 16, a | b << 8 | present << 16}: w (s) counts the
 // opponent hands weaker than (not stronger than) h, aw/as (bw/bs) index the
 // same boundaries inside card a's (b's) segment.
+constexpr int ROW_UNIT = 8;  // rows are padded to this many hands
 constexpr int FAST_SEGS = 54;
 constexpr int FAST_THREADS = 256;
 

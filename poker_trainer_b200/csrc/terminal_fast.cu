@@ -147,9 +147,12 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // so blocks whose tasks are cheap (dead subtrees are skipped) take more.
 // A block claims its next chunk while it starts the current one, so the
 // next task's row can still be prefetched across the chunk boundary.
+//
+// MULTI: a batch's spots (FastArgsT::dims): hand counts and the identical-hand
+// map change with the layout, and a task says how long its reach row is.
 constexpr int FAST_DYN_CHUNK = 8;
 
-template <int E, typename R, bool DYN = false>
+template <int E, typename R, bool DYN = false, bool MULTI = false>
 __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R> A, const FastTask* __restrict__ tasks,
                                                                      int ntasks, uint32_t* __restrict__ counter = nullptr) {
   extern __shared__ __align__(16) unsigned char smem_fast[];
@@ -167,7 +170,6 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
 
   const int p = A.p, o = p ^ 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
-  const bool multi = sizeof(R) == 4 && A.dims != nullptr;  // a batch's spots (FastArgsT::dims)
   __shared__ int s_claim[2];  // DYN: the first chunk, then the chunk after the current one
   int t0, t1;
   if constexpr (DYN) {
@@ -189,13 +191,13 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
       ssame[h] = sm == NONE32 ? (uint16_t)0xFFFF : (uint16_t)sm;
     }
   };
-  if (!multi) stage_same(A.same);
+  if (!MULTI) stage_same(A.same);
   // A task's row: its opponent's hands and no more. Past them a batch's row may
   // hold the other traversal's reach, which must not set the scale below; and
   // the layout staged here may still be another spot's.
-  auto entries = [&](const FastTask& t) { return multi ? (int)t.entries : hpo; };
+  auto entries = [&](const FastTask& t) { return MULTI ? (int)t.entries : hpo; };
   auto prefetch = [&](const FastTask& t, int buf) {
-    const R* src = A.reach + (size_t)t.slot * A.stride;
+    const R* src = A.reach + (MULTI ? (size_t)t.reach * ROW_UNIT : (size_t)t.slot * A.stride);
     R* dst = rbuf + (size_t)buf * A.stride;
     const int n = entries(t);
     for (int i = tid; i < n / PER16; i += FAST_THREADS) cp_async16(dst + PER16 * i, src + PER16 * i);
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   auto stage = [&](uint32_t b) {
     board = b;
     const size_t lay = (size_t)board * 2 + p;
-    if (multi) {
+    if (MULTI) {
       const int4 d = A.dims[board >> 1];
       np = p ? d.y : d.x;
       hpp = p ? d.w : d.z;
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
   stage(T.board);
   pdl_wait();
   pdl_trigger();
-  prefetch(T, 0);
+  prefetch(MULTI ? T : tasks[t0], 0);
   if constexpr (!DYN) {
     const int per = (ntasks + gridDim.x - 1) / gridDim.x;
     turn_pass(A.turn, (ntasks + per - 1) / per);
@@ -244,9 +246,8 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     const bool first = DYN && ti == cbeg;
     if (first && tid == 0) s_claim[1] = (int)atomicAdd(counter, (uint32_t)FAST_DYN_CHUNK);
     const R* r = rbuf + (size_t)buf * A.stride;
-    const FastTask cur = T;
-    // The next task's record: its row is requested after barrier (1).
-    if (!DYN && ti + 1 < t1) T = tasks[ti + 1];
+    FastTask ahead = T;  // MULTI: the next task's record, whose row is requested after barrier (1)
+    if (MULTI && ti + 1 < t1) ahead = tasks[ti + 1];
     // Row ti landed (own copies), partial maxima published.
     cp_async_wait_all();
     R mx = 0;
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
         mx = row_max(mx, row_max(v.x, v.y));
       }
     } else {
-      const int n = entries(cur);
+      const int n = entries(T);
       for (int i = tid; i < n / 4; i += FAST_THREADS) {
         const float4 v = reinterpret_cast<const float4*>(r)[i];
         mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
@@ -275,8 +276,9 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
     } else {
       next = ti + 1;
     }
-    if (DYN && next < t1) T = tasks[next];
-    if (next < t1) prefetch(T, buf ^ 1);
+    if (next < t1) prefetch(MULTI ? ahead : tasks[next], buf ^ 1);
+    const FastTask cur = T;
+    if (next < t1) T = MULTI ? ahead : tasks[next];  // next task's record, loaded early
     if (DYN && next != ti + 1) {
       cbeg = next;
       cend = min(t1, next + FAST_DYN_CHUNK);
@@ -327,8 +329,9 @@ __global__ void __launch_bounds__(FAST_THREADS) fast_terminal_kernel(FastArgsT<R
 
     // Values in hand order. Card c's segment runs from sseg[1+c] to sseg[2+c].
     const long long T0 = G[sseg[1]];
-    R* out = A.vals + (size_t)cur.row * A.stride;
-    R* fout = cur.frow != NONE32 ? A.vals + (size_t)cur.frow * A.stride : nullptr;
+    const size_t unit = MULTI ? ROW_UNIT : A.stride;
+    R* out = A.vals + cur.row * unit;
+    R* fout = cur.frow != NONE32 ? A.vals + cur.frow * unit : nullptr;
     const uint32_t kind = cur.kind;
     const bool fold = kind == T_FOLD_SCALAR || kind == T_FOLD_BATCH;
     const bool scalar = kind == T_FOLD_SCALAR || kind == T_SHOWDOWN_SCALAR;
@@ -409,14 +412,17 @@ static cudaError_t allow_dynamic_smem(const void* fn, int optin) {
 }
 
 template <int E>
-static cudaError_t setup_e(int optin, size_t smem, int& blocks) {
+static cudaError_t setup_e(int optin, size_t smem, bool multi, int& blocks) {
   cudaError_t e = allow_dynamic_smem((const void*)fast_terminal_kernel<E, float>, optin);
   if (e != cudaSuccess) return e;
   e = allow_dynamic_smem((const void*)fast_terminal_kernel<E, double>, optin);
   if (e != cudaSuccess) return e;
   e = allow_dynamic_smem((const void*)fast_terminal_kernel<E, float, true>, optin);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fast_terminal_kernel<E, float>, FAST_THREADS, smem);
+  e = allow_dynamic_smem((const void*)fast_terminal_kernel<E, float, false, true>, optin);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &blocks, multi ? fast_terminal_kernel<E, float, false, true> : fast_terminal_kernel<E, float>, FAST_THREADS, smem);
 }
 
 int fast_emax(int tstride) {
@@ -428,7 +434,7 @@ size_t fast_smem_bytes(int stride, int emax, int cstride, int tstride, int rsize
   return FastSmem(stride, emax, cstride, tstride, rsize).total;
 }
 
-int fast_blocks_per_sm(int stride, int emax, int cstride, int tstride) {
+int fast_blocks_per_sm(int stride, int emax, int cstride, int tstride, bool multi) {
   int blocks = 0;
   const size_t smem = fast_smem_bytes(stride, emax, cstride, tstride, 4);
   // The limit is the device's opt-in maximum (a per-kernel setting shared by
@@ -442,7 +448,7 @@ int fast_blocks_per_sm(int stride, int emax, int cstride, int tstride) {
   switch (emax) {
 #define FAST_E(e_)                          \
   case e_:                                  \
-    e = setup_e<e_>(optin, smem, blocks);   \
+    e = setup_e<e_>(optin, smem, multi, blocks); \
     break;
     FAST_E(1) FAST_E(3) FAST_E(5) FAST_E(7) FAST_E(9) FAST_E(11) FAST_E(13) FAST_E(15) FAST_E(17)
 #undef FAST_E
@@ -778,12 +784,15 @@ static void launch_fast_terminal_t(const FastArgsT<R>& A, const FastTask* tasks,
   const int blocks = ntasks < max_blocks ? ntasks : max_blocks;
   const size_t smem = fast_smem_bytes(A.stride, A.emax, A.cstride, A.tstride, (int)sizeof(R));
   switch (A.emax) {
-#define FAST_E(e_)                                                                                             \
-  case e_:                                                                                                     \
-    if (settled)                                                                                               \
-      launch_dependent(fast_terminal_kernel<e_, R>, (unsigned)blocks, FAST_THREADS, smem, s, A, tasks, ntasks, \
-                       nullptr);                                                                               \
-    else fast_terminal_kernel<e_, R><<<blocks, FAST_THREADS, smem, s>>>(A, tasks, ntasks);                     \
+#define FAST_E(e_)                                                                                                  \
+  case e_:                                                                                                          \
+    if (sizeof(R) == 4 && A.dims)                                                                                   \
+      launch_dependent(fast_terminal_kernel<e_, R, false, sizeof(R) == 4>, (unsigned)blocks, FAST_THREADS, smem, s, \
+                       A, tasks, ntasks, nullptr);                                                                  \
+    else if (settled)                                                                                               \
+      launch_dependent(fast_terminal_kernel<e_, R>, (unsigned)blocks, FAST_THREADS, smem, s, A, tasks, ntasks,      \
+                       nullptr);                                                                                    \
+    else fast_terminal_kernel<e_, R><<<blocks, FAST_THREADS, smem, s>>>(A, tasks, ntasks);                          \
     break;
     FAST_E(1) FAST_E(3) FAST_E(5) FAST_E(7) FAST_E(9) FAST_E(11) FAST_E(13) FAST_E(15) FAST_E(17)
 #undef FAST_E

@@ -66,30 +66,31 @@ __device__ __forceinline__ void group_sync(int id) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(32 * GW) : "memory");
 }
 
-// The group's threads copy the row of `slot` in 16-byte chunks: thread gt
+// The group's threads copy `entries` entries of a row in 16-byte chunks: thread gt
 // takes chunks gt, gt + GT, ... (the same chunks it reads back
 // for its part of the row maximum).
 template <int GW>
-__device__ __forceinline__ void group_row_prefetch(const FastArgs& A, int hpo, uint32_t slot, float* row, int gt) {
+__device__ __forceinline__ void group_row_prefetch(const float* from, int entries, float* row, int gt) {
   constexpr int GT = 32 * GW;
-  const char* src = reinterpret_cast<const char*>(A.reach + (size_t)slot * A.stride);
+  const char* src = reinterpret_cast<const char*>(from);
   const uint32_t dst = (uint32_t)__cvta_generic_to_shared(row);
-  for (int i = gt; i < hpo / 4; i += GT)
+  for (int i = gt; i < entries / 4; i += GT)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 16 * (size_t)i)
                  : "memory");
 }
 
 // One terminal task evaluated by the GT threads of a group (gt
 // = thread in the group). row: the group's copy of the task's reach row, its
-// own chunks waited for by every thread. next_slot / next_row: the row to
-// request after barrier (1) (NONE32: none), `fetch` entries of it. bfirst: the first segment
+// own chunks waited for by every thread. next / next_row: the row to
+// request after barrier (1) (null: none), next_entries entries of it. bfirst: the first segment
 // boundary b >= 1 with seg[b] >= this thread's first scan element.
-template <int GW>
+template <int GW, bool MULTI>
 __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T, const WarpLayout& Y, int hpo, int hpp,
-                                           int np, int fetch, const float* row, long long* G, long long* cst,
-                                           long long* gsum, float* gmax, int gt, int bar, int bfirst,
-                                           uint32_t next_slot, float* next_row) {
+                                           int np, const float* row, long long* G, long long* cst, long long* gsum,
+                                           float* gmax, int gt, int bar, int bfirst, const float* next,
+                                           int next_entries, float* next_row) {
   constexpr int GT = 32 * GW;
+  const size_t unit = MULTI ? ROW_UNIT : A.stride;  // of value rows
   const int lane = gt & 31, w = gt >> 5;
   const int L = Y.L;
   // 1. Row maximum: each thread's own copied chunks, then the group's.
@@ -102,7 +103,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
   if (lane == 0) gmax[w] = mx;
   group_sync<GW>(bar);  // (1)
-  if (next_slot != NONE32) group_row_prefetch<GW>(A, fetch, next_slot, next_row, gt);
+  if (next) group_row_prefetch<GW>(next, next_entries, next_row, gt);
   cp_async_commit();
 #pragma unroll
   for (int k = 0; k < GW; k++) mx = fmaxf(mx, gmax[k]);
@@ -112,7 +113,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   const uint32_t kind = T.kind;
   const bool fold = kind == T_FOLD_SCALAR || kind == T_FOLD_BATCH;
   const bool scalar = kind == T_FOLD_SCALAR || kind == T_SHOWDOWN_SCALAR;
-  float* out = A.vals + (size_t)T.row * A.stride;
+  float* out = A.vals + T.row * unit;
   if (fold) {
     // eval_fold (eval.rs:40-64): the total and each card's total.
     long long t0 = 0;
@@ -211,7 +212,7 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
   // is card 0's start.
   const longlong2* cpair = reinterpret_cast<const longlong2*>(cst);
   const long long T0 = cst[0];
-  float* fout = T.frow != NONE32 ? A.vals + (size_t)T.frow * A.stride : nullptr;
+  float* fout = T.frow != NONE32 ? A.vals + T.frow * unit : nullptr;
   auto value = [&](int h, float& v, float& fv) {
     v = 0.0f;
     fv = 0.0f;
@@ -271,8 +272,9 @@ __device__ __forceinline__ void group_task(const FastArgs& A, const FastTask& T,
 // tasks on one layout) once, with a block barrier only where its range
 // crosses from one unit to the next.
 // MULTI: a batch's spots, a unit each: the players' hand counts and the
-// identical-hand map change with the unit, and rows are fetched to their
-// common stride (the entries past the opponent's hands are not looked at).
+// identical-hand map change with the unit, and a task says where its rows are and
+// how long its reach row is (past the opponent's hands it may hold the other
+// traversal's reach).
 template <int GW, bool MULTI>
 __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
     group_terminal_kernel(FastArgs A, const FastTask* __restrict__ tasks, const TermUnit* __restrict__ units,
@@ -297,7 +299,10 @@ __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
 
   const int p = A.p, o = p ^ 1;
   int hpo = o ? A.hp[1] : A.hp[0], hpp = p ? A.hp[1] : A.hp[0], np = p ? A.n[1] : A.n[0];
-  const int fetch = MULTI ? A.stride : hpo;
+  auto row_of = [&](const FastTask& t) {
+    return A.reach + (MULTI ? (size_t)t.reach * ROW_UNIT : (size_t)t.slot * A.stride);
+  };
+  auto entries = [&](const FastTask& t) { return MULTI ? (int)t.entries : hpo; };
   auto stage_same = [&](const uint32_t* same) {
     for (int h = tid; h < hpp; h += blockDim.x) {
       const uint32_t sm = h < np ? same[h] : NONE32;
@@ -345,7 +350,7 @@ __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
   bool live = false;
   if (next < t1) {
     live = A.alive[tasks[next].slot] != 0;
-    if (live) group_row_prefetch<GW>(A, fetch, tasks[next].slot, row_a, gt);
+    if (live) group_row_prefetch<GW>(row_of(tasks[next]), entries(tasks[next]), row_a, gt);
   }
   cp_async_commit();
   for (; u < nunits && (int)units[u].first < t1; u++) {
@@ -369,14 +374,14 @@ __global__ void __launch_bounds__(32 * GW * group_max(GW), 1)
       float* const nxt_row = buf ? row_a : row_b;
       // Dead subtree (cfr.rs:267-274): row untouched.
       if (live) {
-        group_task<GW>(A, tasks[next], Y, hpo, hpp, np, fetch, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
-                   nlive ? tasks[nx].slot : NONE32, nxt_row);
+        group_task<GW, MULTI>(A, tasks[next], Y, hpo, hpp, np, cur_row, G, cst, gsum, gmax, gt, bar, bfirst,
+                              nlive ? row_of(tasks[nx]) : nullptr, nlive ? entries(tasks[nx]) : 0, nxt_row);
       } else {
         // The group's other warps may still read the previous task's row
         // from the buffer the next row goes to.
         if (nlive) {
           group_sync<GW>(bar);
-          group_row_prefetch<GW>(A, fetch, tasks[nx].slot, nxt_row, gt);
+          group_row_prefetch<GW>(row_of(tasks[nx]), entries(tasks[nx]), nxt_row, gt);
         }
         cp_async_commit();
       }

@@ -54,3 +54,25 @@ def test_past_the_slot_limit(gpu):
     with pytest.raises(SolverError) as e:
         BatchSolver.new([spot(TOO_LARGE, (31, 50))])
     assert e.value.code == abi.ERR_UNSUPPORTED
+
+
+def device_bytes(cfgs):
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    b = BatchSolver.new(cfgs)
+    taken = before - torch.cuda.mem_get_info()[0]
+    b.close()
+    return taken
+
+
+def test_narrow_spots_beside_a_wide_one(gpu):
+    """A spot's rows are as long as its own ranges. What is common to a batch is
+    about 105 KB a spot of 1081 hands (its scan layouts), and the arrays are
+    allocated in pieces of 2 MB."""
+    tree = (["50%", "100%", "allin"], ["50%", "100%", "allin"], 3, 700, 9000)
+    narrow = [spot(tree, (60, 47), i) for i in range(480)]
+    wide = [spot(SMALL, (1081, 1000))]
+    device_bytes(wide)  # the context's own
+    apart = device_bytes(narrow) + device_bytes(wide)
+    assert device_bytes(narrow + wide) <= apart + (len(narrow) + 1) * 110_000 + (24 << 20)
