@@ -433,7 +433,7 @@ typedef struct dcfr_batch_tuning {
   int32_t longest_first;          /* 1: spots taken by decreasing work; 0: input order */
   int32_t candidates;             /* autotune: candidates timed */
   int32_t _pad;
-  double trial_ms;                /* autotune: the best candidate's time */
+  double trial_ms;                /* autotune: the best candidate's time for trial_iterations */
 } dcfr_batch_tuning;
 
 int dcfr_batch_create(const dcfr_config* cfgs, int32_t count, dcfr_batch** out);
@@ -445,8 +445,9 @@ int dcfr_batch_exploitability(dcfr_batch* b, double* out);
 /* One spot's storage in the reference layout (as dcfr_download_storage). */
 int dcfr_batch_storage_len(const dcfr_batch* b, int32_t spot, uint64_t* len);
 int dcfr_batch_download_storage(dcfr_batch* b, int32_t spot, float* regrets, float* sums, uint64_t len);
-/* Times every launch shape that fits on trial_iterations iterations from a
- * snapshot of the storage (restored after each trial) and keeps the fastest. */
+/* Times every launch shape that fits on trial_iterations iterations and two
+ * more, which run outside graphs, from a snapshot of the storage (restored after
+ * each trial), and keeps the fastest. */
 int dcfr_batch_autotune(dcfr_batch* b, uint32_t trial_iterations, dcfr_batch_tuning* out);
 int dcfr_batch_get_tuning(const dcfr_batch* b, dcfr_batch_tuning* out);
 int dcfr_batch_set_tuning(dcfr_batch* b, const dcfr_batch_tuning* t);

@@ -394,8 +394,9 @@ const void* row_fn(int mode, int maxa, bool staged) {
                         : row_fn<M_AVG, SHARE>(maxa, staged);
 }
 
-// Shared memory of `warps` terminals in flight, one a warp, on the largest
-// spot: what bounds dcfr_batch_tuning::warps.
+// What dcfr_batch_tuning::warps is accepted up to: shared memory for that many
+// terminals, one a warp, on the largest spot. (The kernels take no more
+// terminals a block than fit them, whatever is set: Impl::max_groups.)
 size_t tuning_smem(int stride, int cstride, int tstride, int max_slots, int warps) {
   auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
   const size_t fixed = up16((size_t)max_slots * 4) + up16(sizeof(DiscountD)) + 16 + up16((size_t)stride * 2) +
@@ -549,6 +550,7 @@ struct Batch::Impl {
   ~Impl();
   Status init(const dcfr_config* cfgs, int count);
   int occupancy(int warps) const;
+  bool by_blocks(int p) const;
   void enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* out, bool next = false);
   void enqueue_terminals(int p, const dcfr_batch_tuning& t, const PassTurn& turn = PassTurn());
   void enqueue_start(bool advance);
@@ -987,10 +989,15 @@ void Batch::Impl::enqueue_rows(int mode, int up_p, int down_p, bool lpt, float* 
                       params);
 }
 
-// All spots' terminals of one traversal: a block per terminal while there
-// are few of them or hand lists so long that few groups fit a block, two warps
-// per terminal otherwise (1081 hands, five groups, us an iteration, block
-// against group kernel: 37 spots 126 against 135, 512 spots 1148 against 1134).
+// Whether a traversal's terminals take a block each: while there are few of
+// them or hand lists so long that few groups fit a block (1081 hands, five
+// groups, us an iteration, block against group kernel: 37 spots 126 against 135,
+// 512 spots 1148 against 1134). Otherwise two warps each.
+bool Batch::Impl::by_blocks(int p) const {
+  return max_groups <= BATCH_BLOCK_GROUPS || ntasks[p] <= (size_t)BATCH_BLOCK_TASKS_PER_SM * sms;
+}
+
+// All spots' terminals of one traversal.
 void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t, const PassTurn& turn) {
   FastArgs F;
   F.turn = turn;
@@ -1009,7 +1016,7 @@ void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t, const Pas
   F.hp[0] = F.hp[1] = stride;
   F.stride = stride;
   F.p = p;
-  if (max_groups <= BATCH_BLOCK_GROUPS || ntasks[p] <= (size_t)BATCH_BLOCK_TASKS_PER_SM * sms) {
+  if (by_blocks(p)) {
     launch_fast_terminal(F, term[p], (int)ntasks[p], block_blocks, stream);
     return;
   }
@@ -1071,9 +1078,11 @@ Status Batch::Impl::capture(uint32_t iters) {
   BK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
   for (uint32_t i = 0; i < iters; i++) enqueue_iteration(false, false);
   BK(cudaStreamEndCapture(stream, &g));
-  BK(cudaGraphInstantiate(&graph, g, 0));
+  const cudaError_t e = cudaGraphInstantiate(&graph, g, 0);
   cudaGraphDestroy(g);
+  BK(e);
   graph_iters = iters;
+  BK(cudaGraphUpload(graph, stream));
   return Status();
 }
 
@@ -1083,7 +1092,7 @@ Status Batch::Impl::run(uint32_t n) {
   Status s;
   if (!(s = ensure_discounts(iterations + n + 1)).ok()) return s;
   const uint32_t k = std::max<uint32_t>(tuning.iterations_per_launch, 1);
-  if (!(s = capture(k)).ok()) return s;
+  if (n >= 2 && n - 2 >= k && !(s = capture(k)).ok()) return s;
   BK(cudaEventRecord(ev0, stream));
   if (n > 0) {
     enqueue_start(true);
@@ -1161,30 +1170,38 @@ Status Batch::set_tuning(const dcfr_batch_tuning& t) {
   return Status();
 }
 
-// The project's autotuner: times each candidate (warps per block, blocks
-// per SM, iterations per launch, longest-first or natural order) on
-// `trial_iterations` iterations from a snapshot of the storage, restores the
-// snapshot and the iteration counter after every trial, and keeps the
-// fastest candidate.
+// The project's autotuner: times each candidate (warps per block, blocks per
+// SM, iterations per launch, longest-first or natural order) from a snapshot of
+// the storage, restores the snapshot and the iteration counter after every trial,
+// and keeps the fastest candidate and its graph. A trial is two iterations more
+// than trial_iterations: the first and the last of a run are never in a graph.
+// Warps and blocks are a dimension only where a group kernel runs the terminals.
 Status Batch::autotune(uint32_t trial_iterations, dcfr_batch_tuning& best) {
   Impl& I = *impl_;
   Status s;
   const uint64_t n = std::max<uint64_t>(I.total_store, 1);
-  float *r0 = nullptr, *s0 = nullptr;
-  if (!(s = balloc(r0, n, "autotune snapshot")).ok()) return s;
-  if (!(s = balloc(s0, n, "autotune snapshot")).ok()) {
-    bfree(r0);
-    return s;
-  }
-  BK(cudaMemcpyAsync(r0, I.regrets, n * 4, cudaMemcpyDeviceToDevice, I.stream));
-  BK(cudaMemcpyAsync(s0, I.sums, n * 4, cudaMemcpyDeviceToDevice, I.stream));
+  struct Held {
+    float *regrets = nullptr, *sums = nullptr;
+    cudaGraphExec_t graph = nullptr;
+    ~Held() {
+      bfree(regrets);
+      bfree(sums);
+      if (graph) cudaGraphExecDestroy(graph);
+    }
+  } held;
+  if (!(s = balloc(held.regrets, n, "autotune snapshot")).ok()) return s;
+  if (!(s = balloc(held.sums, n, "autotune snapshot")).ok()) return s;
+  BK(cudaMemcpyAsync(held.regrets, I.regrets, n * 4, cudaMemcpyDeviceToDevice, I.stream));
+  BK(cudaMemcpyAsync(held.sums, I.sums, n * 4, cudaMemcpyDeviceToDevice, I.stream));
   const uint32_t t_saved = I.iterations;
   const dcfr_batch_tuning saved = I.tuning;
   std::vector<dcfr_batch_tuning> cands;
-  const uint32_t trial = std::max<uint32_t>(trial_iterations, 1);
-  for (int w = 2; w <= BATCH_MAX_THREADS / 32; w++) {
+  const uint32_t trial = std::max<uint32_t>(trial_iterations, 1), run = trial + 2;
+  if (!(s = I.ensure_discounts(t_saved + run + 1)).ok()) return s;
+  const bool groups = !I.by_blocks(0) || !I.by_blocks(1);
+  for (int w = groups ? 2 : saved.warps; w <= BATCH_MAX_THREADS / 32; w++) {
     if (tuning_smem(I.stride, I.cstride, I.tstride, I.max_slots, w) > (size_t)I.optin) break;
-    if (w > 2 && w > I.max_groups) break;  // no more terminals in flight than at the last candidate
+    if (groups && w > 2 && w > I.max_groups) break;  // no more terminals in flight than at the last candidate
     for (uint32_t ipl : {trial, std::max<uint32_t>(trial / 5, 1u)})
       for (int lpt : {1, 0}) {
         dcfr_batch_tuning t{};
@@ -1194,32 +1211,35 @@ Status Batch::autotune(uint32_t trial_iterations, dcfr_batch_tuning& best) {
         t.longest_first = lpt;
         cands.push_back(t);
       }
+    if (!groups) break;
   }
   double best_ms = 1e300;
   best = saved;
   for (const dcfr_batch_tuning& t : cands) {
     if (!(s = set_tuning(t)).ok()) break;
-    if (!(s = I.run(trial)).ok()) break;
-    const double ms = I.last_ms;
+    if (!(s = I.run(run)).ok()) break;
+    const double ms = I.last_ms * (double)trial / (double)run;
     if (ms < best_ms) {
       best_ms = ms;
       best = I.tuning;
+      std::swap(held.graph, I.graph);
     }
-    BK(cudaMemcpyAsync(I.regrets, r0, n * 4, cudaMemcpyDeviceToDevice, I.stream));
-    BK(cudaMemcpyAsync(I.sums, s0, n * 4, cudaMemcpyDeviceToDevice, I.stream));
+    BK(cudaMemcpyAsync(I.regrets, held.regrets, n * 4, cudaMemcpyDeviceToDevice, I.stream));
+    BK(cudaMemcpyAsync(I.sums, held.sums, n * 4, cudaMemcpyDeviceToDevice, I.stream));
     BK(cudaMemcpyAsync(I.counter, &t_saved, 4, cudaMemcpyHostToDevice, I.stream));
     BK(cudaStreamSynchronize(I.stream));
     I.iterations = t_saved;
   }
-  bfree(r0);
-  bfree(s0);
   if (!s.ok()) {
     set_tuning(saved);
     return s;
   }
   best.trial_ms = best_ms;
   best.candidates = (int)cands.size();
-  return set_tuning(best);
+  if (!(s = set_tuning(best)).ok()) return s;
+  std::swap(held.graph, I.graph);
+  I.graph_iters = best.iterations_per_launch;
+  return Status();
 }
 
 Status Batch::root_values(int mode, std::vector<double>& out) {
