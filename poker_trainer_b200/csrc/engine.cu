@@ -1976,10 +1976,10 @@ Status Engine::solve_loop(const dcfr_solve_options& opts, const volatile int32_t
       CK(cudaStreamSynchronize(stream_));
       return Status();
     }
+    // One at a time under a cancel flag, which is looked at before every one.
+    const uint32_t until = cancel ? iterations + 1 : std::max(next_check, iterations + 1);
     uint32_t k = 0;
-    if (!(s = launch_iterations(std::min(opts.max_iterations, std::max(next_check, iterations + 1)) - iterations, k))
-             .ok())
-      return s;
+    if (!(s = launch_iterations(std::min(opts.max_iterations, until) - iterations, k)).ok()) return s;
     iterations += k;
     bool last = iterations >= opts.max_iterations;
     if (iterations >= next_check || last) {
