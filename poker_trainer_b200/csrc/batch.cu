@@ -448,6 +448,7 @@ Status upload(T*& d, const std::vector<T>& h, const char* what) {
 struct PinnedBlock {
   static constexpr size_t BYTES = 2 << 20, POOL_MOST = 4;
   void* p = nullptr;
+  cudaError_t error = cudaSuccess;
   PinnedBlock() {
     {
       std::lock_guard<std::mutex> hold(pool().lock);
@@ -456,7 +457,8 @@ struct PinnedBlock {
         pool().free.pop_back();
       }
     }
-    if (!p && cudaHostAlloc(&p, BYTES, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+    if (!p) error = cudaHostAlloc(&p, BYTES, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (error != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
     }
@@ -1299,7 +1301,7 @@ Status Batch::download(int spot, float* regrets, float* sums) {
   const Game& g = I.games[spot];
   const std::vector<uint32_t> players = players_in_storage_order(g);
   const PinnedBlock lease;
-  if (!lease.p) return Status{DCFR_ERR_OUT_OF_MEMORY, "page-locked transfer block"};
+  BK(lease.error);
   for (size_t i = 0; i < players.size();) {
     // The nodes that fit: a record and both kinds of cells of each.
     StorageBlockD* rec = static_cast<StorageBlockD*>(lease.p);
