@@ -96,17 +96,22 @@ GemmShape gemm_variant() {
   return GemmShape{(GemmKernel)gemm_bf16_tc_kernel<BN, STAGES, CTAS, DEPTH>, BN, gemm_smem(BN, STAGES, DEPTH)};
 }
 
-// The tile of an [M][N] output. 128 x 128 where that gives three fifths of the
-// SMs a CTA: two to an SM with 3-stage rings once there are more CTAs than
-// SMs (one's epilogue runs under the other's MMAs), else one with long steps.
-// Narrower tiles below (M = 896: 64 wide, M = 256: 32 wide), two to an SM only
+// The tile of an [M][N] output. 128 x 128, two to an SM with 3-stage rings, once
+// that gives more CTAs than SMs (one's epilogue runs under the other's MMAs). With
+// fewer, one to an SM with long steps, of the narrowest tile whose CTAs still
+// run at once: 64 wide where those are 90 or more and no more than the SMs
+// (M = 896, N = 1024), 128 where they are more (us a launch, 64 wide in two waves
+// against 128 in one: 512 x 2688 x 1024 14.7 and 10.9, 2688 x 512 x 512 10.4 and 6.9,
+// 1280 x 1024 x 2816 with GELU 27.7 and 20.3, 1408 x 1024 x 1024 18.2 and 14.1; 144 CTAs
+// of 64, 512 x 2304 x 1024, 8.0 and 10.9). Below, 32 wide (M = 256), two to an SM only
 // where there are more CTAs than SMs.
+constexpr int SMS = 148;
 GemmShape gemm_shape(int M, int N) {
   const int rows = M / GEMM_BM;
-  if (rows * (N / 128) > 148) return gemm_variant<128, 3, 2>();
-  if (rows * (N / 128) >= 90) return gemm_variant<128, 3, 1, 2>();
+  if (rows * (N / 128) > SMS) return gemm_variant<128, 3, 2>();
+  if (rows * (N / 64) > SMS) return gemm_variant<128, 3, 1, 2>();
   if (rows * (N / 64) >= 90) return gemm_variant<64, 3, 1, 3>();
-  if (rows * (N / 32) > 148) return gemm_variant<32, 5, 2>();
+  if (rows * (N / 32) > SMS) return gemm_variant<32, 5, 2>();
   return gemm_variant<32, 3, 1, 3>();
 }
 
