@@ -236,8 +236,11 @@ KERNEL_NAMES = {"terminal": "fast_terminal_kernel", "down": "down_kernel", "up":
 # The CUDA kernel behind each terminal kernel name of dcfr_terminal_kernel.
 TERMINAL_FN = {"panel": "panel_terminal_kernel", "warp": "warp_terminal_kernel", "block": "fast_terminal_kernel",
                "group": "group_terminal_kernel", "exact": "exact_terminal_kernel"}
-# "group" on a flop (384 terminals a multiprocessor and more): tiles of terminals.
-FLOP_TERMINAL_FN = dict(TERMINAL_FN, group="tile_terminal_kernel")
+
+
+def terminal_fn(kernel: str, together: int) -> str:
+    """The CUDA kernel behind Solver.terminal_kernel(): "group" with a count runs tiles."""
+    return "tile_terminal_kernel" if kernel == "group" and together else TERMINAL_FN[kernel]
 
 
 def spawn_ranks(n: int) -> int:
@@ -407,7 +410,7 @@ def run_ours(args, world, rank, local):
     expl = g.exploitability()
     pot = float(cfg.root.pot)
     it_bytes = g.iteration_bytes()
-    tkname, _ = g.terminal_kernel()
+    tkname = terminal_fn(*g.terminal_kernel())
     g.close()
 
     value = world * K / (ms / 1000.0)
@@ -437,7 +440,7 @@ def run_ours(args, world, rank, local):
     working = it_bytes
     kname = KERNEL_NAMES[dom]
     if dom == "terminal":
-        kname = TERMINAL_FN[tkname]
+        kname = tkname
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W,
         "ms_per_step": ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -507,7 +510,7 @@ def run_turn_secondary(args, grp, local):
     return {"workload": WORKLOADS["turn"], "value": grp.world * args.steps / (ms / 1000.0), "unit": UNIT,
             "ms_per_iteration": ms / args.steps,
             "iteration_roofline_frac": it_bytes * args.steps / (ms / 1000.0) / 1e9 / peak,
-            "terminal_kernel": TERMINAL_FN[kname], "terminals_per_panel": per_panel,
+            "terminal_kernel": terminal_fn(kname, per_panel), "terminals_per_panel": per_panel,
             "terminal_gbs": t["bytes"] / (t["ms"] / 1000.0) / 1e9 if t["ms"] > 0 else None,
             "terminal_frac": (t["bytes"] / (t["ms"] / 1000.0) / 1e9 / peak) if t["ms"] > 0 else None,
             "peak_kind": f"of {peak_kind}"}
@@ -583,7 +586,7 @@ def run_flop(args, world, rank, local):
     per_launch_ms = dc["ms"] / max(dc["launches"], 1)
     per_launch_bytes = dc["bytes"] / max(dc["launches"], 1)
     achieved = per_launch_bytes / (per_launch_ms / 1000.0) / 1e9 if per_launch_ms > 0 else 0.0
-    kfull = FLOP_TERMINAL_FN[kname] if dom == "terminal" else KERNEL_NAMES[dom]
+    kfull = terminal_fn(kname, per_panel) if dom == "terminal" else KERNEL_NAMES[dom]
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1

@@ -400,8 +400,8 @@ int dcfr_setup_profile_get(const dcfr_solver* s, dcfr_setup_profile* out);
 
 /* Measurement hook, no counterpart in the reference: the terminal kernel
  * this handle's f32 traversals launch (DCFR_TERMINAL_*; GROUP: two or four
- * warps per terminal, tiles of terminals in large trees), and for the panel kernel the terminals evaluated together per
- * panel (0 otherwise). */
+ * warps per terminal, or tiles of terminals in large trees), and how many
+ * terminals are evaluated together, per panel or per tile (0: neither). */
 enum {
   DCFR_TERMINAL_PANEL = 0,
   DCFR_TERMINAL_WARP = 1,

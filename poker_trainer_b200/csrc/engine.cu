@@ -467,10 +467,13 @@ Status Engine::ensure_fast_layouts() {
   }
   // The f32 solve's terminal kernel: a warp per terminal for short hand
   // lists, a block-wide scan per terminal for long ones (measured fastest);
-  // DCFR_TERMINAL_KERNEL selects another one (panel, panel4, panel8, warp,
-  // block) for comparisons.
+  // DCFR_TERMINAL_KERNEL selects another one (panel, panel4, panel8, warp, block,
+  // group, tile) for comparisons.
   const char* sel = std::getenv("DCFR_TERMINAL_KERNEL");
-  const std::string want = sel ? sel : (tstride_ <= WARP_TERMINAL_MAX_HANDS ? "warp" : "block");
+  const std::string usual = tstride_ <= WARP_TERMINAL_MAX_HANDS ? "warp" : "block";
+  std::string want = sel ? sel : usual;
+  const bool tiles = want == "tile";  // where the hand lists allow them, else the usual kernel
+  if (tiles) want = usual;
   term_kernel_ = want == "warp" || want == "warpdyn" || want == "group" ? TK_WARP
                  : want == "block" || want == "blockdyn" ? TK_BLOCK
                                                          : TK_PANEL;
@@ -501,9 +504,9 @@ Status Engine::ensure_fast_layouts() {
   // SM lose to staging and part tiles, 99 against 87 (777 hands) and 51 against
   // 46 (470).
   tile_T_ = 0;
-  if (fast_ && (want == "tile" || (sel == nullptr && g.stats.terminal >= (uint64_t)TILE_TERMINALS_PER_SM * sms)))
+  if (fast_ && (tiles || (sel == nullptr && g.stats.terminal >= (uint64_t)TILE_TERMINALS_PER_SM * sms)))
     tile_T_ = tile_terminal_setup(g.n[0], g.n[1], hp_[0], hp_[1]);
-  if (want == "tile" && tile_T_ > 0) term_group_ = true;
+  if (tiles && tile_T_ > 0) term_group_ = true;
   if (tile_T_ > 0 && !(s = dalloc(tile_claims_, 2, "terminal counter")).ok()) return s;
   if (term_kernel_ == TK_PANEL) {
     const int o0 = 1, o1 = 0;  // opponent of traverser 0 and 1

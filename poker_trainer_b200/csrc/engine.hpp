@@ -236,10 +236,10 @@ class Engine {
   Status ranges_after(const std::vector<dcfr_step>& path, float out[2][DCFR_NUM_COMBOS]);
   Status actions_at(const std::vector<dcfr_step>& path, std::vector<Act>& out, bool& decision);
   double iteration_bytes() const;
-  // The f32 traversals' terminal kernel (DCFR_TERMINAL_*) and panel width.
+  // The f32 traversals' terminal kernel (DCFR_TERMINAL_*) and panel or tile width.
   void terminal_kernel(int32_t& kernel, int32_t& per_panel) const {
     kernel = !fast_ ? DCFR_TERMINAL_EXACT : term_group_ ? DCFR_TERMINAL_GROUP : term_kernel_;
-    per_panel = fast_ && term_kernel_ == TK_PANEL ? panel_T_ : 0;
+    per_panel = !fast_ ? 0 : term_group_ ? tile_T_ : term_kernel_ == TK_PANEL ? panel_T_ : 0;
   }
   int isomorphic_pairs() const;
   // Offset of a decision node's block in the reference storage layout.

@@ -479,9 +479,9 @@ class Solver:
         return {f[0]: getattr(sp, f[0]) for f in abi.SetupProfile._fields_}
 
     def terminal_kernel(self) -> tuple:
-        """(kernel name, terminals per panel) of this handle's f32 terminal
-        evaluation: "panel", "warp", "block", "group" (two or
-        four warps per terminal, tiles of terminals in large trees) or "exact"."""
+        """(kernel name, terminals per panel or tile) of this handle's f32
+        terminal evaluation: "panel", "warp", "block", "group" (two or four
+        warps per terminal; with a count, tiles of so many) or "exact"."""
         k = C.c_int32()
         t = C.c_int32()
         check(lib().dcfr_terminal_kernel(self._h, C.byref(k), C.byref(t)))
