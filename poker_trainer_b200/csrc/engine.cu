@@ -48,6 +48,8 @@ static void dfree(T*& p) {
 
 // Terminals per SM from which the tile kernel evaluates them.
 constexpr int TILE_TERMINALS_PER_SM = 384;
+// Decision nodes per level up to which a root segment takes segment passes.
+constexpr size_t SEG_NODES_PER_LEVEL = 14;
 
 // To be called between cudaMemcpy from host arrays and work on a handle's stream
 // that reads them: the copy from pageable memory may still be on its way when
@@ -898,7 +900,16 @@ Status Engine::build_plan(uint32_t root, int p, Plan& plan) {
       plan.seg_up[l].push_back(Plan::Level{(uint32_t)plan.h_up.size(), (uint32_t)sup[l][d].size(), maxa, {0, 0, 0}});
       plan.h_up.insert(plan.h_up.end(), sup[l][d].begin(), sup[l][d].end());
     }
-  plan.seg = !compressed_ && g.nodes[root].kind == N_PLAYER;
+  // Segment passes for a root segment of few nodes a level: a slice's block takes
+  // a level's nodes eight at a time, the level kernels have a block a node. us an
+  // iteration, passes against levels (rivers, 5 levels): 46 nodes of up to 9
+  // actions, 200 hands 39 and 51; 62 nodes, 40 hands 32 and 46, 1081 hands 43 and 53;
+  // 102 nodes, 200 hands 70 and 53, 1081 hands 64 and 56; 142 nodes 98 and 62. With 6
+  // levels: 84 nodes 51.7 and 52.7, 162 nodes 97 and 60.
+  size_t seg_nodes = 0, seg_levels = 0;
+  if (!plan.seg_up.empty())
+    for (const Plan::Level& lv : plan.seg_up[0]) seg_nodes += lv.count, seg_levels++;
+  plan.seg = !compressed_ && g.nodes[root].kind == N_PLAYER && seg_nodes <= SEG_NODES_PER_LEVEL * seg_levels;
   // One task per terminal, grouped by layout. A fold below
   // a river decision node is evaluated on its river board's layout: the
   // opponent hands that layout leaves out hold a board card and have zero
