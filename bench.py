@@ -232,6 +232,11 @@ def ncu_traffic(kernel: str, workload: str):
     return None
 
 
+def flop_name(args) -> str:
+    """The flop's name in profiles/: the captures are of f32 storage and every card."""
+    return "flop" + ("-sampled" if args.chance == "sampled" else "") + ("" if args.storage == "f32" else "-16bit")
+
+
 KERNEL_NAMES = {"terminal": "fast_terminal_kernel", "down": "down_kernel", "up": "up_kernel", "other": "other"}
 # The CUDA kernel behind each terminal kernel name of dcfr_terminal_kernel.
 TERMINAL_FN = {"panel": "panel_terminal_kernel", "warp": "warp_terminal_kernel", "block": "fast_terminal_kernel",
@@ -634,7 +639,7 @@ def run_flop(args, world, rank, local):
                         "iteration"},
         "roofline": {"bound": "hbm", "kernel": kfull, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
-                     "traffic": ncu_traffic(kfull, "flop"), "bytes_per_launch": per_launch_bytes,
+                     "traffic": ncu_traffic(kfull, flop_name(args)), "bytes_per_launch": per_launch_bytes,
                      "ms_per_launch": per_launch_ms, "terminals_per_panel": per_panel},
         "iteration_roofline": {"bytes_per_iteration": it_bytes,
                                "achieved": it_bytes * (K / (ms / 1000.0)) / 1e9, "peak": peak, "unit": "GB/s",

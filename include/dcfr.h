@@ -422,7 +422,8 @@ int dcfr_iterate_profiled(dcfr_solver* s, uint32_t iterations, dcfr_kernel_profi
  * one shared DcfrParams) solved together: each DCFR iteration of every spot
  * is the same as a single dcfr_create/dcfr_iterate solve of that spot, done
  * by a few launches over all of them from a captured CUDA graph; spots of
- * uneven tree size are taken longest first. */
+ * uneven tree size are taken longest first. A spot's tree may have up to 4096
+ * reach slots a traversal (about 8,000 nodes), else DCFR_ERR_UNSUPPORTED. */
 typedef struct dcfr_batch dcfr_batch;
 
 /* Launch shape of the batched kernel, chosen by dcfr_batch_autotune. */

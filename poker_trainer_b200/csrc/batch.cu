@@ -18,7 +18,7 @@
 //     the scan layouts per spot (terminal_group.cu; terminal_fast.cu for few).
 // A persistent block per spot, for whole iterations, left a spot's 400 nodes
 // to 6 warps and the GPU to its longest spots: 37 spots of 1081 hands took
-// 1622 us an iteration where they now take 105, 512 spots 2078 us, now 1011.
+// 1622 us an iteration where they now take 105, 512 spots 2078 us, now 960.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1026,7 +1026,7 @@ void Batch::Impl::enqueue_terminals(int p, const dcfr_batch_tuning& t, const Pas
                         sms * std::max(t.blocks_per_sm, 1), stream);
 }
 
-// One iteration (M_CFR), best-response or average pair of every spot.
+// Before a run's first down pass: flags cleared, and the iteration stepped.
 void Batch::Impl::enqueue_start(bool advance) {
   launch_traversal_start(alive, (int)total_slots, alive + total_slots, (int)total_slots, reach, roots, 0,
                          advance ? counter : nullptr, disc, disc_len, cur_disc, nullptr, stream);
@@ -1050,7 +1050,7 @@ Status Batch::Impl::launch_evaluation(int mode, const dcfr_batch_tuning& t) {
 // second traversal is one launch with the next iteration's first down pass,
 // and the terminal kernels do what a start kernel would (PassTurn), as in
 // Engine::enqueue_rolled (us an iteration against separate ones: 37 spots 113
-// to 105, 512 spots 1018 to 1011).
+// to 105, 512 spots 1018 to 1011 then).
 void Batch::Impl::enqueue_iteration(bool first, bool last) {
   const bool lpt = tuning.longest_first != 0;
   PassTurn turn;

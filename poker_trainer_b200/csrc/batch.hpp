@@ -13,7 +13,7 @@
 
 namespace dcfr {
 
-constexpr int BATCH_MAX_THREADS = 256;  // threads per block of the batched kernel
+constexpr int BATCH_MAX_THREADS = 256;  // 32 x the most dcfr_batch_tuning::warps
 constexpr int BATCH_MAX_SLOTS = 4096;   // reach slots of one spot's traversal
 
 class Batch {

@@ -172,8 +172,6 @@ constexpr int ROW_UNIT = 8;  // rows are padded to this many hands
 constexpr int FAST_SEGS = 54;
 constexpr int FAST_THREADS = 256;
 
-// R is the row type: float for the solve, double for the FP64 best-response
-// oracle (br64.cu).
 // Between two traversals that share a segment pass across the end of an
 // iteration (Engine::enqueue_rolled), a terminal kernel clears the other
 // traverser's liveness flags, whose last reader is done and whose next writer
@@ -191,6 +189,8 @@ struct PassTurn {
   DiscountD* cur = nullptr;
 };
 
+// R is the row type: float for the solve, double for the FP64 best-response
+// oracle (br64.cu).
 template <typename R>
 struct FastArgsT {
   const R* reach;

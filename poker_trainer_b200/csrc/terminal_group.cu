@@ -31,11 +31,11 @@
 
 namespace dcfr {
 
+// Groups of two per SM up to which a group takes four warps.
+constexpr int GROUP_WIDE_MAX = 8;
 // Groups per block (named barriers 1..group_max). 24 warps leave 80 registers a
 // thread with no spills; 28 (72 registers, a few spills) measured 1.5% slower
 // on the flop.
-// Groups of two per SM up to which a group takes four warps.
-constexpr int GROUP_WIDE_MAX = 8;
 constexpr int group_max(int warps) { return 24 / warps; }
 
 // Shared memory of a block: the staged layout (shared by the block's

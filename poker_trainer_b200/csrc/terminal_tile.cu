@@ -25,7 +25,9 @@
 // Values are bit-identical to the other kernels': the same integer sums, the
 // same conversions and the same rounding order per terminal kind.
 //
-// Bound by shared-memory wavefronts, at two thirds of their rate: a tile of 16
+// Bound by shared memory's latency and barriers at one block an SM: 0.53 of its
+// one wavefront a cycle on a flop, 0.46 with sampled cards (ncu; short scoreboard
+// and barrier are the largest stalls). A tile of 16
 // terminals at 470 hands takes 14,600 cycles, of which maxima 360, X 1530, run
 // sums 870, card lists 3040, placing 1850 and values 6940 (two warps per
 // terminal: 16 x 1125 cycles). A flop's terminals, ms a traversal: 10.8 to 8.3.
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 1)
     __syncthreads();
   };
   // The live tasks among the TILE_THREADS from `from` on, in order: their
-  // number to scount[2], their places to slist.
+  // places go to slist, their number is returned.
   auto window = [&](int from, int end) {
     const int i = from + tid;
     const bool live = i < end && A.alive[tasks[i].slot] != 0;  // dead subtree (cfr.rs:267-274): rows untouched
